@@ -28,7 +28,9 @@ template <int BM, int BN, int WM, int WN>
 __global__ void __launch_bounds__(WM * WN * 32)
     dmma_gemm(int64_t m, int64_t n, int64_t k, int64_t kc, const double* __restrict__ A, int64_t rsa,
               int64_t csa, const double* __restrict__ B, int64_t rsb, int64_t csb,
-              double* __restrict__ C, int64_t ldc, int accumulate, double* __restrict__ P) {
+              double* __restrict__ C, int64_t ldc, int accumulate, double* __restrict__ P,
+              const uint32_t* __restrict__ unless) {
+  if (unless && *unless) return;
   using Tile = Dmma<BM, BN, WM, WN>;
   __shared__ __align__(16) uint8_t smem[Tile::kSmem];
   Tile t;
@@ -42,16 +44,22 @@ __global__ void __launch_bounds__(WM * WN * 32)
 }
 
 // C := p_0 + p_1 + ... + p_{S-1} (slab order), or C += that sum: the product
-// is rounded before it meets C, as without the split.
+// is rounded (to T) before it meets C, as without the split. With `choice`,
+// the slab count is `splits_if` where *choice != 0, else `splits`; one slab
+// means C is already written.
+template <typename T>
 __global__ void splitk_finish(const double* __restrict__ P, int splits, int64_t m, int64_t n,
-                              double* __restrict__ C, int64_t ldc, int accumulate) {
+                              T* __restrict__ C, int64_t ldc, int accumulate, const uint32_t* __restrict__ choice,
+                              int splits_if) {
+  if (choice && *choice) splits = splits_if;
+  if (splits <= 1) return;
   const int64_t mn = m * n;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < mn;
        e += (int64_t)gridDim.x * blockDim.x) {
     double v = P[e];
     for (int z = 1; z < splits; ++z) v += P[z * mn + e];
-    double* c = C + (e / n) * ldc + (e % n);
-    *c = accumulate ? *c + v : v;
+    T* c = C + (e / n) * ldc + (e % n);
+    *c = accumulate ? *c + (T)v : (T)v;
   }
 }
 
@@ -101,7 +109,8 @@ template <typename T, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM * BN >= 128 * 128 ? 2 : 1))
     simt_gemm(int64_t m, int64_t n, int64_t k, const T* __restrict__ A, int64_t rsa, int64_t csa,
               const T* __restrict__ B, int64_t rsb, int64_t csb, T* __restrict__ C, int64_t ldc,
-              int accumulate) {
+              int accumulate, const uint32_t* __restrict__ unless) {
+  if (unless && *unless) return;
   using Tile = Simt<T, BM, BN, BK, TM, TN>;
   __shared__ __align__(16) uint8_t smem[Tile::kSmem];
   Tile t;
@@ -159,16 +168,75 @@ dim3 tiles(int64_t m, int64_t n, int bm, int bn) {
 
 }  // namespace
 
+namespace {
+
+void launch_dmma(nrs_handle* h, const DmmaPlan& pl, int64_t m, int64_t k, int64_t n, const double* A, int64_t rsa,
+                 int64_t csa, const double* B, int64_t rsb, int64_t csb, double* C, int64_t ldc, int acc, double* P,
+                 const uint32_t* unless) {
+  dim3 g = tiles(m, n, pl.tile, pl.tile);
+  g.z = (unsigned)pl.splits;
+  if (pl.tile == 64)
+    dmma_gemm<64, 64, 2, 4><<<g, 256, 0, h->stream>>>(m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, P, unless);
+  else
+    dmma_gemm<32, 32, 2, 2><<<g, 128, 0, h->stream>>>(m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, P, unless);
+}
+
+int finish_grid(nrs_handle* h, int64_t m, int64_t n) {
+  const int64_t blocks = (m * n + 255) / 256;
+  return (int)(blocks < (int64_t)h->num_sms * 8 ? blocks : (int64_t)h->num_sms * 8);
+}
+
+// f32 tile size by the size of C.
+int f32_variant(int64_t m, int64_t n) { return (m * n >= 256LL * 256 * 16) ? NRS_GEMM_SIMT : NRS_GEMM_SIMT_SMALL; }
+
+void launch_simt_f32(nrs_handle* h, bool large, int64_t m, int64_t k, int64_t n, const float* A, int64_t rsa,
+                     int64_t csa, const float* B, int64_t rsb, int64_t csb, float* C, int64_t ldc, int acc,
+                     const uint32_t* unless) {
+  if (large)
+    simt_gemm<float, 128, 128, 8, 8, 8><<<tiles(m, n, 128, 128), 256, 0, h->stream>>>(m, n, k, A, rsa, csa, B, rsb,
+                                                                                      csb, C, ldc, acc, unless);
+  else
+    simt_gemm<float, 32, 32, 16, 2, 2><<<tiles(m, n, 32, 32), 256, 0, h->stream>>>(m, n, k, A, rsa, csa, B, rsb, csb,
+                                                                                   C, ldc, acc, unless);
+}
+
+bool grid_too_large(int64_t m, int64_t n) { return (n + 31) / 32 > 0x7fffffffLL || (m + 31) / 32 > 65535; }
+
+}  // namespace
+
+int nrs_dmma_splits(int64_t m, int64_t k, int64_t n) { return plan_dmma(m, n, k, NRS_PLAN_SMS).splits; }
+
+int nrs_plain_gemm_unless(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t rsa,
+                          int64_t csa, const void* B, int64_t rsb, int64_t csb, void* C, int64_t ldc,
+                          bool accumulate, const uint32_t* unless, double* slab, int tc_splits) {
+  const int acc = accumulate ? 1 : 0;
+  if (dtype == NRS_F64) {
+    const DmmaPlan pl = plan_dmma(m, n, k, NRS_PLAN_SMS);
+    launch_dmma(h, pl, m, k, n, (const double*)A, rsa, csa, (const double*)B, rsb, csb, (double*)C, ldc, acc, slab,
+                unless);
+    if (pl.splits > 1 || tc_splits > 1)
+      splitk_finish<double><<<finish_grid(h, m, n), 256, 0, h->stream>>>(slab, pl.splits, m, n, (double*)C, ldc, acc,
+                                                                         unless, tc_splits);
+  } else {
+    launch_simt_f32(h, f32_variant(m, n) == NRS_GEMM_SIMT, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb,
+                    csb, (float*)C, ldc, acc, unless);
+    if (tc_splits > 1)
+      splitk_finish<float><<<finish_grid(h, m, n), 256, 0, h->stream>>>(slab, 1, m, n, (float*)C, ldc, acc, unless,
+                                                                        tc_splits);
+  }
+  return nrs_after_launch(h, "plain GEMM behind the slice products");
+}
+
 // Launches one plain GEMM. Sizes are validated by the caller.
 int nrs_plain_gemm_launch(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n,
                           const void* A, int64_t rsa, int64_t csa, const void* B, int64_t rsb,
                           int64_t csb, void* C, int64_t ldc, bool accumulate, int variant) {
   const int acc = accumulate ? 1 : 0;
   cudaStream_t s = h->stream;
-  if ((n + 31) / 32 > 0x7fffffffLL || (m + 31) / 32 > 65535) variant = NRS_GEMM_GENERIC;
+  if (grid_too_large(m, n)) variant = NRS_GEMM_GENERIC;
   if (variant == NRS_GEMM_AUTO) {
     if (dtype == NRS_F64) variant = NRS_GEMM_DMMA;
-    else if (dtype == NRS_F32) variant = (m * n >= 256LL * 256 * 16) ? NRS_GEMM_SIMT : NRS_GEMM_SIMT_SMALL;
+    else if (dtype == NRS_F32) variant = f32_variant(m, n);
     else variant = NRS_GEMM_GENERIC;
   }
   if (variant == NRS_GEMM_DMMA && dtype == NRS_F64) {
@@ -180,34 +248,20 @@ int nrs_plain_gemm_launch(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
       P = (double*)nrs_workspace(h, (size_t)pl.splits * (size_t)(m * n) * sizeof(double), &st);
       if (!P) return st;
     }
-    dim3 g = tiles(m, n, pl.tile, pl.tile);
-    g.z = (unsigned)pl.splits;
-    if (pl.tile == 64)
-      dmma_gemm<64, 64, 2, 4><<<g, 256, 0, s>>>(m, n, k, pl.kc, (const double*)A, rsa, csa, (const double*)B,
-                                                rsb, csb, (double*)C, ldc, acc, P);
-    else
-      dmma_gemm<32, 32, 2, 2><<<g, 128, 0, s>>>(m, n, k, pl.kc, (const double*)A, rsa, csa, (const double*)B,
-                                                rsb, csb, (double*)C, ldc, acc, P);
-    if (pl.splits > 1) {
-      const int64_t blocks = (m * n + 255) / 256;
-      const int grid = (int)(blocks < (int64_t)h->num_sms * 8 ? blocks : (int64_t)h->num_sms * 8);
-      splitk_finish<<<grid, 256, 0, s>>>(P, pl.splits, m, n, (double*)C, ldc, acc);
-    }
+    launch_dmma(h, pl, m, k, n, (const double*)A, rsa, csa, (const double*)B, rsb, csb, (double*)C, ldc, acc, P,
+                nullptr);
+    if (pl.splits > 1)
+      splitk_finish<double><<<finish_grid(h, m, n), 256, 0, s>>>(P, pl.splits, m, n, (double*)C, ldc, acc, nullptr, 0);
     return nrs_after_launch(h, "dmma_gemm");
   }
-  if (variant == NRS_GEMM_SIMT && dtype == NRS_F32) {
-    simt_gemm<float, 128, 128, 8, 8, 8><<<tiles(m, n, 128, 128), 256, 0, s>>>(
-        m, n, k, (const float*)A, rsa, csa, (const float*)B, rsb, csb, (float*)C, ldc, acc);
-    return nrs_after_launch(h, "simt_gemm<f32,128>");
-  }
-  if (variant == NRS_GEMM_SIMT_SMALL && dtype == NRS_F32) {
-    simt_gemm<float, 32, 32, 16, 2, 2><<<tiles(m, n, 32, 32), 256, 0, s>>>(
-        m, n, k, (const float*)A, rsa, csa, (const float*)B, rsb, csb, (float*)C, ldc, acc);
-    return nrs_after_launch(h, "simt_gemm<f32,32>");
+  if ((variant == NRS_GEMM_SIMT || variant == NRS_GEMM_SIMT_SMALL) && dtype == NRS_F32) {
+    launch_simt_f32(h, variant == NRS_GEMM_SIMT, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb, csb,
+                    (float*)C, ldc, acc, nullptr);
+    return nrs_after_launch(h, "simt_gemm<f32>");
   }
   if (variant == NRS_GEMM_SIMT && dtype == NRS_F64) {
     simt_gemm<double, 64, 64, 8, 4, 4><<<tiles(m, n, 64, 64), 256, 0, s>>>(
-        m, n, k, (const double*)A, rsa, csa, (const double*)B, rsb, csb, (double*)C, ldc, acc);
+        m, n, k, (const double*)A, rsa, csa, (const double*)B, rsb, csb, (double*)C, ldc, acc, nullptr);
     return nrs_after_launch(h, "simt_gemm<f64,64>");
   }
   if (variant != NRS_GEMM_GENERIC && variant != NRS_GEMM_DMMA && variant != NRS_GEMM_SIMT &&
@@ -267,6 +321,10 @@ extern "C" int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t 
     return nrs_after_launch(h, "zero_fill_2d");
   }
   if (!A || !B) return nrs_fail(h, NRS_ERR_INVALID, "null A or B");
+  if (variant == NRS_GEMM_AUTO && !grid_too_large(m, n)) {
+    st = nrs_tc_gemm_auto(h, dtype, m, k, n, A, lda, ta, B, ldb, tb, C, ldc, accumulate);
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   const int64_t rsa = ta ? 1 : lda, csa = ta ? lda : 1;
   const int64_t rsb = tb ? 1 : ldb, csb = tb ? ldb : 1;
   return nrs_plain_gemm_launch(h, dtype, m, k, n, A, rsa, csa, B, rsb, csb, C, ldc, accumulate,

@@ -29,6 +29,8 @@ struct nrs_host_stage;  // pinned staging slots for file I/O (npy.cu)
 // the handle's num_sms, plans from this constant, so results do not depend
 // on the device or on the handle's SM budget.
 constexpr int NRS_PLAN_SMS = 152;
+// Scratch of an 8192^3 product (3.5 GB) with some room.
+constexpr uint64_t kPoolKeep = 4608ull << 20;
 
 struct nrs_handle {
   int device = 0;
@@ -39,6 +41,10 @@ struct nrs_handle {
   // Grow-only device workspace for kernels that need scratch memory.
   void* workspace = nullptr;
   size_t workspace_bytes = 0;
+  // Stream-ordered scratch of the calls that choose the tensor cores by
+  // themselves (null: they keep to the plain kernels). Up to kPoolKeep bytes
+  // stay with the pool between calls; it goes with the handle.
+  cudaMemPool_t pool = nullptr;
   // Device error word written by kernels whose waits are bounded.
   uint32_t* dev_error = nullptr;
   std::string last_error;
@@ -90,6 +96,16 @@ void nrs_tuner_forget(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n)
 int nrs_plain_gemm_launch(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n,
                           const void* A, int64_t rsa, int64_t csa, const void* B, int64_t rsb,
                           int64_t csb, void* C, int64_t ldc, bool accumulate, int variant);
+
+// The plain kernel behind a tensor-core launch: its blocks return at once when
+// *unless != 0. `slab` holds the K-split partials of whichever of the two ran
+// (tc_splits of them, or the plain plan's), added in order into C.
+int nrs_plain_gemm_unless(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t rsa,
+                          int64_t csa, const void* B, int64_t rsb, int64_t csb, void* C, int64_t ldc,
+                          bool accumulate, const uint32_t* unless, double* slab, int tc_splits);
+int nrs_dmma_splits(int64_t m, int64_t k, int64_t n);
+int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
+                     const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate);
 
 // ---------------------------------------------------------------------------
 // Device helpers: mbarrier and TMA (inline PTX, sm_90+ forms valid on sm_103a)

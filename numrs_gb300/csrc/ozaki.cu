@@ -143,6 +143,17 @@ NRS_DEV void tc_commit(uint64_t* bar) {
       : "memory");
 }
 
+// One lane of a converged warp (the same one every time).
+NRS_DEV bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // 32 lanes x 16 consecutive 32-bit columns.
 NRS_DEV void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
@@ -201,6 +212,41 @@ NRS_DEV uint64_t smem_desc_sw128(uint32_t saddr) {
   return d;
 }
 
+// What a slice count has to satisfy (oz_decide).
+struct OzRule {
+  int target_bits;  // operand bits wanted at spread 1 (53 for f64, 26 for f32)
+  int digit_bits;
+  int max_slices;   // beyond: 0 (the caller's FP64 / FP32 kernel runs instead)
+  int exp_limit;    // max row + column exponent whose dot products cannot overflow T
+};
+
+// Words of the decision block, zeroed by oz_max, filled by oz_est and the
+// estimate product.
+// OZ_W_COUNT: the slice count that oz_slice decided on, read by the launches
+// behind it.
+enum { OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_EXP_A = 2, OZ_W_EXP_B = 3, OZ_W_COUNT = 4, OZ_WORDS = 5 };
+constexpr int kExpBias = 4096;  // exponents are collected biased, as unsigned maxima
+
+// The slice count for the measured spread R (float bits): the smallest S with
+// R <= 2^(b S - target), so that 2^-(bS) R stays at the target; 0 when no
+// count up to the limit reaches it, an operand holds Inf or NaN, or a partial
+// sum could overflow the element type (the plain kernel then gives its own
+// Inf / NaN).
+__device__ __forceinline__ int oz_decide(const uint32_t* w, const OzRule& r) {
+  const uint32_t spread = __ldcg(w + OZ_W_SPREAD);
+  if (__ldcg(w + OZ_W_NONFINITE)) return 0;
+  const int e = (int)__ldcg(w + OZ_W_EXP_A) + (int)__ldcg(w + OZ_W_EXP_B) - 2 * kExpBias;
+  if (e > r.exp_limit) return 0;
+  int S = (r.target_bits + r.digit_bits - 1) / r.digit_bits;
+  for (; S <= r.max_slices; ++S)
+    if (spread <= (uint32_t)(127 + r.digit_bits * S - r.target_bits) << 23) return S;
+  return 0;
+}
+
+// Fixed-point scale of the estimate's row / column sums of |x'| (smaller for
+// K beyond 2^15): integers add in any order to the same sum.
+constexpr float kSumScale = 65536.0f;
+
 struct OzParams {
   int64_t m, n, k, kpad;
   int slices;
@@ -211,19 +257,28 @@ struct OzParams {
   const int* ea;   // row exponents of A
   const int* eb;   // column exponents of B
   __int128* acc;   // per-CTA digit slots (16-byte aligned)
-  double* C;
+  double* C;       // float when f32 (and not split)
   int64_t ldc;
-  int final_shift; // 2 - 2b - b(S-1) for b-bit digits
   int digit_bits;  // b
   int kchunk;      // exact FP32 K chunk, 2^(26-2b)
   int accumulate;  // C += result instead of C = result
   uint32_t* err;
   // Spread estimate only (EST kernel): row sums of |A'| and column sums of
-  // |B'| (operands scaled by their row / column exponents), and the word
-  // that collects max_ij of the ratio as float bits.
-  const float* ra;
-  const float* cb;
+  // |B'| (operands scaled by their row / column exponents; fixed point, in
+  // units of sum_unit), and the word that collects max_ij of the ratio as
+  // float bits.
+  const uint32_t* ra;
+  const uint32_t* cb;
+  float sum_unit;
   uint32_t* est;
+  // Slice count decided on the device (null: the count is `slices`). A count
+  // of 0 makes the launch return at once.
+  const uint32_t* count;
+  // One problem on 128 x 128 tiles (grouped geometry, no tile list): K in
+  // `splits` ranges of split_blocks 64-wide blocks. With several, range z
+  // writes its product to the f64 slab C + z m n (row pitch n).
+  int splits, split_blocks;
+  int f32;
   // Grouped launch only: the tile list and the problems it points into.
   const struct OzTile* tiles;
   const struct OzProb* probs;
@@ -250,6 +305,7 @@ struct OzTile {
 struct TileCtx {
   int64_t m, n;        // the problem's C dimensions
   int64_t arow, brow;  // TMA row coordinates of the tile's A / B^T boxes
+  int kbase;           // first 64-wide K block
   int64_t row0, col0;  // tile origin inside the problem
   int kblocks, n_pairs, kchunks;
   const int* ea;
@@ -320,83 +376,134 @@ __device__ __forceinline__ int group_size(const PairIter& pi, int gm, int kchunk
 
 
 // Writes 8 consecutive columns of one tile row of C (f64, or f32 when F32):
-// R values w, digit words per column (S <= 5: digits 0..S-2 in lw; else
-// digits 0..3 in lw and 4..7 in hw), digits 8..14 from the 8-byte records
-// `pitch` apart (S > 9 only) and the column exponents; `left` of the 8
-// columns lie inside the problem; the row starts at element `off` of C. The
-// conversions run straight-line for all 8 (interleaved); zero, subnormal and
-// overflowing results are redone by the exact path.
-template <bool F32>
-__device__ __forceinline__ void retire8(const uint32_t (&w)[8], const uint32_t (&lw)[8], const uint32_t (&hw)[8],
-                                        const uint8_t* rec, size_t pitch, const int* eb, int left, int b, int S,
-                                        int ebase, void* C, int64_t off, bool accumulate) {
+// R values w, digits 0..7 of each column in `lo` (digit t = byte t; with B8,
+// i.e. 8-bit digits, and S <= 9 left-aligned instead, digit S-2 on top),
+// digits 8..14 from the 8-byte records `pitch` apart (S > 9 only) and the
+// column exponents; `left` of the 8 columns lie inside the problem; the row
+// starts at element `off` of C. The conversions run straight-line for all 8
+// (the digit width is a template argument and the slice count is tested
+// once, so no branch separates the elements' chains: with both tested per
+// element this pass took 75,000 cycles per 128 x 128 tile, two thirds of a
+// small tile's time); zero, tiny, subnormal and overflowing results are redone by
+// the exact path.
+template <bool F32, bool B8>
+__device__ __forceinline__ void retire8(const uint32_t (&w)[8], const uint64_t (&lo)[8], const uint8_t* rec,
+                                        size_t pitch, const int* eb, int left, int b, int S, int ebase, void* C,
+                                        int64_t off, bool accumulate) {
   using Fmt = typename std::conditional<F32, NrsF32Fmt, NrsF64Fmt>::type;
+  const int nd = S - 1;
   uint64_t hi[8], bits[8];
   int ex[8];
   unsigned special = 0;
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     hi[e] = 0;
-    ex[e] = 0;
-    if (e < left) {
-      if (S > 9) hi[e] = __ldcg(reinterpret_cast<const unsigned long long*>(rec + (size_t)e * pitch));
-      ex[e] = eb[e];
-    }
+    ex[e] = e < left ? eb[e] : 0;
   }
-  if (F32 && b == 8 && S <= 5) {
-    // T = R 2^(8(S-1)) + digits < 2^63: one rounding int64 -> f32 in
-    // hardware, the scale added to the exponent field (exact while the
-    // result stays normal; otherwise the exact path below).
-    const int sh = 8 * (S - 1);
+  const bool top = B8 && nd <= 8;
+  if (top) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const int64_t t = (int64_t)(int32_t)w[e] * ((int64_t)1 << sh) + (int64_t)(lw[e] & (uint32_t)((1ull << sh) - 1));
-      const uint32_t fb = __float_as_uint(__ll2float_rn(t));
-      const int fe = (int)((fb >> 23) & 0xFF) + ebase + ex[e];
-      bits[e] = fb + ((uint32_t)(ebase + ex[e]) << 23);
-      special |= (unsigned)(t == 0 || fe < 1 || fe > 254) << e;
+      bool sp;
+      bits[e] = ozaki_round96<Fmt>((int32_t)w[e], (uint32_t)(lo[e] >> 32), (uint32_t)lo[e], ebase + ex[e] + 8 * nd, sp);
+      special |= (unsigned)sp << e;
     }
   } else {
+    if (S > 9) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (e < left) hi[e] = __ldcg(reinterpret_cast<const unsigned long long*>(rec + (size_t)e * pitch));
+    }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const uint64_t lo = S - 1 > 4 ? (uint64_t)lw[e] | (uint64_t)hw[e] << 32 : (uint64_t)lw[e];
       bool neg, sp;
       uint64_t mhi, mlo;
-      ozaki_exact_total((int32_t)w[e], lo, hi[e], b, S, neg, mhi, mlo);
+      ozaki_exact_total((int32_t)w[e], lo[e], hi[e], B8 ? 8 : b, S, neg, mhi, mlo);
       bits[e] = int128_to_float_bits_fast<Fmt>(neg, mhi, mlo, ebase + ex[e], sp);
       special |= (unsigned)sp << e;
     }
   }
   if (special) {
-#pragma unroll
+#pragma unroll 1
     for (int e = 0; e < 8; ++e) {
       if (!((special >> e) & 1)) continue;
-      const uint64_t lo = S - 1 > 4 ? (uint64_t)lw[e] | (uint64_t)hw[e] << 32 : (uint64_t)lw[e];
+      uint64_t l = 0, h = 0;
+      uint32_t r = 0;
+      int x = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q == e) {
+          l = lo[q];
+          h = hi[q];
+          r = w[q];
+          x = ex[q];
+        }
+      if (top) l = nd ? l >> (64 - 8 * nd) : 0;
       bool neg;
       uint64_t mhi, mlo;
-      ozaki_exact_total((int32_t)w[e], lo, hi[e], b, S, neg, mhi, mlo);
-      bits[e] = int128_to_float_bits<Fmt>(neg, mhi, mlo, ebase + ex[e]);
+      ozaki_exact_total((int32_t)r, l, h, b, S, neg, mhi, mlo);
+      const uint64_t v = int128_to_float_bits<Fmt>(neg, mhi, mlo, ebase + x);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q == e) bits[q] = v;
     }
   }
+  using T = typename std::conditional<F32, float, double>::type;
+  constexpr int PER = 16 / (int)sizeof(T);
+  T* cp = static_cast<T*>(C) + off;
+  T v[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    if (e >= left) continue;
-    if (F32) {
-      float* cp = static_cast<float*>(C) + off + e;
-      const float r = __uint_as_float((uint32_t)bits[e]);
-      *cp = accumulate ? *cp + r : r;
-    } else {
-      double* cp = static_cast<double*>(C) + off + e;
-      const double r = __longlong_as_double((long long)bits[e]);
-      *cp = accumulate ? *cp + r : r;
+    if constexpr (F32) v[e] = __uint_as_float((uint32_t)bits[e]);
+    else v[e] = __longlong_as_double((long long)bits[e]);
+  }
+  if (!accumulate && left >= 8 && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
+#pragma unroll
+    for (int q = 0; q < 8 / PER; ++q) {
+      uint4 u;
+      memcpy(&u, &v[q * PER], 16);
+      reinterpret_cast<uint4*>(cp)[q] = u;
     }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (e < left) cp[e] = accumulate ? cp[e] + v[e] : v[e];
   }
 }
 
+// `S`: the launch's slice count (tile lists carry their own pair counts).
 template <bool G>
-__device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int tile) {
+__device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int S, int tile) {
   TileCtx c;
-  if (G) {
+  c.kbase = 0;
+  if (G && !P.tiles) {
+    const int per = P.tiles_m * P.tiles_n;
+    const int z = tile / per;
+    int tm, tn;
+    tile_coords(tile - z * per, P, tm, tn);
+    c.m = P.m;
+    c.n = P.n;
+    c.row0 = c.arow = (int64_t)tm * OZ_BM;
+    c.col0 = c.brow = (int64_t)tn * OzGeom<true>::BN;
+    c.kbase = z * P.split_blocks;
+    const int kb = (int)((P.kpad + OZ_BK - 1) / OZ_BK) - c.kbase;
+    c.kblocks = kb < P.split_blocks ? kb : P.split_blocks;
+    const int chunk_blocks = P.kchunk / OZ_BK;
+    c.kchunks = (c.kblocks + chunk_blocks - 1) / chunk_blocks;
+    c.n_pairs = S * (S + 1) / 2 * c.kchunks;
+    c.ea = P.ea;
+    c.eb = P.eb;
+    if (P.splits > 1) {
+      c.C = P.C + (int64_t)z * P.m * P.n;
+      c.ldc = P.n;
+      c.accumulate = c.f32 = 0;
+    } else {
+      c.C = P.C;
+      c.ldc = P.ldc;
+      c.accumulate = P.accumulate;
+      c.f32 = P.f32;
+    }
+  } else if (G) {
     const OzTile t = P.tiles[tile];
     const OzProb& q = P.probs[t.prob];
     c.m = q.m;
@@ -422,14 +529,14 @@ __device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int tile) {
     c.row0 = c.arow = (int64_t)tm * OZ_BM;
     c.col0 = c.brow = (int64_t)tn * OZ_BN;
     c.kblocks = (int)((P.kpad + OZ_BK - 1) / OZ_BK);
-    c.n_pairs = P.n_pairs;
+    c.n_pairs = P.count ? S * (S + 1) / 2 * P.kchunks : P.n_pairs;
     c.kchunks = P.kchunks;
     c.ea = P.ea;
     c.eb = P.eb;
     c.C = P.C;
     c.ldc = P.ldc;
     c.accumulate = P.accumulate;
-    c.f32 = 0;
+    c.f32 = P.f32;
   }
   return c;
 }
@@ -441,7 +548,8 @@ __device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int tile) {
 //              products N = |A'| 1_B^T + 1_A |B'|^T of slices 0 and 1 (|x'|
 //              and the nonzero indicator). The epilogue folds
 //              max_ij (numerator_ij / D_ij) into P.est instead of writing C.
-template <bool EST, bool G>
+// B8: 8-bit digits (else 7 or 6, P.digit_bits).
+template <bool EST, bool G, bool B8>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     ozaki_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                     OzParams P) {
@@ -456,8 +564,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (warp-uniform, and known to be)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n_tiles = G ? P.n_tiles : P.tiles_m * P.tiles_n;
+  const int S = P.count ? (int)__ldcg(P.count) : P.slices;
+  if (S == 0) return;  // (the same words for every thread)
+  const int final_shift = 2 - 2 * P.digit_bits - P.digit_bits * (S - 1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Geo::STAGES; ++s) {
@@ -495,25 +607,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      uint32_t it = 0;
+    if (elect_one()) {
+      uint32_t s = 0, ph = 1, it = 0;  // ring slot, its empty phase, loads issued
       bool ok = true;
+      const int chunk_blocks = P.kchunk / OZ_BK;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const TileCtx c = tile_ctx<G>(P, tile);
+        const TileCtx c = tile_ctx<G>(P, S, tile);
+        const int32_t arow = (int32_t)c.arow, brow = (int32_t)c.brow;
         PairIter pr;
-        pr.start(P.slices);
+        pr.start(S);
         for (int u = 0; u < c.n_pairs && ok; ++u, pr.next(c.kchunks)) {
-          const int kb0 = pr.chunk * (P.kchunk / OZ_BK);
-          int kb1 = kb0 + P.kchunk / OZ_BK;
-          if (kb1 > c.kblocks) kb1 = c.kblocks;
-          for (int kb = kb0; kb < kb1; ++kb, ++it) {
-            const int s = it % Geo::STAGES;
-            const uint32_t ph = (it / Geo::STAGES) & 1;
-            if (!bounded(&empty[s], ph ^ 1, 1)) { ok = false; break; }
+          const int kb0 = pr.chunk * chunk_blocks;
+          const int kb1 = kb0 + chunk_blocks < c.kblocks ? kb0 + chunk_blocks : c.kblocks;
+          const int32_t sa = pr.s, sb = pr.t();
+          int32_t x = (c.kbase + kb0) * OZ_BK;
+          for (int kb = kb0; kb < kb1; ++kb, ++it, x += OZ_BK) {
+            if (!bounded(&empty[s], ph, 1)) { ok = false; break; }
             uint8_t* st = smem + s * Geo::STAGE_BYTES;
             mbar_arrive_expect_tx(&full[s], Geo::STAGE_BYTES);
-            tma_load_3d(st, &mapA, &full[s], kb * OZ_BK, (int32_t)c.arow, pr.s);
-            tma_load_3d(st + OZ_A_BYTES, &mapB, &full[s], kb * OZ_BK, (int32_t)c.brow, pr.t());
+            tma_load_3d(st, &mapA, &full[s], x, arow, sa);
+            tma_load_3d(st + OZ_A_BYTES, &mapB, &full[s], x, brow, sb);
+            if (++s == Geo::STAGES) {
+              s = 0;
+              ph ^= 1;
+            }
           }
         }
       }
@@ -525,41 +642,48 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      uint32_t it = 0, ai = 0;
+    if (elect_one()) {
+      uint32_t s = 0, ph = 0, ai = 0;  // ring slot, its full phase, accumulation groups
       bool ok = true;
+      const bool two = EST ? P.slices == 1 : Geo::ACC_BUFS == 2;
+      const int chunk_blocks = P.kchunk / OZ_BK;
+      const uint64_t adesc0 = smem_desc_sw128(smem_u32(smem));
+      const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem) + OZ_A_BYTES);
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const TileCtx c = tile_ctx<G>(P, tile);
+        const TileCtx c = tile_ctx<G>(P, S, tile);
         const int gm = merge_count(c, P, EST);
         PairIter pr;
-        pr.start(P.slices);
+        pr.start(S);
         for (int u = 0; u < c.n_pairs && ok; ++ai) {
           const int g = group_size(pr, gm, c.kchunks);
-          // One accumulator (TMEM columns 0..255) or two (0..127, 128..255,
-          // grouped launches), used in turn; the epilogue frees one as soon
-          // as it has read it.
-          const int buf = Geo::ACC_BUFS == 2 ? (int)(ai & 1) : 0;
-          const uint32_t aph = (Geo::ACC_BUFS == 2 ? ai >> 1 : ai) & 1;
+          // One accumulator (TMEM columns 0..255) or two (0..127, 128..255 in
+          // grouped launches, 0..255, 256..511 in the estimate's first
+          // pass), used in turn; the epilogue frees one as soon as it has
+          // read it.
+          const int buf = two ? (int)(ai & 1) : 0;
+          const uint32_t aph = (two ? ai >> 1 : ai) & 1;
           if (!bounded(&acce[buf], aph ^ 1, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(buf * Geo::BN);
+          uint32_t accum = 0;
           for (int j = 0; j < g && ok; ++j, pr.next(c.kchunks)) {
-            const int kb0 = pr.chunk * (P.kchunk / OZ_BK);
-            int kb1 = kb0 + P.kchunk / OZ_BK;
-            if (kb1 > c.kblocks) kb1 = c.kblocks;
-            for (int kb = kb0; kb < kb1; ++kb, ++it) {
-              const int s = it % Geo::STAGES;
-              const uint32_t ph = (it / Geo::STAGES) & 1;
+            const int kb0 = pr.chunk * chunk_blocks;
+            const int kb1 = kb0 + chunk_blocks < c.kblocks ? kb0 + chunk_blocks : c.kblocks;
+            for (int kb = kb0; kb < kb1; ++kb) {
               if (!bounded(&full[s], ph, 3)) { ok = false; break; }
               tc_fence_after();
-              const uint32_t a_addr = smem_u32(smem + s * Geo::STAGE_BYTES);
-              const uint32_t b_addr = a_addr + OZ_A_BYTES;
+              // (a stage or K step moves the descriptors' 16-byte address field)
+              const uint64_t off = (uint64_t)(s * (Geo::STAGE_BYTES / 16));
 #pragma unroll
               for (int kk = 0; kk < OZ_BK / 16; ++kk) {
-                tc_mma_bf16(d_tmem, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32),
-                            Geo::IDESC, (j > 0 || kb > kb0 || kk > 0) ? 1u : 0u);
+                tc_mma_bf16(d_tmem, adesc0 + off + kk * 2, bdesc0 + off + kk * 2, Geo::IDESC, accum);
+                accum = 1;
               }
               tc_commit(&empty[s]);  // frees the stage once these MMAs have read it
+              if (++s == Geo::STAGES) {
+                s = 0;
+                ph ^= 1;
+              }
             }
           }
           if (!ok) break;
@@ -589,64 +713,52 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     float rmax = 0.0f;
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileCtx tc = tile_ctx<G>(P, tile);
+      const TileCtx tc = tile_ctx<G>(P, S, tile);
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int64_t col0 = tc.col0 + half * (OZ_BN / 2);
-      const float ra = row_ok ? P.ra[row] : 0.0f;
+      const float ra = row_ok ? (float)P.ra[row] : 0.0f;
+      const bool pass1 = P.slices == 1;
       PairIter pr;
-      pr.start(P.slices);
+      pr.start(S);
       for (int u = 0; u < tc.n_pairs; ++u, ++ai, pr.next(1)) {
-        if (!bounded(&accf[0], ai & 1, 4)) { ok = false; break; }
+        const int buf = pass1 ? (int)(ai & 1) : 0;
+        if (!bounded(&accf[buf], (pass1 ? ai >> 1 : ai) & 1, 4)) { ok = false; break; }
         tc_fence_after();
-        uint32_t v[OZ_BN / 2];
-#pragma unroll
-        for (int c = 0; c < OZ_BN / 32; ++c) tmem_ld16_nowait(acc_t + c * 16, v + c * 16);
-        tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[0]);
-        if (pr.d == 1) {
-#pragma unroll
-          for (int c = 0; c < OZ_BN / 32; ++c) {
-            uint32_t w[16];
+#pragma unroll 1
+        for (int c = 0; c < OZ_BN / 32; ++c) {
+          uint32_t v[16], w[16];
+          tmem_ld16_nowait(acc_t + buf * OZ_BN + c * 16, v);
+          if (!pass1 && (pr.d == 0 || pr.s == 1)) tmem_ld16_nowait(dsum_t + c * 16, w);
+          tmem_wait_ld();
+          if (pr.d == 1) {
             if (pr.s == 1) {
-              tmem_ld16(dsum_t + c * 16, w);
 #pragma unroll
               for (int e = 0; e < 16; ++e)
-                w[e] = __float_as_uint(__uint_as_float(w[e]) + __uint_as_float(v[c * 16 + e]));
+                w[e] = __float_as_uint(__uint_as_float(w[e]) + __uint_as_float(v[e]));
+              tmem_st16(dsum_t + c * 16, w);
             } else {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) w[e] = v[c * 16 + e];
+              tmem_st16(dsum_t + c * 16, v);
             }
-            tmem_st16(dsum_t + c * 16, w);
+            continue;
           }
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          continue;
-        }
-#pragma unroll
-        for (int c = 0; c < OZ_BN / 32; ++c) {  // unrolled: v[] stays in registers
-          uint32_t w[16];
-          if (P.slices == 2) tmem_ld16(dsum_t + c * 16, w);  // warp-uniform
-          if (!row_ok) continue;
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const int64_t col = col0 + c * 16 + e;
-            if (col >= tc.n) continue;
-            const float D = __uint_as_float(v[c * 16 + e]);
-            const float num = P.slices == 2 ? __uint_as_float(w[e]) : ra + P.cb[col];
-            float r;
-            if (D > 0.0f) {
-              r = num / D;
-              if (P.slices != 2) r *= 0x1p96f;
-            } else {
-              r = num > 0.0f ? __uint_as_float(0x7f800000u) : 0.0f;
-            }
-            rmax = fmaxf(rmax, r);
+            const float D = __uint_as_float(v[e]);
+            float num, r;
+            if (pass1) num = (ra + (float)(col < tc.n ? P.cb[col] : 0u)) * (0x1p96f * P.sum_unit);
+            else num = __uint_as_float(w[e]);
+            // (the threshold test of the count tolerates the approximate
+            // division's two ulp)
+            r = D > 0.0f ? __fdividef(num, D) : num > 0.0f ? __uint_as_float(0x7f800000u) : 0.0f;
+            if (row_ok && col < tc.n) rmax = fmaxf(rmax, r);
           }
         }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acce[buf]);
       }
     }
     for (int off = 16; off; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
@@ -680,7 +792,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
     const uint32_t dsum_t = lane_base + 2 * BN;  // R
     const uint32_t dig_t = lane_base + 3 * BN;   // digits 0..3
-    const int b = P.digit_bits, S = P.slices, nd = S - 1;
+    const int b = B8 ? 8 : P.digit_bits, nd = S - 1;
     const uint32_t dmask = (1u << b) - 1;
     uint8_t* const slot = reinterpret_cast<uint8_t*>(P.acc) + (size_t)blockIdx.x * (kColPitch * BN) +
                           (size_t)row_in_tile * OZ_DIGIT_BYTES;
@@ -690,13 +802,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint32_t ai = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileCtx tc = tile_ctx<G>(P, tile);
+      const TileCtx tc = tile_ctx<G>(P, S, tile);
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int ncols = (int)(tc.n - tc.col0 < BN ? tc.n - tc.col0 : BN);
       int nch = (ncols - 16 * half + 31) / 32;  // chunks of this warp inside the problem
       if (nch < 0 || tc.row0 + q * 32 >= tc.m) nch = 0;
-      const int ecol_base = row_ok ? tc.ea[row] + P.final_shift : 0;
+      const int ecol_base = row_ok ? tc.ea[row] + final_shift : 0;
       // Column exponents of this warp's columns j = lane, lane + 32 (chunk
       // j / 16, column j % 16): loaded now, used by the retire pass at the
       // end of the tile (their latency hides behind the tile's groups).
@@ -727,41 +839,54 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         // Chunk by chunk: the accumulator and R in flight together, R
         // updated and stored back; the accumulator goes back to the MMA warp
         // after the last chunk is read (the other one is in use meanwhile).
+        // The conditions are uniform and tested per chunk, not per element
+        // (a test per element cost 3,500 of a group's 5,200 cycles).
         const int dig_i = nd - 1 - d;  // digit index of diagonal d + 1
-        const int dsh = 8 * (dig_i & 3);
+        const bool push = diag_start && !tile_first;
+        const int rsh = push ? b : 0;
 #pragma unroll
         for (int i = 0; i < BN / 32; ++i) {
           if (i >= nch) continue;
           const int col_t = (2 * i + half) * 16;
           uint32_t v[16], w[16];
           tmem_ld16_nowait(lane_base + buf * BN + col_t, v);
-          if (!tile_first) tmem_ld16_nowait(dsum_t + col_t, w);
-          tmem_wait_ld();
-          if (tile_first) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) w[e] = (uint32_t)__float2int_rn(__uint_as_float(v[e]));
-          } else if (diag_start) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int32_t r = (int32_t)w[e];
-              const uint32_t dg = (uint32_t)r & dmask;
-              if (dig_i < 8) {
-                dreg[i * 16 + e] = (dsh ? dreg[i * 16 + e] : 0u) | dg << dsh;
-              } else if (row_ok && col_t + e < ncols) {
-                slot[(size_t)(col_t + e) * kColPitch + (dig_i - 8)] = (uint8_t)dg;
-              }
-              w[e] = (uint32_t)((r >> b) + __float2int_rn(__uint_as_float(v[e])));
-            }
-            if (dig_i == 3) tmem_st16(dig_t + col_t, *reinterpret_cast<const uint32_t(*)[16]>(dreg + i * 16));
+          if (!tile_first) {
+            tmem_ld16_nowait(dsum_t + col_t, w);
           } else {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) w[e] = (uint32_t)((int32_t)w[e] + __float2int_rn(__uint_as_float(v[e])));
+            for (int e = 0; e < 16; ++e) w[e] = 0;
           }
+          tmem_wait_ld();
+          if (push) {
+            if (dig_i < 8) {
+              // 8-bit digits enter at the top of the word, so that a word
+              // that is not full is left-aligned
+              if constexpr (B8) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) dreg[i * 16 + e] = __funnelshift_r(dreg[i * 16 + e], w[e], 8);
+              } else {
+                const int dsh = 8 * (dig_i & 3);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) dreg[i * 16 + e] |= (w[e] & dmask) << dsh;
+              }
+            } else if (row_ok) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e)
+                if (col_t + e < ncols) slot[(size_t)(col_t + e) * kColPitch + (dig_i - 8)] = (uint8_t)(w[e] & dmask);
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e) w[e] = (uint32_t)(((int32_t)w[e] >> rsh) + __float2int_rn(__uint_as_float(v[e])));
           tmem_st16(dsum_t + col_t, w);
+          if (push && dig_i == 3) {
+            tmem_st16(dig_t + col_t, *reinterpret_cast<const uint32_t(*)[16]>(dreg + i * 16));
+#pragma unroll
+            for (int e = 0; e < 16; ++e) dreg[i * 16 + e] = 0;
+          }
           // The last group parks the register digit word in TMEM for the
           // retire pass below: digits 4..7 in this accumulator's columns
-          // (held until then), or digits 0..S-2 in 384..511 when S <= 5.
-          if (final_group)
+          // (held until then), or digits 0..S-2 in 384..511 when S < 5.
+          if (final_group && nd != 4)
             tmem_st16(nd > 4 ? lane_base + buf * BN + col_t : dig_t + col_t,
                       *reinterpret_cast<const uint32_t(*)[16]>(dreg + i * 16));
         }
@@ -790,14 +915,25 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           tmem_ld8_nowait(dig_t + col_t, lw);
           if (nd > 4) tmem_ld8_nowait(lane_base + last_buf * BN + col_t, hw);
           tmem_wait_ld();
-          if (!row_ok) continue;
+          if (row_ok) {
+          // digits 0..7 as retire8 takes them: with 8-bit digits the last
+          // word is left-aligned, a full first word follows it
+          uint64_t lo[8];
+          const int fsh = nd >= 8 || !B8 ? 0 : nd > 4 ? 64 - 8 * nd : 32;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            lo[e] = nd > 4 ? (uint64_t)hw[e] << 32 | (uint64_t)lw[e] << fsh : (uint64_t)lw[e] << fsh;
+          }
           const int64_t off = row * tc.ldc + tc.col0 + col_t;
+          const uint8_t* rec = slot + (size_t)col_t * kColPitch;
           if (tc.f32)
-            retire8<true>(w, lw, hw, slot + (size_t)col_t * kColPitch, kColPitch, sm_eb + i * 16 + h8,
-                          ncols - col_t, b, S, ecol_base, tc.C, off, tc.accumulate);
+            retire8<true, B8>(w, lo, rec, kColPitch, sm_eb + i * 16 + h8, ncols - col_t, b, S, ecol_base, tc.C, off,
+                              tc.accumulate);
           else
-            retire8<false>(w, lw, hw, slot + (size_t)col_t * kColPitch, kColPitch, sm_eb + i * 16 + h8,
-                           ncols - col_t, b, S, ecol_base, tc.C, off, tc.accumulate);
+            retire8<false, B8>(w, lo, rec, kColPitch, sm_eb + i * 16 + h8, ncols - col_t, b, S, ecol_base, tc.C, off,
+                               tc.accumulate);
+          }
+          __syncwarp();  // (the loads above are warp-wide)
         }
       }
       tc_fence_before();
@@ -823,7 +959,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + half * (OZ_BN / 2);
     const uint32_t acc_t = lane_base;           // accumulator columns
     const uint32_t dsum_t = lane_base + OZ_BN;  // R
-    const int b = P.digit_bits, S = P.slices, nd = S - 1;
+    const int b = B8 ? 8 : P.digit_bits, nd = S - 1;
     const uint32_t dmask = (1u << b) - 1;
     constexpr size_t pitch = (size_t)OZ_BM * 16;  // record bytes between tile columns
     uint8_t* const slot = reinterpret_cast<uint8_t*>(P.acc) + (size_t)blockIdx.x * (OZ_BM * OZ_BN * 16) +
@@ -831,12 +967,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint32_t ai = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileCtx tc = tile_ctx<G>(P, tile);
+      const TileCtx tc = tile_ctx<G>(P, S, tile);
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int64_t col0 = tc.col0 + half * (OZ_BN / 2);
       const int ncols = (int)(tc.n - col0 < OZ_BN / 2 ? (tc.n - col0 > 0 ? tc.n - col0 : 0) : OZ_BN / 2);
-      const int ecol_base = row_ok ? tc.ea[row] + P.final_shift : 0;
+      const int ecol_base = row_ok ? tc.ea[row] + final_shift : 0;
       const int gm = merge_count(tc, P, false);
       PairIter pr;
       pr.start(S);
@@ -861,29 +997,27 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&acce[0]);
         const int dig_i = nd - 1 - d;  // digit index of diagonal d + 1
+        const bool push = diag_start && !tile_first;
+        const int rsh = push ? b : 0;
 #pragma unroll
         for (int c = 0; c < OZ_BN / 32; ++c) {
           uint32_t w[16];
           if (tile_first) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) w[e] = (uint32_t)__float2int_rn(__uint_as_float(v[c * 16 + e]));
+            for (int e = 0; e < 16; ++e) w[e] = 0;
           } else {
             tmem_ld16(dsum_t + c * 16, w);
-            if (diag_start) {
-              uint8_t* sp = slot + (size_t)(c * 16) * pitch + dig_i;
-              const int nv = row_ok ? ncols - c * 16 : 0;  // columns of this chunk inside the problem
-#pragma unroll
-              for (int e = 0; e < 16; ++e) {
-                const int32_t r = (int32_t)w[e];
-                if (e < nv) sp[(size_t)e * pitch] = (uint8_t)((uint32_t)r & dmask);
-                w[e] = (uint32_t)((r >> b) + __float2int_rn(__uint_as_float(v[c * 16 + e])));
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < 16; ++e)
-                w[e] = (uint32_t)((int32_t)w[e] + __float2int_rn(__uint_as_float(v[c * 16 + e])));
-            }
           }
+          if (push) {
+            uint8_t* sp = slot + (size_t)(c * 16) * pitch + dig_i;
+            const int nv = row_ok ? ncols - c * 16 : 0;  // columns of this chunk inside the problem
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              if (e < nv) sp[(size_t)e * pitch] = (uint8_t)(w[e] & dmask);
+          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            w[e] = (uint32_t)(((int32_t)w[e] >> rsh) + __float2int_rn(__uint_as_float(v[c * 16 + e])));
           tmem_st16(dsum_t + c * 16, w);
         }
         tmem_wait_st();
@@ -896,20 +1030,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 #pragma unroll 1
       for (int c8 = 0; c8 < OZ_BN / 2; c8 += 8) {
         if (c8 >= ncols) break;  // warp-uniform
-        uint32_t w[8], lw[8], hw[8];
+        uint32_t w[8];
+        uint64_t lo[8];
         tmem_ld8_nowait(dsum_t + c8, w);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          uint64_t r = 0;
-          if (row_ok && c8 + e < ncols)
-            r = __ldcg(reinterpret_cast<const unsigned long long*>(slot + (size_t)(c8 + e) * pitch));
-          lw[e] = (uint32_t)r;
-          hw[e] = (uint32_t)(r >> 32);
-        }
+        for (int e = 0; e < 8; ++e)
+          lo[e] = row_ok && c8 + e < ncols
+                      ? __ldcg(reinterpret_cast<const unsigned long long*>(slot + (size_t)(c8 + e) * pitch))
+                      : 0;
         tmem_wait_ld();
-        if (!row_ok) continue;
-        retire8<false>(w, lw, hw, slot + (size_t)c8 * pitch + 8, pitch, tc.eb + col0 + c8, ncols - c8, b, S,
-                       ecol_base, tc.C, row * tc.ldc + col0 + c8, tc.accumulate);
+        if (row_ok) {
+        if (B8 && nd <= 8) {  // left-aligned; bytes the digits do not reach drop out
+#pragma unroll
+          for (int e = 0; e < 8; ++e) lo[e] = nd ? lo[e] << (64 - 8 * nd) : 0;
+        }
+        const uint8_t* rec = slot + (size_t)c8 * pitch + 8;
+        const int64_t off = row * tc.ldc + col0 + c8;
+        if (tc.f32)
+          retire8<true, B8>(w, lo, rec, pitch, tc.eb + col0 + c8, ncols - c8, b, S, ecol_base, tc.C, off,
+                            tc.accumulate);
+        else
+          retire8<false, B8>(w, lo, rec, pitch, tc.eb + col0 + c8, ncols - c8, b, S, ecol_base, tc.C, off,
+                             tc.accumulate);
+        }
+        __syncwarp();  // (the loads above are warp-wide)
       }
     }
   }
@@ -924,81 +1068,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 // ---------------------------------------------------------------------------
 // Scaling exponents and slicing
 // ---------------------------------------------------------------------------
-// frexp-style exponent of max |x| over a row (one warp per row; T double or
-// float, widened exactly). `flag` (may be null) gets bit 0 set when a row
-// holds an Inf or a NaN.
-template <typename T>
-__global__ void row_exponents(const T* __restrict__ A, int64_t m, int64_t k, int64_t lda,
-                              int* __restrict__ ea, uint32_t* __restrict__ flag) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (row >= m) return;
-  uint64_t mx = 0;
-  for (int64_t j = lane; j < k; j += 32) {
-    uint64_t b = (uint64_t)__double_as_longlong((double)A[row * lda + j]) & 0x7FFFFFFFFFFFFFFFULL;
-    mx = b > mx ? b : mx;
-  }
-  for (int off = 16; off; off >>= 1) {
-    uint64_t o = __shfl_xor_sync(0xffffffffu, mx, off);
-    mx = o > mx ? o : mx;
-  }
-  if (lane == 0) {
-    int e = (int)(mx >> 52) - 1022;  // |max| < 2^e
-    if ((mx >> 52) == 0) e = -1021;  // zero or subnormal
-    ea[row] = e;
-    if (flag && (mx >> 52) == 0x7FF) atomicOr(flag, 1u);
-  }
-}
-
-// Column maxima of |B| (k x n row-major) as IEEE bit patterns (ordered like
-// the magnitudes): a 2-D grid of 256-row strips, coalesced across columns,
-// combined with atomicMax on the bit pattern into a zeroed array.
-constexpr int kColStrip = 256;
-template <typename T>
-__global__ void col_max_bits(const T* __restrict__ B, int64_t k, int64_t n, int64_t ldb,
-                             unsigned long long* __restrict__ colmax) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= n) return;
-  const int64_t r0 = (int64_t)blockIdx.y * kColStrip;
-  const int64_t r1 = (r0 + kColStrip) < k ? (r0 + kColStrip) : k;
-  unsigned long long mx = 0;
-  for (int64_t i = r0; i < r1; ++i) {
-    const unsigned long long b =
-        (unsigned long long)__double_as_longlong((double)B[i * ldb + col]) & 0x7FFFFFFFFFFFFFFFULL;
-    mx = b > mx ? b : mx;
-  }
-  atomicMax(&colmax[col], mx);
-}
+constexpr int kColStrip = 256;  // K rows per block of the grouped column maxima
 
 // frexp-style exponent from a max-magnitude bit pattern.
 __global__ void exponents_from_bits(const unsigned long long* __restrict__ mx, int64_t n,
-                                    int* __restrict__ e, uint32_t* __restrict__ flag) {
+                                    int* __restrict__ e) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned long long b = mx[i];
   e[i] = ((b >> 52) == 0) ? -1021 : (int)(b >> 52) - 1022;
-  if (flag && (b >> 52) == 0x7FF) atomicOr(flag, 1u);
 }
 
 // X = round(x * 2^(126 - e)) as a signed 128-bit integer (|x| < 2^e).
-__device__ __forceinline__ __int128 fixed126(double x, int e) {
-  const uint64_t bits = (uint64_t)__double_as_longlong(x);
-  const bool neg = bits >> 63;
-  const int biased = (int)((bits >> 52) & 0x7FF);
-  uint64_t mant = bits & 0xFFFFFFFFFFFFFULL;
+template <typename T>
+__device__ __forceinline__ __int128 fixed126(T x, int e) {
+  bool neg;
+  uint64_t mant;
   int E;
-  if (biased == 0) {
-    E = -1022 - 52;  // subnormal: x = mant * 2^-1074
-  } else {
-    mant |= 1ULL << 52;
-    E = biased - 1023 - 52;  // x = mant * 2^E
-  }
+  ozaki_decode(x, neg, mant, E);  // |x| = mant 2^E
   const int sh = E + 126 - e;
   __int128 X;
   if (mant == 0) {
     X = 0;
   } else if (sh >= 0) {
-    X = (__int128)mant << sh;  // sh <= 73 because |x| < 2^e
+    X = (__int128)mant << sh;  // sh <= 73 because |x| < 2^e (102 for a float)
   } else if (sh > -64) {
     X = (__int128)((mant + (1ULL << (-sh - 1))) >> (-sh));
   } else {
@@ -1033,139 +1126,139 @@ __device__ __forceinline__ uint32_t bf16_of_int(int v) {
   return __float_as_uint((float)v) >> 16;
 }
 
-// A (m x k) -> slices [S][m][kpad], K-major; zero beyond k. A thread takes 8
-// consecutive k of one row (kpad is a multiple of 8; four 16-byte loads when
-// aligned) and writes one 16-byte vector per slice.
-// SMALL (b S <= 64): the same digits from 64-bit arithmetic (ozaki_z64).
-template <int b, bool VEC, bool SMALL>
-__global__ void __launch_bounds__(256)
-    slice_rows(const double* __restrict__ A, int64_t m, int64_t k, int64_t lda, int64_t kpad,
-               const int* __restrict__ ea, int S, uint16_t* __restrict__ out) {
-  const int64_t gpr = kpad / 8;
-  const int64_t total = m * gpr;
-  const unsigned __int128 C = digit_offset(S, b);
-  const uint64_t C64 = ozaki_offset64(S, b);
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = g / gpr, j0 = (g - i * gpr) * 8;
-    const int e = ea[i];
-    double x[8];
-    const double* row = A + i * lda + j0;
-    if (VEC && j0 + 8 <= k) {  // four 16-byte loads
+// ---------------------------------------------------------------------------
+// One problem's operands: exponents, spread-estimate operands, slices
+// ---------------------------------------------------------------------------
+// One operand as the kernels see it: `rows` output rows (m for A, n for B)
+// along K. rows_contig: element (r, kk) at p[r * ld + kk] (A as given, or B
+// passed transposed); otherwise at p[kk * ld + r] (B as given, or A passed
+// transposed), which is read coalesced along r and transposed through shared
+// memory. Each kernel takes both operands in one launch: the first `blocks`
+// blocks work on the first operand.
+//
+// All three kernels stream their operand once and are bound by HBM at large
+// sizes; for small products what counts is that they are three launches
+// instead of eight (512^3: 0.05 ms -> 0.015 ms of the chain before the
+// products).
+template <typename T>
+struct OzPrep {
+  const T* p;
+  int64_t ld, rows;
+  int rows_contig;
+  int vec;            // rows_contig: every row starts 16-byte aligned
+  int strips;         // column layout: K strips of the partial maxima
+  int64_t strip_len;
+  uint32_t* part;     // column layout: [strips][rows] maxima, as abs_bits
+  int* e;             // exponents
+  uint32_t* sums;     // sum_k |x'| in units of 1 / scale
+  uint16_t* out;      // slices (or estimate slices) [S][rows][kpad]
+  unsigned blocks;
+};
+
+// The bits of |x| that decide its exponent, ordered like |x| up to equal
+// exponents: the high word of a double, all of a float.
+__device__ __forceinline__ uint32_t abs_bits(double x) { return (uint32_t)__double2hiint(x) & 0x7FFFFFFFu; }
+__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+// frexp-style exponent (|x| < 2^e) of a maximum's abs_bits; a double that is
+// zero or subnormal gives -1021, Inf / NaN the value kNonFinite.
+template <typename T>
+__device__ __forceinline__ int exp_of_bits(uint32_t m) {
+  if constexpr (sizeof(T) == 8) {
+    const int be = (int)(m >> 20);
+    return be == 0 ? -1021 : be - 1022;
+  } else {
+    const int be = (int)(m >> 23);
+    if (be == 0) return m == 0 ? -1021 : -116 - __clz((int)m);  // 2^(31 - clz) 2^-149 <= |x|
+    return be - 126;
+  }
+}
+template <typename T>
+constexpr int kNonFinite = sizeof(T) == 8 ? 1025 : 129;
+
+// 16 bytes of T (8 doubles' worth of slots are filled by several calls).
+template <typename T, int N>
+__device__ __forceinline__ void load_run(const T* src, bool vec, int64_t left, T (&x)[N]) {
+  constexpr int PER = 16 / (int)sizeof(T);
+  if (vec && left >= N) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double2 d2 = reinterpret_cast<const double2*>(row)[q];
-        x[2 * q] = d2.x;
-        x[2 * q + 1] = d2.y;
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 8; ++q) x[q] = j0 + q < k ? row[q] : 0.0;
+    for (int q = 0; q < N / PER; ++q) {
+      const uint4 u = reinterpret_cast<const uint4*>(src)[q];
+      memcpy(&x[q * PER], &u, 16);
     }
-    // The eight offset values, then one slice at a time (one 16-byte store
-    // each), so only the current slice's packed words are live.
-    uint16_t* o = out + i * kpad + j0;
-    if constexpr (SMALL) {
-      OzakiZ64 Z[8];
+  } else {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) Z[q] = ozaki_z64(x[q], e, b, S, C64);
-#pragma unroll
-      for (int t = 0; t < OZ_MAX_SLICES; ++t) {
-        if (t < S) {
-          uint32_t pk[4];
-#pragma unroll
-          for (int h = 0; h < 4; ++h)
-            pk[h] = bf16_of_int(ozaki_digit64<b>(Z[2 * h], t)) |
-                    (bf16_of_int(ozaki_digit64<b>(Z[2 * h + 1], t)) << 16);
-          *reinterpret_cast<uint4*>(o + (int64_t)t * m * kpad) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        }
-      }
-    } else {
-      unsigned __int128 Z[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) Z[q] = (unsigned __int128)fixed126(x[q], e) + C;
-#pragma unroll
-      for (int t = 0; t < OZ_MAX_SLICES; ++t) {
-        if (t < S) {
-          uint32_t pk[4];
-#pragma unroll
-          for (int h = 0; h < 4; ++h)
-            pk[h] = bf16_of_int(digit_at<b>(Z[2 * h], t)) | (bf16_of_int(digit_at<b>(Z[2 * h + 1], t)) << 16);
-          *reinterpret_cast<uint4*>(o + (int64_t)t * m * kpad) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        }
-      }
-    }
+    for (int q = 0; q < N; ++q) x[q] = q < left ? src[q] : T(0);
   }
 }
 
-// B (k x n row-major) -> slices of B^T [S][n][kpad]. A block takes 64 k x 32 n:
-// thread (nn = tid % 32, kk pair) reads B coalesced along n, packs the digits
-// of two consecutive k into one 32-bit word of a shared tile [S][32 n][33
-// words] (the pad word keeps both phases free of bank conflicts), then every
-// thread writes one 16-byte vector (8 k of one n row) per slice.
+// Exponents of contiguous rows; per-strip maxima of columns. Also zeroes
+// the decision words and the column sums that oz_est adds into.
+template <typename T>
+__global__ void __launch_bounds__(256) oz_max(OzPrep<T> a, OzPrep<T> bT, int64_t k, uint32_t* __restrict__ words) {
+  if (blockIdx.x == 0 && threadIdx.x < OZ_WORDS) words[threadIdx.x] = 0;
+  const bool first = blockIdx.x < a.blocks;
+  const OzPrep<T>& o = first ? a : bT;
+  const int64_t blk = first ? blockIdx.x : blockIdx.x - a.blocks;
+  if (o.rows_contig) {
+    const int64_t row = blk * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (row >= o.rows) return;
+    const T* xr = o.p + row * o.ld;
+    uint32_t mx = 0;
+#pragma unroll 2
+    for (int64_t j = lane * 8; j < k; j += 256) {
+      T x[8];
+      load_run(xr + j, o.vec, k - j, x);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) mx = max(mx, abs_bits(x[q]));
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) o.e[row] = exp_of_bits<T>(mx);
+  } else {
+    const int64_t nx = (o.rows + 255) / 256;
+    const int64_t strip = blk / nx, col = (blk - strip * nx) * 256 + threadIdx.x;
+    if (col >= o.rows) return;
+    const int64_t r0 = strip * o.strip_len;
+    const int64_t r1 = r0 + o.strip_len < k ? r0 + o.strip_len : k;
+    uint32_t mx = 0;
+#pragma unroll 8
+    for (int64_t i = r0; i < r1; ++i) mx = max(mx, abs_bits(o.p[i * o.ld + col]));
+    o.part[strip * o.rows + col] = mx;
+    if (strip == 0 && o.sums) o.sums[col] = 0;
+  }
+}
+
 constexpr int kSliceColK = 64, kSliceColN = 32, kSliceColPitch = kSliceColK / 2 + 1;
-template <int b, bool SMALL>
-__global__ void __launch_bounds__(256)
-    slice_cols(const double* __restrict__ B, int64_t k, int64_t n, int64_t ldb, int64_t kpad,
-               const int* __restrict__ eb, int S, uint16_t* __restrict__ out) {
-  extern __shared__ uint32_t tile[];  // [S][32][33]
-  const int64_t k0 = (int64_t)blockIdx.y * kSliceColK, n0 = (int64_t)blockIdx.x * kSliceColN;
+
+// The exponents of a block's 32 columns from the strip maxima (a whole block
+// of 256 threads); thread `ty * 32 + tx` returns column n0 + tx's. The
+// blocks of the first K tile also store them.
+template <typename T>
+__device__ __forceinline__ int block_col_exps(const OzPrep<T>& o, int64_t n0, bool store, uint32_t (&sh)[8][32]) {
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const unsigned __int128 C = digit_offset(S, b);
-  const uint64_t C64 = ozaki_offset64(S, b);
-  {
-    const int64_t nn = n0 + tx;
-    const int e = nn < n ? eb[nn] : 0;
-#pragma unroll
-    for (int r = 0; r < kSliceColK / 16; ++r) {  // word column w = ty + 8r: k rows 2w, 2w+1
-      const int w = ty + 8 * r;
-      const int64_t kk = k0 + 2 * w;
-      const double x0 = kk < k && nn < n ? B[kk * ldb + nn] : 0.0;
-      const double x1 = kk + 1 < k && nn < n ? B[(kk + 1) * ldb + nn] : 0.0;
-      if constexpr (SMALL) {
-        const OzakiZ64 Z0 = ozaki_z64(x0, e, b, S, C64), Z1 = ozaki_z64(x1, e, b, S, C64);
-#pragma unroll
-        for (int t = 0; t < OZ_MAX_SLICES; ++t)
-          if (t < S)
-            tile[(t * kSliceColN + tx) * kSliceColPitch + w] =
-                bf16_of_int(ozaki_digit64<b>(Z0, t)) | (bf16_of_int(ozaki_digit64<b>(Z1, t)) << 16);
-      } else {
-        const unsigned __int128 Z0 = (unsigned __int128)fixed126(x0, e) + C;
-        const unsigned __int128 Z1 = (unsigned __int128)fixed126(x1, e) + C;
-#pragma unroll
-        for (int t = 0; t < OZ_MAX_SLICES; ++t)
-          if (t < S)
-            tile[(t * kSliceColN + tx) * kSliceColPitch + w] =
-                bf16_of_int(digit_at<b>(Z0, t)) | (bf16_of_int(digit_at<b>(Z1, t)) << 16);
-      }
-    }
-  }
+  const int64_t nn = n0 + tx;
+  uint32_t mx = 0;
+  if (nn < o.rows)
+    for (int s = ty; s < o.strips; s += 8) mx = max(mx, o.part[(int64_t)s * o.rows + nn]);
+  sh[ty][tx] = mx;
   __syncthreads();
-  const int r = threadIdx.x >> 3, c = threadIdx.x & 7;  // n row, 16-byte chunk (8 k)
-  const int64_t nn = n0 + r, kk = k0 + c * 8;
-  if (nn < n && kk < kpad) {
-    for (int t = 0; t < S; ++t) {
-      const uint32_t* src = tile + (t * kSliceColN + r) * kSliceColPitch + c * 4;
-      *reinterpret_cast<uint4*>(out + (int64_t)t * n * kpad + nn * kpad + kk) =
-          make_uint4(src[0], src[1], src[2], src[3]);
-    }
-  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) mx = max(mx, sh[q][tx]);
+  const int e = exp_of_bits<T>(mx);
+  if (store && ty == 0 && nn < o.rows) o.e[nn] = e;
+  return e;
 }
 
 // ---------------------------------------------------------------------------
 // Spread estimate operands
 // ---------------------------------------------------------------------------
-// For the automatic slice count the operands are also written as two BF16
-// "slices": slice 0 = |x'| 2^48 (x' = x 2^-e, so |x'| < 1; rounded to
-// nearest) and slice 1 = 2^48 where x != 0, else 0. The 2^48 factors keep
-// products of small |x'| above FP32's underflow threshold while every sum
-// over K stays below 2^96 * 2^31 < 2^128. Row sums of |x'| (fp32, fixed
-// order) give the pass-1 numerator.
+// For a slice count that follows the operands' spread they are also written
+// as two BF16 "slices": slice 0 = |x'| 2^48 (x' = x 2^-e, so |x'| < 1;
+// rounded to nearest) and, for the second pass only, slice 1 = 2^48 where
+// x != 0, else 0. The 2^48 factors keep products of small |x'| above FP32's
+// underflow threshold while every sum over K stays below 2^96 * 2^31 <
+// 2^128. Row sums of |x'| (fixed point) give the pass-1 numerator.
 constexpr uint32_t kBf16Two48 = 0x5780u;  // 2^48 in BF16
-
-__device__ __forceinline__ bool nonzero(double x) {
-  return ((uint64_t)__double_as_longlong(x) << 1) != 0;  // integer test, +-0 excluded
-}
 
 // |x| 2^-e from the bit pattern alone (no FP64 arithmetic: GB300's FP64 pipe
 // is slow): *f = |x'| as fp32 (mantissa truncated), return value = |x'| 2^48
@@ -1187,104 +1280,246 @@ __device__ __forceinline__ uint32_t est_bits(double x, int e, float* f) {
   if (rem > half || (rem == half && (h & 1u))) ++h;
   return h;
 }
-
-// X (rows x k, row pitch ld, contiguous along k) -> out [2][rows][kpad],
-// sums[row] = sum_k |x'|. One warp per row, 8 consecutive k per lane step.
-template <bool VEC, typename T>
-__global__ void __launch_bounds__(256)
-    est_rows(const T* __restrict__ X, int64_t rows, int64_t k, int64_t ld, int64_t kpad,
-             const int* __restrict__ e, uint16_t* __restrict__ out, float* __restrict__ sums) {
-  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const int er = e[row];
-  const T* xr = X + row * ld;
-  float s = 0.0f;
-  for (int64_t j0 = (int64_t)lane * 8; j0 < kpad; j0 += 256) {
-    double x[8];
-    if (VEC && j0 + 8 <= k) {  // (T = double only)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double2 d2 = reinterpret_cast<const double2*>(xr + j0)[q];
-        x[2 * q] = d2.x;
-        x[2 * q + 1] = d2.y;
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 8; ++q) x[q] = j0 + q < k ? (double)xr[j0 + q] : 0.0;
-    }
-    uint32_t pa[4], pi[4];
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      float f0, f1;
-      const uint32_t b0 = est_bits(x[2 * h], er, &f0), b1 = est_bits(x[2 * h + 1], er, &f1);
-      s += f0;
-      s += f1;
-      pa[h] = b0 | (b1 << 16);
-      pi[h] = (nonzero(x[2 * h]) ? kBf16Two48 : 0u) | ((nonzero(x[2 * h + 1]) ? kBf16Two48 : 0u) << 16);
-    }
-    uint16_t* o = out + row * kpad + j0;
-    *reinterpret_cast<uint4*>(o) = make_uint4(pa[0], pa[1], pa[2], pa[3]);
-    *reinterpret_cast<uint4*>(o + rows * kpad) = make_uint4(pi[0], pi[1], pi[2], pi[3]);
+__device__ __forceinline__ uint32_t est_bits(float x, int e, float* f) {
+  const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
+  const int be = (int)(u >> 23);
+  const uint32_t mant = u & 0x7FFFFFu;
+  const int fe = be - 127 - e;
+  if (be == 0) {
+    *f = 0.0f;
+    return 0u;
   }
-  for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) sums[row] = s;
+  *f = (fe + 127 >= 1) ? __uint_as_float(((uint32_t)(fe + 127) << 23) | mant) : 0.0f;
+  if (fe + 48 + 127 < 1) return 0u;
+  uint32_t h = ((uint32_t)(fe + 48 + 127) << 7) | (mant >> 16);
+  const uint32_t rem = mant & 0xFFFFu;
+  if (rem > 0x8000u || (rem == 0x8000u && (h & 1u))) ++h;
+  return h;
+}
+// 2^48 in BF16 where x is not +-0 (an integer test)
+__device__ __forceinline__ uint32_t two48_if(double x) {
+  return ((uint64_t)__double_as_longlong(x) << 1) != 0 ? kBf16Two48 : 0u;
+}
+__device__ __forceinline__ uint32_t two48_if(float x) { return x != 0.0f ? kBf16Two48 : 0u; }
+// Raises a word to at least v; most callers find it there already.
+__device__ __forceinline__ void raise_word(uint32_t* w, uint32_t v) {
+  if (__ldcg(w) < v) atomicMax(w, v);
 }
 
-// X (k x cols row-major) -> out [2][cols][kpad] (transposed through shared
-// memory like slice_cols), part[strip][col] = sum of |x'| over the block's
-// 64 k; est_strip_sums adds the strips in order (deterministic).
-template <typename T>
+// Both operands' estimate slices, sums and exponent maxima. `kside`: the
+// decision word of the operand's exponent maximum.
+template <typename T, bool PASS2>
 __global__ void __launch_bounds__(256)
-    est_cols(const T* __restrict__ X, int64_t k, int64_t cols, int64_t ld, int64_t kpad,
-             const int* __restrict__ e, uint16_t* __restrict__ out, float* __restrict__ part) {
-  __shared__ uint32_t tile[2][kSliceColN][kSliceColPitch];
+    oz_est(OzPrep<T> a, OzPrep<T> bT, int64_t k, int64_t kpad, float scale, uint32_t* __restrict__ words) {
+  __shared__ uint32_t tile[PASS2 ? 2 : 1][kSliceColN][kSliceColPitch];
   __shared__ float csum[8][kSliceColN];
-  const int64_t k0 = (int64_t)blockIdx.y * kSliceColK, n0 = (int64_t)blockIdx.x * kSliceColN;
+  __shared__ uint32_t cexp[8][32];
+  const bool first = blockIdx.x < a.blocks;
+  const OzPrep<T>& o = first ? a : bT;
+  const int64_t blk = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const int word = first ? OZ_W_EXP_A : OZ_W_EXP_B;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if (o.rows_contig) {
+    const int64_t row = blk * 8 + ty;
+    if (row >= o.rows) return;
+    const int er = o.e[row];
+    const T* xr = o.p + row * o.ld;
+    float s = 0.0f;
+    for (int64_t j0 = (int64_t)tx * 8; j0 < kpad; j0 += 256) {
+      T x[8];
+      load_run(xr + j0, o.vec, k - j0, x);
+      uint32_t pa[4], pi[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        float f0, f1;
+        const uint32_t b0 = est_bits(x[2 * h], er, &f0), b1 = est_bits(x[2 * h + 1], er, &f1);
+        s += f0;
+        s += f1;
+        pa[h] = b0 | (b1 << 16);
+        pi[h] = two48_if(x[2 * h]) | (two48_if(x[2 * h + 1]) << 16);
+      }
+      uint16_t* q = o.out + row * kpad + j0;
+      *reinterpret_cast<uint4*>(q) = make_uint4(pa[0], pa[1], pa[2], pa[3]);
+      if (PASS2) *reinterpret_cast<uint4*>(q + o.rows * kpad) = make_uint4(pi[0], pi[1], pi[2], pi[3]);
+    }
+    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (tx == 0) {
+      o.sums[row] = __float2uint_ru(s * scale);
+      raise_word(&words[word], (uint32_t)(er + kExpBias));
+      if (er == kNonFinite<T>) words[OZ_W_NONFINITE] = 1;
+    }
+    return;
+  }
+  // 64 k x 32 columns, transposed through shared memory (the pad word of a
+  // tile row keeps both phases free of bank conflicts)
+  const int64_t nx = (o.rows + kSliceColN - 1) / kSliceColN;
+  const int64_t ky = blk / nx, n0 = (blk - ky * nx) * kSliceColN, k0 = ky * kSliceColK;
   const int64_t nn = n0 + tx;
-  const int ec = nn < cols ? e[nn] : 0;
+  T x0[kSliceColK / 16], x1[kSliceColK / 16];
+#pragma unroll
+  for (int r = 0; r < kSliceColK / 16; ++r) {  // word column w = ty + 8r: k rows 2w, 2w+1
+    const int64_t kk = k0 + 2 * (ty + 8 * r);
+    x0[r] = kk < k && nn < o.rows ? o.p[kk * o.ld + nn] : T(0);
+    x1[r] = kk + 1 < k && nn < o.rows ? o.p[(kk + 1) * o.ld + nn] : T(0);
+  }
+  const int ec = block_col_exps(o, n0, ky == 0, cexp);
   float s = 0.0f;
 #pragma unroll
   for (int r = 0; r < kSliceColK / 16; ++r) {
     const int w = ty + 8 * r;
-    const int64_t kk = k0 + 2 * w;
-    const double x0 = kk < k && nn < cols ? (double)X[kk * ld + nn] : 0.0;
-    const double x1 = kk + 1 < k && nn < cols ? (double)X[(kk + 1) * ld + nn] : 0.0;
     float f0, f1;
-    const uint32_t b0 = est_bits(x0, ec, &f0), b1 = est_bits(x1, ec, &f1);
+    const uint32_t b0 = est_bits(x0[r], ec, &f0), b1 = est_bits(x1[r], ec, &f1);
     s += f0;
     s += f1;
     tile[0][tx][w] = b0 | (b1 << 16);
-    tile[1][tx][w] = (nonzero(x0) ? kBf16Two48 : 0u) | ((nonzero(x1) ? kBf16Two48 : 0u) << 16);
+    if (PASS2) tile[PASS2 ? 1 : 0][tx][w] = two48_if(x0[r]) | (two48_if(x1[r]) << 16);
   }
   csum[ty][tx] = s;
   __syncthreads();
-  if (ty == 0 && nn < cols) {
+  if (ty == 0 && nn < o.rows) {
     float t = 0.0f;
 #pragma unroll
     for (int q = 0; q < 8; ++q) t += csum[q][tx];
-    part[(int64_t)blockIdx.y * cols + nn] = t;
+    atomicAdd(&o.sums[nn], __float2uint_ru(t * scale));  // (integers: any order)
+    if (ky == 0) {
+      raise_word(&words[word], (uint32_t)(ec + kExpBias));
+      if (ec == kNonFinite<T>) words[OZ_W_NONFINITE] = 1;
+    }
   }
   const int r = threadIdx.x >> 3, c = threadIdx.x & 7;
   const int64_t n2 = n0 + r, k2 = k0 + c * 8;
-  if (n2 < cols && k2 < kpad) {
+  if (n2 < o.rows && k2 < kpad) {
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
+    for (int t = 0; t < (PASS2 ? 2 : 1); ++t) {
       const uint32_t* src = &tile[t][r][c * 4];
-      *reinterpret_cast<uint4*>(out + (int64_t)t * cols * kpad + n2 * kpad + k2) =
+      *reinterpret_cast<uint4*>(o.out + (int64_t)t * o.rows * kpad + n2 * kpad + k2) =
           make_uint4(src[0], src[1], src[2], src[3]);
     }
   }
 }
 
-__global__ void est_strip_sums(const float* __restrict__ part, int64_t strips, int64_t cols,
-                               float* __restrict__ sums) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float t = 0.0f;
-  for (int64_t s = 0; s < strips; ++s) t += part[s * cols + c];
-  sums[c] = t;
+// The digits of N values at slice t: 64-bit arithmetic when b S <= 64, else
+// 128-bit (the same digits).
+template <int b, int N>
+struct OzDigits64 {
+  OzakiZ64 z[N];
+  template <typename T>
+  __device__ __forceinline__ void set(int i, T x, int e, int S, uint64_t off) { z[i] = ozaki_z64(x, e, b, S, off); }
+  __device__ __forceinline__ uint32_t pair(int i, int t) const {
+    return bf16_of_int(ozaki_digit64<b>(z[i], t)) | (bf16_of_int(ozaki_digit64<b>(z[i + 1], t)) << 16);
+  }
+};
+template <int b, int N>
+struct OzDigits128 {
+  unsigned __int128 z[N];
+  template <typename T>
+  __device__ __forceinline__ void set(int i, T x, int e, int S, unsigned __int128 off) {
+    z[i] = (unsigned __int128)fixed126(x, e) + off;
+  }
+  __device__ __forceinline__ uint32_t pair(int i, int t) const {
+    return bf16_of_int(digit_at<b>(z[i], t)) | (bf16_of_int(digit_at<b>(z[i + 1], t)) << 16);
+  }
+};
+
+// 8 consecutive k of one row -> one 16-byte vector per slice, one slice at a
+// time so that only the current slice's packed words are live.
+template <typename D, typename T, typename O>
+__device__ __forceinline__ void slice_run8(const T (&x)[8], int e, int S, O off, uint16_t* out, int64_t plane) {
+  D d;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) d.set(q, x[q], e, S, off);
+#pragma unroll
+  for (int t = 0; t < OZ_MAX_SLICES; ++t)
+    if (t < S)
+      *reinterpret_cast<uint4*>(out + (int64_t)t * plane) =
+          make_uint4(d.pair(0, t), d.pair(2, t), d.pair(4, t), d.pair(6, t));
+}
+
+// 64 k x 32 columns: thread (tx, ty) holds the k pairs 2 (ty + 8 r), packs
+// two digits of a column into one word of a shared tile per slice, and every
+// thread writes one 16-byte vector (8 k of one column) per slice; kSliceSet
+// slices at a time share the tile.
+constexpr int kSliceSet = 8;
+template <typename D, typename T, typename O>
+__device__ __forceinline__ void slice_tile(const T (&x0)[4], const T (&x1)[4], int e, int S, O off, uint32_t* tile,
+                                           uint16_t* out, int64_t rows, int64_t kpad, int64_t n0, int64_t k0) {
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  D d;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    d.set(2 * r, x0[r], e, S, off);
+    d.set(2 * r + 1, x1[r], e, S, off);
+  }
+  const int rr = threadIdx.x >> 3, c = threadIdx.x & 7;  // column, 16-byte chunk (8 k)
+  const int64_t nn = n0 + rr, kk = k0 + c * 8;
+#pragma unroll
+  for (int t0 = 0; t0 < OZ_MAX_SLICES; t0 += kSliceSet) {
+    if (t0 >= S) break;
+    if (t0) __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int t = t0; t < t0 + kSliceSet; ++t)
+        if (t < S) tile[((t - t0) * kSliceColN + tx) * kSliceColPitch + ty + 8 * r] = d.pair(2 * r, t);
+    __syncthreads();
+    if (nn < rows && kk < kpad) {
+#pragma unroll
+      for (int t = 0; t < kSliceSet; ++t) {
+        if (t0 + t >= S) break;
+        const uint32_t* src = tile + (t * kSliceColN + rr) * kSliceColPitch + c * 4;
+        *reinterpret_cast<uint4*>(out + (int64_t)(t0 + t) * rows * kpad + nn * kpad + kk) =
+            make_uint4(src[0], src[1], src[2], src[3]);
+      }
+    }
+  }
+}
+
+// Both operands -> slices [S][rows][kpad], K-major, zero beyond k. S as
+// given, or decided on the device (0: nothing to do).
+template <typename T, int b>
+__global__ void __launch_bounds__(256)
+    oz_slice(OzPrep<T> a, OzPrep<T> bT, int64_t k, int64_t kpad, int S_given, uint32_t* decide, OzRule rule) {
+  __shared__ uint32_t tile[kSliceSet * kSliceColN * kSliceColPitch];
+  __shared__ uint32_t cexp[8][32];
+  const int S = decide ? oz_decide(decide, rule) : S_given;
+  if (decide && blockIdx.x == 0 && threadIdx.x == 0) decide[OZ_W_COUNT] = (uint32_t)S;
+  if (S == 0) return;
+  const bool first = blockIdx.x < a.blocks;
+  const OzPrep<T>& o = first ? a : bT;
+  const int64_t blk = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const bool small = b * S <= 64;
+  const uint64_t c64 = small ? ozaki_offset64(S, b) : 0;
+  const unsigned __int128 c128 = small ? 0 : digit_offset(S, b);
+  if (o.rows_contig) {
+    const int64_t gpr = kpad / 8, total = o.rows * gpr, plane = o.rows * kpad;
+    for (int64_t g = blk * 256 + threadIdx.x; g < total; g += (int64_t)o.blocks * 256) {
+      const int64_t i = g / gpr, j0 = (g - i * gpr) * 8;
+      T x[8];
+      load_run(o.p + i * o.ld + j0, o.vec, k - j0, x);
+      uint16_t* out = o.out + i * kpad + j0;
+      if (small)
+        slice_run8<OzDigits64<b, 8>>(x, o.e[i], S, c64, out, plane);
+      else
+        slice_run8<OzDigits128<b, 8>>(x, o.e[i], S, c128, out, plane);
+    }
+    return;
+  }
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t nx = (o.rows + kSliceColN - 1) / kSliceColN;
+  const int64_t ky = blk / nx, n0 = (blk - ky * nx) * kSliceColN, k0 = ky * kSliceColK;
+  const int64_t nn = n0 + tx;
+  T x0[4], x1[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int64_t kk = k0 + 2 * (ty + 8 * r);
+    x0[r] = kk < k && nn < o.rows ? o.p[kk * o.ld + nn] : T(0);
+    x1[r] = kk + 1 < k && nn < o.rows ? o.p[(kk + 1) * o.ld + nn] : T(0);
+  }
+  const int e = block_col_exps(o, n0, ky == 0, cexp);
+  if (small)
+    slice_tile<OzDigits64<b, 8>>(x0, x1, e, S, c64, tile, o.out, o.rows, kpad, n0, k0);
+  else
+    slice_tile<OzDigits128<b, 8>>(x0, x1, e, S, c128, tile, o.out, o.rows, kpad, n0, k0);
 }
 
 bool make_slice_map(CUtensorMap* map, const void* base, int64_t kpad, int64_t rows, int S,
@@ -1304,121 +1539,153 @@ bool make_slice_map(CUtensorMap* map, const void* base, int64_t kpad, int64_t ro
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
-// One operand as the kernels see it: `rows` output rows (m for A, n for B)
-// along K. rows_contig: element (r, kk) at p[r * ld + kk] (A as given, or B
-// passed transposed); otherwise at p[kk * ld + r] (B as given, or A passed
-// transposed), which the column kernels read coalesced and transpose.
 struct OzOperand {
-  const void* p;  // double, or float when f32 (the spread estimate only)
+  const void* p;  // double or float
   int64_t ld;
   int64_t rows;
   bool rows_contig;
-  bool f32 = false;
-  const double* d() const { return static_cast<const double*>(p); }
-  const float* f() const { return static_cast<const float*>(p); }
 };
 
-int launch_exponents(nrs_handle* h, const OzOperand& o, int64_t k, int* e,
-                     unsigned long long* colmax, uint32_t* flag) {
-  cudaStream_t s = h->stream;
-  if (o.rows_contig) {
-    if (o.f32)
-      row_exponents<float><<<(unsigned)((o.rows + 7) / 8), 256, 0, s>>>(o.f(), o.rows, k, o.ld, e, flag);
-    else
-      row_exponents<double><<<(unsigned)((o.rows + 7) / 8), 256, 0, s>>>(o.d(), o.rows, k, o.ld, e, flag);
-  } else {
-    int st = nrs_cuda_check(h, cudaMemsetAsync(colmax, 0, (size_t)o.rows * 8, s), "cudaMemsetAsync");
-    if (st) return st;
-    const dim3 grid((unsigned)((o.rows + 255) / 256), (unsigned)((k + kColStrip - 1) / kColStrip));
-    if (o.f32)
-      col_max_bits<float><<<grid, 256, 0, s>>>(o.f(), k, o.rows, o.ld, colmax);
-    else
-      col_max_bits<double><<<grid, 256, 0, s>>>(o.d(), k, o.rows, o.ld, colmax);
-    exponents_from_bits<<<(unsigned)((o.rows + 255) / 256), 256, 0, s>>>(colmax, o.rows, e, flag);
-  }
-  return nrs_after_launch(h, "ozaki exponents");
+// Device buffers of one problem, carved from one block of scratch memory:
+// exponents | sums | strip maxima | decision words, then an area that holds
+// the estimate operands first and the slices after the estimate product.
+struct OzScratch {
+  int *ea, *eb;
+  uint32_t *ra, *cb;
+  uint32_t *part_a, *part_b;
+  uint32_t* words;
+  uint16_t* area_a;
+  uint16_t* area_b;
+  uint8_t* tail;  // `tail_bytes` behind the areas
+};
+constexpr int kMaxStrips = 32;
+inline size_t oz_al(size_t v) { return (v + 1023) & ~size_t(1023); }
+// `planes`: BF16 planes per operand that the areas hold.
+size_t oz_scratch(int64_t m, int64_t n, int64_t kpad, int planes, size_t tail_bytes, uint8_t* base, OzScratch* o) {
+  const size_t mb = oz_al((size_t)m * 4), nb = oz_al((size_t)n * 4);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    uint8_t* q = base + off;
+    off += bytes;
+    return q;
+  };
+  OzScratch r;
+  r.ea = (int*)take(mb);
+  r.eb = (int*)take(nb);
+  r.ra = (uint32_t*)take(mb);
+  r.cb = (uint32_t*)take(nb);
+  r.part_a = (uint32_t*)take(oz_al((size_t)kMaxStrips * m * 4));
+  r.part_b = (uint32_t*)take(oz_al((size_t)kMaxStrips * n * 4));
+  r.words = (uint32_t*)take(1024);
+  r.area_a = (uint16_t*)take(oz_al((size_t)planes * m * kpad * 2));
+  r.area_b = (uint16_t*)take(oz_al((size_t)planes * n * kpad * 2));
+  r.tail = take(oz_al(tail_bytes));
+  if (o) *o = r;
+  return off;
 }
 
-template <int b, bool SMALL>
-int launch_slices_bs(nrs_handle* h, const OzOperand& o, int64_t k, int64_t kpad, const int* e, int S,
-                     uint16_t* out) {
-  cudaStream_t s = h->stream;
-  if (o.rows_contig) {
-    const int64_t groups = o.rows * (kpad / 8);
-    const int grid = (int)std::min<int64_t>((groups + 255) / 256, (int64_t)h->num_sms * 8);
-    // 16-byte row loads when every row start is 16-byte aligned.
-    if (((reinterpret_cast<uintptr_t>(o.p) & 15) == 0) && (o.ld % 2 == 0))
-      slice_rows<b, true, SMALL><<<grid, 256, 0, s>>>(o.d(), o.rows, k, o.ld, kpad, e, S, out);
-    else
-      slice_rows<b, false, SMALL><<<grid, 256, 0, s>>>(o.d(), o.rows, k, o.ld, kpad, e, S, out);
-  } else {
-    const int smem = (int)((size_t)S * kSliceColN * kSliceColPitch * 4);
-    int st = nrs_cuda_check(h,
-                            cudaFuncSetAttribute(slice_cols<b, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem),
-                            "cudaFuncSetAttribute(slice_cols)");
-    if (st) return st;
-    dim3 g((unsigned)((o.rows + kSliceColN - 1) / kSliceColN), (unsigned)((kpad + kSliceColK - 1) / kSliceColK));
-    slice_cols<b, SMALL><<<g, 256, smem, s>>>(o.d(), k, o.rows, o.ld, kpad, e, S, out);
-  }
-  return nrs_after_launch(h, "ozaki slicing");
-}
-// b S <= 64: the 64-bit digit path (the same digits, fewer integer operations)
-template <int b>
-int launch_slices_b(nrs_handle* h, const OzOperand& o, int64_t k, int64_t kpad, const int* e, int S,
-                    uint16_t* out) {
-  return b * S <= 64 ? launch_slices_bs<b, true>(h, o, k, kpad, e, S, out)
-                     : launch_slices_bs<b, false>(h, o, k, kpad, e, S, out);
+template <typename T>
+OzPrep<T> oz_prep(const OzOperand& o, int64_t k, int* e, uint32_t* part, uint32_t* sums, uint16_t* out) {
+  OzPrep<T> q{};
+  q.p = static_cast<const T*>(o.p);
+  q.ld = o.ld;
+  q.rows = o.rows;
+  q.rows_contig = o.rows_contig ? 1 : 0;
+  q.vec = (reinterpret_cast<uintptr_t>(o.p) & 15) == 0 && (o.ld * sizeof(T)) % 16 == 0;
+  // at least 32 K rows per strip, so that small operands still fill the GPU
+  q.strips = (int)std::min<int64_t>(kMaxStrips, (k + 31) / 32);
+  q.strip_len = (k + q.strips - 1) / q.strips;
+  q.part = part;
+  q.e = e;
+  q.sums = sums;
+  q.out = out;
+  return q;
 }
 
-int launch_slices(nrs_handle* h, const OzOperand& o, int64_t k, int64_t kpad, const int* e, int b, int S,
-                  uint16_t* out) {
-  return b == 8 ? launch_slices_b<8>(h, o, k, kpad, e, S, out)
-                : b == 7 ? launch_slices_b<7>(h, o, k, kpad, e, S, out)
-                         : launch_slices_b<6>(h, o, k, kpad, e, S, out);
+// Exponents (columns: strip maxima) of both operands; zeroes the words.
+template <typename T>
+int launch_oz_max(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t k, const OzScratch& w) {
+  auto blocks = [](const OzPrep<T>& q) {
+    return (unsigned)(q.rows_contig ? (q.rows + 7) / 8 : (q.rows + 255) / 256 * q.strips);
+  };
+  OzPrep<T> qa = oz_prep<T>(a, k, w.ea, w.part_a, w.ra, w.area_a), qb = oz_prep<T>(bT, k, w.eb, w.part_b, w.cb, w.area_b);
+  qa.blocks = blocks(qa);
+  qb.blocks = blocks(qb);
+  oz_max<T><<<qa.blocks + qb.blocks, 256, 0, h->stream>>>(qa, qb, k, w.words);
+  return nrs_after_launch(h, "oz_max");
 }
 
-int launch_est_operand(nrs_handle* h, const OzOperand& o, int64_t k, int64_t kpad, const int* e,
-                       uint16_t* out, float* sums, float* part) {
-  cudaStream_t s = h->stream;
-  if (o.rows_contig) {
-    const unsigned grid = (unsigned)((o.rows + 7) / 8);
-    if (o.f32)
-      est_rows<false, float><<<grid, 256, 0, s>>>(o.f(), o.rows, k, o.ld, kpad, e, out, sums);
-    else if (((reinterpret_cast<uintptr_t>(o.p) & 15) == 0) && (o.ld % 2 == 0))
-      est_rows<true, double><<<grid, 256, 0, s>>>(o.d(), o.rows, k, o.ld, kpad, e, out, sums);
-    else
-      est_rows<false, double><<<grid, 256, 0, s>>>(o.d(), o.rows, k, o.ld, kpad, e, out, sums);
-  } else {
-    const int64_t strips = (kpad + kSliceColK - 1) / kSliceColK;
-    dim3 g((unsigned)((o.rows + kSliceColN - 1) / kSliceColN), (unsigned)strips);
-    if (o.f32)
-      est_cols<float><<<g, 256, 0, s>>>(o.f(), k, o.rows, o.ld, kpad, e, out, part);
-    else
-      est_cols<double><<<g, 256, 0, s>>>(o.d(), k, o.rows, o.ld, kpad, e, out, part);
-    est_strip_sums<<<(unsigned)((o.rows + 255) / 256), 256, 0, s>>>(part, strips, o.rows, sums);
-  }
-  return nrs_after_launch(h, "ozaki spread operands");
+// Scale of the fixed-point sums of up to k values below 1.
+float oz_sum_scale(int64_t k) {
+  float s = kSumScale;
+  while ((double)s * (double)k >= 2147483648.0 && s > 1.0f) s *= 0.5f;
+  return s;
+}
+
+template <typename T>
+int launch_oz_est(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t k, int64_t kpad,
+                  const OzScratch& w, bool pass2) {
+  auto blocks = [&](const OzPrep<T>& q) {
+    return (unsigned)(q.rows_contig ? (q.rows + 7) / 8
+                                    : (q.rows + kSliceColN - 1) / kSliceColN * ((kpad + kSliceColK - 1) / kSliceColK));
+  };
+  OzPrep<T> qa = oz_prep<T>(a, k, w.ea, w.part_a, w.ra, w.area_a), qb = oz_prep<T>(bT, k, w.eb, w.part_b, w.cb, w.area_b);
+  qa.blocks = blocks(qa);
+  qb.blocks = blocks(qb);
+  const float scale = oz_sum_scale(k);
+  if (pass2)
+    oz_est<T, true><<<qa.blocks + qb.blocks, 256, 0, h->stream>>>(qa, qb, k, kpad, scale, w.words);
+  else
+    oz_est<T, false><<<qa.blocks + qb.blocks, 256, 0, h->stream>>>(qa, qb, k, kpad, scale, w.words);
+  return nrs_after_launch(h, "oz_est");
+}
+
+// decide != null: the count is decided on the device under `rule`.
+template <typename T>
+int launch_oz_slice(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t k, int64_t kpad, int b, int S,
+                    uint32_t* decide, const OzRule& rule, const OzScratch& w) {
+  auto blocks = [&](const OzPrep<T>& q) {
+    return (unsigned)(q.rows_contig
+                          ? std::min<int64_t>((q.rows * (kpad / 8) + 255) / 256, (int64_t)h->num_sms * 8)
+                          : (q.rows + kSliceColN - 1) / kSliceColN * ((kpad + kSliceColK - 1) / kSliceColK));
+  };
+  OzPrep<T> qa = oz_prep<T>(a, k, w.ea, w.part_a, w.ra, w.area_a), qb = oz_prep<T>(bT, k, w.eb, w.part_b, w.cb, w.area_b);
+  qa.blocks = blocks(qa);
+  qb.blocks = blocks(qb);
+  const unsigned grid = qa.blocks + qb.blocks;
+  if (b == 8)
+    oz_slice<T, 8><<<grid, 256, 0, h->stream>>>(qa, qb, k, kpad, S, decide, rule);
+  else if (b == 7)
+    oz_slice<T, 7><<<grid, 256, 0, h->stream>>>(qa, qb, k, kpad, S, decide, rule);
+  else
+    oz_slice<T, 6><<<grid, 256, 0, h->stream>>>(qa, qb, k, kpad, S, decide, rule);
+  return nrs_after_launch(h, "oz_slice");
 }
 
 // rows_a / rows_b: rows of the (stacked) slice buffers; P.kpad: their pitch.
-template <bool EST, bool G>
-int launch_tc(nrs_handle* h, const void* sa, const void* sb, int S, const OzParams& P, int64_t rows_a,
-              int64_t rows_b, cudaStream_t stream) {
+template <bool EST, bool G, bool B8>
+int launch_tc_b(nrs_handle* h, const void* sa, const void* sb, int S, const OzParams& P, int64_t rows_a,
+                int64_t rows_b, cudaStream_t stream) {
   CUtensorMap mapA, mapB;
   if (!make_slice_map(&mapA, sa, P.kpad, rows_a, S, OZ_BM) ||
       !make_slice_map(&mapB, sb, P.kpad, rows_b, S, OzGeom<G>::BN))
     return nrs_fail(h, NRS_ERR_CUDA, "cuTensorMapEncodeTiled failed for the slices");
   // Set on every call: the attribute belongs to the current device's context.
-  int st = nrs_cuda_check(h, cudaFuncSetAttribute(ozaki_tc_kernel<EST, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  OzGeom<G>::SMEM),
+  int st = nrs_cuda_check(h, cudaFuncSetAttribute(ozaki_tc_kernel<EST, G, B8>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, OzGeom<G>::SMEM),
                           "cudaFuncSetAttribute(ozaki)");
   if (st) return st;
   const int n_tiles = G ? P.n_tiles : P.tiles_m * P.tiles_n;
   const int ctas = n_tiles < h->num_sms ? n_tiles : h->num_sms;
   if (ctas < 1) return NRS_OK;
-  ozaki_tc_kernel<EST, G><<<ctas, OZ_THREADS, OzGeom<G>::SMEM, stream>>>(mapA, mapB, P);
+  ozaki_tc_kernel<EST, G, B8><<<ctas, OZ_THREADS, OzGeom<G>::SMEM, stream>>>(mapA, mapB, P);
   return nrs_after_launch(h, EST ? "ozaki_tc_kernel<est>" : "ozaki_tc_kernel");
+}
+template <bool EST, bool G>
+int launch_tc(nrs_handle* h, const void* sa, const void* sb, int S, const OzParams& P, int64_t rows_a,
+              int64_t rows_b, cudaStream_t stream) {
+  if (EST || P.digit_bits == 8) return launch_tc_b<EST, G, true>(h, sa, sb, S, P, rows_a, rows_b, stream);
+  return launch_tc_b<EST, G, EST>(h, sa, sb, S, P, rows_a, rows_b, stream);
 }
 
 OzParams base_params(nrs_handle* h, int64_t m, int64_t n, int64_t k, int64_t kpad) {
@@ -1477,46 +1744,41 @@ struct SpreadResult {
   uint32_t flags;  // bit 0: an operand holds Inf or NaN
 };
 
-// Runs the spread estimate: exponents, estimate operands and one (pass 1) or
-// three (pass 2) BF16 products, then reads max_ij R_ij back (one stream
-// synchronisation).
-int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, int64_t n, int64_t k,
-                    int64_t kpad, int pass, SpreadResult* res) {
-  auto al = [](size_t v) { return (v + 1023) & ~size_t(1023); };
-  const int64_t strips = (kpad + kSliceColK - 1) / kSliceColK;
-  const size_t ea_b = al((size_t)m * 4), eb_b = al((size_t)n * 4), ra_b = al((size_t)m * 4),
-               cb_b = al((size_t)n * 4), cm_b = al((size_t)std::max(m, n) * 8),
-               part_b = al((size_t)strips * std::max(m, n) * 4), sa_b = al((size_t)2 * m * kpad * 2),
-               sb_b = al((size_t)2 * n * kpad * 2), word_b = 1024;
+// Enqueues the spread estimate: exponents, estimate operands and one (pass
+// 1) or three (pass 2) BF16 products into the decision words.
+template <typename T>
+int launch_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, int64_t n, int64_t k,
+                    int64_t kpad, int pass, const OzScratch& w) {
   int st;
-  uint8_t* ws = (uint8_t*)nrs_workspace(h, ea_b + eb_b + ra_b + cb_b + cm_b + part_b + sa_b + sb_b + word_b, &st);
-  if (!ws) return st;
-  int* ea = (int*)ws;
-  int* eb = (int*)(ws + ea_b);
-  float* ra = (float*)(ws + ea_b + eb_b);
-  float* cb = (float*)(ws + ea_b + eb_b + ra_b);
-  unsigned long long* colmax = (unsigned long long*)(ws + ea_b + eb_b + ra_b + cb_b);
-  float* part = (float*)(ws + ea_b + eb_b + ra_b + cb_b + cm_b);
-  uint16_t* sa = (uint16_t*)(ws + ea_b + eb_b + ra_b + cb_b + cm_b + part_b);
-  uint16_t* sb = (uint16_t*)((uint8_t*)sa + sa_b);
-  uint32_t* word = (uint32_t*)((uint8_t*)sb + sb_b);  // [0] max R bits, [1] flags
-  cudaStream_t s = h->stream;
-  if ((st = nrs_cuda_check(h, cudaMemsetAsync(word, 0, 8, s), "cudaMemsetAsync"))) return st;
-  if ((st = launch_exponents(h, a, k, ea, colmax, word + 1))) return st;
-  if ((st = launch_exponents(h, bT, k, eb, colmax, word + 1))) return st;
-  if ((st = launch_est_operand(h, a, k, kpad, ea, sa, ra, part))) return st;
-  if ((st = launch_est_operand(h, bT, k, kpad, eb, sb, cb, part))) return st;
+  if ((st = launch_oz_max<T>(h, a, bT, k, w))) return st;
+  if ((st = launch_oz_est<T>(h, a, bT, k, kpad, w, pass == 2))) return st;
   OzParams P = base_params(h, m, n, k, kpad);
   P.slices = pass;
   P.kchunks = 1;
   P.n_pairs = pass == 1 ? 1 : 3;
   P.kchunk = (int)(((kpad + OZ_BK - 1) / OZ_BK) * OZ_BK);
-  P.ra = ra;
-  P.cb = cb;
-  P.est = word;
-  if ((st = launch_tc<true, false>(h, sa, sb, 2, P, m, n, s))) return st;
+  P.ra = w.ra;
+  P.cb = w.cb;
+  P.sum_unit = 1.0f / oz_sum_scale(k);
+  P.est = w.words + OZ_W_SPREAD;
+  return launch_tc<true, false>(h, w.area_a, w.area_b, pass, P, m, n, h->stream);
+}
+
+// The estimate with its result read back (one stream synchronisation).
+int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, bool f32, int64_t m, int64_t n, int64_t k,
+                    int64_t kpad, int pass, SpreadResult* res) {
+  int st;
+  OzScratch w;
+  uint8_t* ws = (uint8_t*)nrs_workspace(h, oz_scratch(m, n, kpad, pass, 0, nullptr, nullptr), &st);
+  if (!ws) return st;
+  oz_scratch(m, n, kpad, pass, 0, ws, &w);
+  st = f32 ? launch_estimate<float>(h, a, bT, m, n, k, kpad, pass, w)
+           : launch_estimate<double>(h, a, bT, m, n, k, kpad, pass, w);
+  if (st) return st;
+  cudaStream_t s = h->stream;
   uint32_t host[2] = {0, 0};
-  if ((st = nrs_cuda_check(h, cudaMemcpyAsync(host, word, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync")))
+  static_assert(OZ_W_SPREAD == 0 && OZ_W_NONFINITE == 1, "the two words read back");
+  if ((st = nrs_cuda_check(h, cudaMemcpyAsync(host, w.words, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync")))
     return st;
   if ((st = nrs_cuda_check(h, cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return st;
   uint32_t derr = 0;
@@ -1530,44 +1792,146 @@ int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int6
   return NRS_OK;
 }
 
+// Digit slots of the 128 x 256 kernel: 16 bytes per element and CTA.
+size_t oz_slot_bytes(nrs_handle* h, int64_t m, int64_t n) {
+  const int64_t tiles = ((m + OZ_BM - 1) / OZ_BM) * ((n + OZ_BN - 1) / OZ_BN);
+  return (size_t)std::min<int64_t>(tiles, h->hw_sms) * OZ_BM * OZ_BN * 16;
+}
+
 int ozaki_run(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, int64_t n, int64_t k,
               int64_t kpad, int b, int S, int kchunks, double* C, int64_t ldc, bool accumulate) {
-  auto al = [](size_t v) { return (v + 1023) & ~size_t(1023); };
-  // Workspace: exponents | A slices | B slices | digit slots, one 128 x 256
-  // x 16-byte slot per CTA (the column maxima of a column-major operand go
-  // through the slots first).
-  const size_t ea_b = al((size_t)m * 4), eb_b = al((size_t)n * 4);
-  const size_t sa_b = al((size_t)S * m * kpad * 2), sb_b = al((size_t)S * n * kpad * 2);
-  const int64_t tiles = ((m + OZ_BM - 1) / OZ_BM) * ((n + OZ_BN - 1) / OZ_BN);
-  const int64_t ctas = std::min<int64_t>(tiles, h->hw_sms);
-  const size_t acc_b = al(std::max((size_t)ctas * OZ_BM * OZ_BN * 16, (size_t)std::max(m, n) * 8));
   int st;
-  uint8_t* ws = (uint8_t*)nrs_workspace(h, ea_b + eb_b + sa_b + sb_b + acc_b, &st);
+  OzScratch w;
+  const size_t slots = oz_slot_bytes(h, m, n);
+  uint8_t* ws = (uint8_t*)nrs_workspace(h, oz_scratch(m, n, kpad, S, slots, nullptr, nullptr), &st);
   if (!ws) return st;
-  int* ea = (int*)ws;
-  int* eb = (int*)(ws + ea_b);
-  uint16_t* sa = (uint16_t*)(ws + ea_b + eb_b);
-  uint16_t* sb = (uint16_t*)(ws + ea_b + eb_b + sa_b);
-  __int128* acc = (__int128*)(ws + ea_b + eb_b + sa_b + sb_b);
-  unsigned long long* colmax = reinterpret_cast<unsigned long long*>(acc);
-  if ((st = launch_exponents(h, a, k, ea, colmax, nullptr))) return st;
-  if ((st = launch_exponents(h, bT, k, eb, colmax, nullptr))) return st;
-  if ((st = launch_slices(h, a, k, kpad, ea, b, S, sa))) return st;
-  if ((st = launch_slices(h, bT, k, kpad, eb, b, S, sb))) return st;
+  oz_scratch(m, n, kpad, S, slots, ws, &w);
+  if ((st = launch_oz_max<double>(h, a, bT, k, w))) return st;
+  if ((st = launch_oz_slice<double>(h, a, bT, k, kpad, b, S, nullptr, OzRule{}, w))) return st;
   OzParams P = base_params(h, m, n, k, kpad);
   P.slices = S;
   P.kchunks = kchunks;
   P.n_pairs = S * (S + 1) / 2 * (kchunks > 0 ? kchunks : 1);
-  P.ea = ea;
-  P.eb = eb;
-  P.acc = acc;
+  P.ea = w.ea;
+  P.eb = w.eb;
+  P.acc = reinterpret_cast<__int128*>(w.tail);
   P.C = C;
   P.ldc = ldc;
-  P.final_shift = 2 - 2 * b - b * (S - 1);
   P.digit_bits = b;
   P.kchunk = kChunkOf(b);
   P.accumulate = accumulate ? 1 : 0;
-  return launch_tc<false, false>(h, sa, sb, S, P, m, n, h->stream);
+  return launch_tc<false, false>(h, w.area_a, w.area_b, S, P, m, n, h->stream);
+}
+
+// ---------------------------------------------------------------------------
+// Plain GEMM calls on the tensor cores
+// ---------------------------------------------------------------------------
+// The slice GEMM as the everyday form of C = A*B: the slice count follows the
+// operands' spread as in nrs_gemm_ozaki, but it is decided on the device, so
+// the call neither synchronises nor copies anything back. The launches:
+// oz_max, oz_est, the estimate product, oz_slice (decides), the slice
+// products, and the plain FP64 / FP32 kernel, whose blocks return at once
+// unless the count is 0 (Inf / NaN operands, sums that could overflow, or a
+// spread beyond the slice limit).
+//
+// One problem runs either on 128 x 256 tiles (the least panel traffic per
+// flop) or on the grouped 128 x 128 geometry with K split into ranges whose
+// f64 products are added in order, which fills the GPU at small sizes.
+struct TcPlan {
+  bool big;
+  int splits, split_blocks;
+  double us;
+};
+constexpr int kAutoMaxSlices = 12;
+
+// The form with the least modelled time (us). A 64-wide K block of one slice
+// pair takes 0.21 us on a 128 x 128 tile and 0.37 us on a 128 x 256 one; a
+// tile's fold and rounding 25 and 90 us. Measured against it (f64, S = 7):
+// 4096^3 2956 us (128 x 128) and 3389 us (128 x 256), 2048^3 497 and 544,
+// 1999 x 3001 x 1537 705, 623 with two K ranges, 709 on 128 x 256 tiles;
+// 1024^3 166 whole, 137 in two; 512^3 111, 94, 84, 84 in 1, 2, 4, 8.
+TcPlan plan_tc(int64_t m, int64_t n, int64_t kpad, int S) {
+  const double pairs = 0.5 * S * (S + 1);
+  const int kb = (int)((kpad + OZ_BK - 1) / OZ_BK);
+  const int64_t tm = (m + OZ_BM - 1) / OZ_BM;
+  auto waves = [](int64_t tiles) { return (double)((tiles + NRS_PLAN_SMS - 1) / NRS_PLAN_SMS); };
+  TcPlan best{true, 1, kb, waves(tm * ((n + OZ_BN - 1) / OZ_BN)) * (pairs * kb * 0.37 + 90.0)};
+  const int64_t t128 = tm * ((n + 127) / 128);
+  for (int z = 1; z <= 16 && z <= kb; z *= 2) {
+    const int blocks = (kb + z - 1) / z;
+    const int splits = (kb + blocks - 1) / blocks;
+    if (splits != z || (z > 1 && (double)z * (double)(m * n) * 8.0 > 256.0 * (1 << 20))) continue;
+    double us = waves(t128 * z) * (pairs * blocks * 0.21 + 25.0);
+    if (z > 1) us += 3.0 + (double)z * (double)(m * n) * 8.0 / 4e6;
+    if (us < best.us) best = TcPlan{false, splits, blocks, us};
+  }
+  return best;
+}
+
+template <typename T>
+int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, int64_t k, int64_t n, void* C,
+            int64_t ldc, bool accumulate) {
+  constexpr bool F32 = sizeof(T) == 4;
+  const int64_t kpad = (k + 7) / 8 * 8;
+  // 8-bit digits up to K = 10240, then 7-bit (exact int32 diagonal sums for
+  // every count up to the limit)
+  const int b = digits_fit(8, kAutoMaxSlices, kpad, kMaxChunkSlicesGrouped) ? 8 : 7;
+  if (!digits_fit(b, kAutoMaxSlices, kpad, kMaxChunkSlicesGrouped)) return NRS_ERR_UNSUPPORTED;
+  int klog = 0;
+  while (((int64_t)1 << klog) < k) ++klog;
+  const OzRule rule{F32 ? 26 : 53, b, kAutoMaxSlices, (F32 ? 127 : 1023) - klog - 1};
+  const TcPlan pl = plan_tc(m, n, kpad, F32 ? 4 : 7);
+  const int plain_splits = F32 ? 1 : nrs_dmma_splits(m, k, n);
+  const int slabs = std::max(pl.splits > 1 ? pl.splits : 0, plain_splits > 1 ? plain_splits : 0);
+  // Behind the slices: the kernel's digit slots (the grouped geometry needs
+  // them beyond 9 slices only), then the partial slabs.
+  const size_t slots = oz_al(pl.big ? oz_slot_bytes(h, m, n)
+                                    : (size_t)h->hw_sms * OZ_BM * OzGeom<true>::BN * OZ_DIGIT_BYTES);
+  const size_t tail = slots + (size_t)slabs * (size_t)(m * n) * 8;
+  cudaStream_t s = h->stream;
+  const size_t bytes = oz_scratch(m, n, kpad, kAutoMaxSlices, tail, nullptr, nullptr);
+  void* ws = nullptr;
+  if (cudaMallocFromPoolAsync(&ws, bytes, h->pool, s) != cudaSuccess) {
+    cudaGetLastError();  // no room: the plain kernel needs none
+    return NRS_ERR_UNSUPPORTED;
+  }
+  OzScratch w;
+  oz_scratch(m, n, kpad, kAutoMaxSlices, tail, (uint8_t*)ws, &w);
+  double* const slab = reinterpret_cast<double*>(w.tail + slots);
+  auto run = [&]() -> int {
+    int st;
+    if ((st = launch_estimate<T>(h, a, bT, m, n, k, kpad, 1, w))) return st;
+    if ((st = launch_oz_slice<T>(h, a, bT, k, kpad, b, 0, w.words, rule, w))) return st;
+    OzParams P = base_params(h, m, n, k, kpad);
+    P.count = w.words + OZ_W_COUNT;
+    P.kchunks = (int)((kpad + kChunkOf(b) - 1) / kChunkOf(b));
+    P.ea = w.ea;
+    P.eb = w.eb;
+    P.acc = reinterpret_cast<__int128*>(w.tail);
+    P.C = pl.splits > 1 ? slab : static_cast<double*>(C);
+    P.ldc = ldc;
+    P.digit_bits = b;
+    P.kchunk = kChunkOf(b);
+    P.accumulate = accumulate ? 1 : 0;
+    P.f32 = F32 ? 1 : 0;
+    if (pl.big) {
+      st = launch_tc<false, false>(h, w.area_a, w.area_b, kAutoMaxSlices, P, m, n, s);
+    } else {
+      P.tiles_n = (int)((n + OzGeom<true>::BN - 1) / OzGeom<true>::BN);
+      P.splits = pl.splits;
+      P.split_blocks = pl.split_blocks;
+      P.n_tiles = P.tiles_m * P.tiles_n * pl.splits;
+      st = launch_tc<false, true>(h, w.area_a, w.area_b, kAutoMaxSlices, P, m, n, s);
+    }
+    if (st) return st;
+    const int64_t rsa = a.rows_contig ? a.ld : 1, csa = a.rows_contig ? 1 : a.ld;
+    const int64_t rsb = bT.rows_contig ? 1 : bT.ld, csb = bT.rows_contig ? bT.ld : 1;
+    return nrs_plain_gemm_unless(h, F32 ? NRS_F32 : NRS_F64, m, k, n, a.p, rsa, csa, bT.p, rsb, csb, C, ldc,
+                                 accumulate, P.count, slab, pl.splits);
+  };
+  const int st = run();
+  cudaFreeAsync(ws, s);
+  return st;
 }
 
 // ---------------------------------------------------------------------------
@@ -1654,7 +2018,7 @@ __global__ void __launch_bounds__(256)
     if constexpr (SMALL) {
       OzakiZ64 Z[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) Z[t] = ozaki_z64(j0 + t < q.k ? (double)src[t] : 0.0, e, b, S, C64);
+      for (int t = 0; t < 8; ++t) Z[t] = ozaki_z64(j0 + t < q.k ? src[t] : T(0), e, b, S, C64);
 #pragma unroll
       for (int t = 0; t < OZ_MAX_SLICES; ++t) {
         if (t < S) {
@@ -1669,7 +2033,7 @@ __global__ void __launch_bounds__(256)
     } else {
       unsigned __int128 Z[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) Z[t] = (unsigned __int128)fixed126(j0 + t < q.k ? (double)src[t] : 0.0, e) + C;
+      for (int t = 0; t < 8; ++t) Z[t] = (unsigned __int128)fixed126(j0 + t < q.k ? src[t] : T(0), e) + C;
 #pragma unroll
       for (int t = 0; t < OZ_MAX_SLICES; ++t) {
         if (t < S) {
@@ -1704,8 +2068,8 @@ __global__ void __launch_bounds__(256)
     for (int r = 0; r < kSliceColK / 16; ++r) {
       const int w = ty + 8 * r;
       const int64_t kk = k0 + 2 * w;
-      const double x0 = kk < q.k && nn < q.n ? (double)Bq[kk * q.ldb + nn] : 0.0;
-      const double x1 = kk + 1 < q.k && nn < q.n ? (double)Bq[(kk + 1) * q.ldb + nn] : 0.0;
+      const T x0 = kk < q.k && nn < q.n ? Bq[kk * q.ldb + nn] : T(0);
+      const T x1 = kk + 1 < q.k && nn < q.n ? Bq[(kk + 1) * q.ldb + nn] : T(0);
       if constexpr (SMALL) {
         const OzakiZ64 Z0 = ozaki_z64(x0, e, b, S, C64), Z1 = ozaki_z64(x1, e, b, S, C64);
 #pragma unroll
@@ -1737,6 +2101,35 @@ __global__ void __launch_bounds__(256)
 }
 
 }  // namespace
+
+// f64 GEMMs for which the slice GEMM is the faster form; NRS_ERR_UNSUPPORTED:
+// not one of them (nothing was enqueued). The rule compares both forms'
+// modelled times: the FP64 tensor path's 1.05 TFLOP/s on 32-wide tiles
+// against plan_tc's. Both sides measured (us, DMMA / slices): 256^3 51 / 76,
+// 384^3 124 / 85, 512^3 279 / 84, 1024^3 1983 / 137, 2048^3 15661 / 497,
+// 4096^3 124903 / 2956, 3000 x 2000 x 10 379 / 163, 64 x 4096 x 64 91 / 114.
+int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
+                     const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate) {
+  if (!h->pool || dtype != NRS_F64) return NRS_ERR_UNSUPPORTED;
+  if (m > (1LL << 24) || n > (1LL << 24) || k > (1LL << 24)) return NRS_ERR_UNSUPPORTED;
+  const double mk = (double)m * k, kn = (double)k * n;
+  const double plain_us = (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * 2.0 / 1.05e6 + 10.0;
+  if (plain_us < 60.0) return NRS_ERR_UNSUPPORTED;
+  // exponents, estimate, slicing: seven launches, 40 bytes per operand element
+  const double tc_us = 45.0 + (mk + kn) * 40.0 / 3e6 + plan_tc(m, n, (k + 7) / 8 * 8, 7).us * (1.0 + 1.0 / 28.0);
+  if (tc_us > 0.9 * plain_us) return NRS_ERR_UNSUPPORTED;
+  // Under stream capture the plain kernel runs, as its launches hold no
+  // allocation.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return NRS_ERR_UNSUPPORTED;
+  }
+  if (cap != cudaStreamCaptureStatusNone) return NRS_ERR_UNSUPPORTED;
+  const OzOperand a{A, lda, m, !ta};
+  const OzOperand bT{B, ldb, n, tb};
+  return tc_gemm<double>(h, a, bT, m, k, n, C, ldc, accumulate);
+}
 
 extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, const double* A,
                               int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc,
@@ -1797,13 +2190,13 @@ extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, co
   double spread = 0.0;
   if (slices == 0) {
     SpreadResult r{};
-    if ((st = spread_estimate(h, a, bT, m, n, k, kpad, 1, &r))) return st;
+    if ((st = spread_estimate(h, a, bT, false, m, n, k, kpad, 1, &r))) return st;
     if (r.flags & 1u) return fallback("non-finite operand");
     double need = kTargetBits + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
     if (!(std::isfinite((double)r.rmax) && choose_digits(kpad, need, &b, &S, &kchunks))) {
       // The pass-1 numerator counts every k; pass 2 counts only the k where
       // the other operand is nonzero (sparse and structured operands).
-      if ((st = spread_estimate(h, a, bT, m, n, k, kpad, 2, &r))) return st;
+      if ((st = spread_estimate(h, a, bT, false, m, n, k, kpad, 2, &r))) return st;
       need = kTargetBits + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
       if (!(std::isfinite((double)r.rmax) && choose_digits(kpad, need, &b, &S, &kchunks))) {
         if (info) info->spread = std::isfinite((double)r.rmax) ? (double)r.rmax : HUGE_VAL;
@@ -1896,14 +2289,14 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
     }
     const int64_t kpad8 = (g.k + 7) / 8 * 8;
     SpreadResult r{};
-    const OzOperand a{g.A, g.lda, g.m, true, f32}, bT{g.B, g.ldb, g.n, false, f32};
-    int st = spread_estimate(h, a, bT, g.m, g.n, g.k, kpad8, 1, &r);
+    const OzOperand a{g.A, g.lda, g.m, true}, bT{g.B, g.ldb, g.n, false};
+    int st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad8, 1, &r);
     if (st) return st;
     if (r.flags & 1u) continue;
     double need = target + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
     int bb, SS, kc;
     if (!(std::isfinite((double)r.rmax) && choose_digits(kp_max, need, &bb, &SS, &kc, kMaxChunkSlicesGrouped))) {
-      if ((st = spread_estimate(h, a, bT, g.m, g.n, g.k, kpad8, 2, &r))) return st;
+      if ((st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad8, 2, &r))) return st;
       need = target + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
       if (!(std::isfinite((double)r.rmax) && choose_digits(kp_max, need, &bb, &SS, &kc, kMaxChunkSlicesGrouped)))
         continue;
@@ -2056,7 +2449,7 @@ template <typename T>
 int group_prepare(nrs_handle* h, nrs_ozaki_group* G, cudaStream_t s) {
   g_row_exponents<T><<<(unsigned)G->n_rowch, 256, 0, s>>>(G->d_in, G->d_rowch, G->d_ea);
   g_col_max_bits<T><<<(unsigned)G->n_colch, 256, 0, s>>>(G->d_in, G->d_colch, G->d_colmax);
-  exponents_from_bits<<<(unsigned)((G->rows_b + 255) / 256), 256, 0, s>>>(G->d_colmax, G->rows_b, G->d_eb, nullptr);
+  exponents_from_bits<<<(unsigned)((G->rows_b + 255) / 256), 256, 0, s>>>(G->d_colmax, G->rows_b, G->d_eb);
   int st = nrs_after_launch(h, "grouped ozaki exponents");
   if (st) return st;
   return G->b == 8 ? group_slices<T, 8>(h, G, s) : G->b == 7 ? group_slices<T, 7>(h, G, s)
@@ -2077,7 +2470,6 @@ int nrs_ozaki_group_launch(nrs_handle* h, nrs_ozaki_group* G, cudaStream_t s) {
   P.ea = G->d_ea;
   P.eb = G->d_eb;
   P.acc = G->d_acc;
-  P.final_shift = 2 - 2 * G->b - G->b * (G->S - 1);
   P.digit_bits = G->b;
   P.kchunk = kChunkOf(G->b);
   P.err = h->dev_error;
@@ -2132,3 +2524,4 @@ extern "C" int nrs_gemm_ozaki_grouped(nrs_handle* h, int64_t count, const nrs_ge
   }
   return st;
 }
+

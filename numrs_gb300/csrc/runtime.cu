@@ -113,6 +113,17 @@ extern "C" int nrs_create(int device, nrs_handle** out) {
     delete h;
     return st;
   }
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  uint64_t keep = kPoolKeep;
+  if (cudaMemPoolCreate(&h->pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();
+    if (h->pool) cudaMemPoolDestroy(h->pool);
+    h->pool = nullptr;
+  }
   h->hw_sms = h->num_sms;
   h->stream = h->own_stream;
   *out = h;
@@ -132,6 +143,7 @@ extern "C" int nrs_destroy(nrs_handle* h) {
   cudaSetDevice(h->device);
   cudaStreamSynchronize(h->stream);
   if (h->workspace) cudaFree(h->workspace);
+  if (h->pool) cudaMemPoolDestroy(h->pool);
   if (h->dev_error) cudaFree(h->dev_error);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   nrs_tuner_free(h);
