@@ -15,9 +15,12 @@
 #include <cmath>
 #include <type_traits>
 
+#include <cooperative_groups.h>
+
 #include "gemm_tiles.cuh"
 
 using namespace nrs_tiles;
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -119,6 +122,52 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM * BN >= 128 * 128 ?
   tile_store<T>(t, C, ldc, m, n, m0, n0, accumulate != 0);
 }
 
+// The 64 x 64 f32 tile with K split over a cluster of gridDim.z CTAs: CTA z
+// takes k-values [z*kc, min(k, (z+1)*kc)) and leaves its product in shared
+// memory; then every CTA adds a share of the tile's elements over the ranks
+// in order (through distributed shared memory) and writes them. One launch
+// and no scratch, so it needs no workspace shared between streams and runs
+// under capture.
+constexpr int kSplitTile = 64;
+using SplitTile = Simt<float, kSplitTile, kSplitTile, 16, 4, 4>;
+static_assert(SplitTile::kSmem >= kSplitTile * kSplitTile * 4, "the partial tile reuses the operand buffers");
+__global__ void __launch_bounds__(SplitTile::NT, 3)
+    simt_gemm_split(int64_t m, int64_t n, int64_t k, int64_t kc, const float* __restrict__ A, int64_t rsa, int64_t csa,
+                    const float* __restrict__ B, int64_t rsb, int64_t csb, float* __restrict__ C, int64_t ldc,
+                    int accumulate, const uint32_t* __restrict__ unless) {
+  if (unless && *unless) return;  // (the same word for every CTA of the cluster)
+  __shared__ __align__(16) uint8_t smem[SplitTile::kSmem];
+  SplitTile t;
+  const int64_t m0 = (int64_t)blockIdx.y * kSplitTile, n0 = (int64_t)blockIdx.x * kSplitTile;
+  const int64_t k0 = (int64_t)blockIdx.z * kc, k1 = (k0 + kc < k) ? k0 + kc : k;
+  t.run(A, rsa, csa, B, rsb, csb, m, n, m0, n0, k0, k1, smem);
+  const int splits = (int)gridDim.z;
+  if (splits == 1) {
+    tile_store<float>(t, C, ldc, m, n, m0, n0, accumulate != 0);
+    return;
+  }
+  float* part = reinterpret_cast<float*>(smem);  // (run() ends with a barrier)
+#pragma unroll
+  for (int e = 0; e < SplitTile::kPerThread; ++e) {
+    int r, c;
+    t.coords(e, r, c);
+    part[r * kSplitTile + c] = t.value(e);
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  const int share = kSplitTile * kSplitTile / splits;
+  for (int i = threadIdx.x; i < share; i += SplitTile::NT) {
+    const int idx = (int)blockIdx.z * share + i;
+    const int64_t gi = m0 + idx / kSplitTile, gj = n0 + idx % kSplitTile;
+    if (gi >= m || gj >= n) continue;
+    float v = cluster.map_shared_rank(part, 0)[idx];
+    for (int z = 1; z < splits; ++z) v += cluster.map_shared_rank(part, z)[idx];
+    float* c = C + gi * ldc + gj;
+    *c = accumulate ? *c + v : v;
+  }
+  cluster.sync();  // a CTA's shared memory outlives its readers
+}
+
 // Generic GEMM: one thread per C element, k ascending, one rounding per op.
 template <typename T> __device__ __forceinline__ T gmul(T a, T b) { return a * b; }
 template <typename T> __device__ __forceinline__ T gadd(T a, T b) { return a + b; }
@@ -186,8 +235,49 @@ int finish_grid(nrs_handle* h, int64_t m, int64_t n) {
   return (int)(blocks < (int64_t)h->num_sms * 8 ? blocks : (int64_t)h->num_sms * 8);
 }
 
-// f32 tile size by the size of C.
-int f32_variant(int64_t m, int64_t n) { return (m * n >= 256LL * 256 * 16) ? NRS_GEMM_SIMT : NRS_GEMM_SIMT_SMALL; }
+// f32 GEMMs by themselves: 128 x 128 tiles, or 64 x 64 tiles with K split over
+// up to 8 CTAs of a cluster (whole 16-wide k tiles, at least 64 values each),
+// whichever the busiest SM finishes first (planned for NRS_PLAN_SMS, as the
+// split decides the rounding). Measured (us, before with 32 x 32 or 128 x 128
+// tiles / now): 300 x 1000 x 257 35 / 20, 512^3 29 / 19, 1024^3 124 / 76,
+// 64 x 4096 x 64 115 / 29, 3000 x 2000 x 10 65 / 35.
+struct F32Plan {
+  int tile;
+  int splits;
+  int64_t kc;
+  double us;
+};
+F32Plan plan_f32(int64_t m, int64_t n, int64_t k) {
+  auto waves = [](double ctas) { return std::ceil(ctas / NRS_PLAN_SMS); };
+  const double t128 = (double)((m + 127) / 128) * (double)((n + 127) / 128);
+  F32Plan best{128, 1, k, 4.0 + waves(t128) * (double)k * (128.0 * 128.0 / 1.45e5)};
+  const double t64 = (double)((m + 63) / 64) * (double)((n + 63) / 64);
+  for (int z = 1; z <= 8; z *= 2) {
+    const int64_t kc = ((k + z - 1) / z + 15) / 16 * 16;
+    if (z > 1 && (kc < 64 || (k + kc - 1) / kc != z)) break;
+    const double us = 4.0 + waves(t64 * z) * (double)kc * (64.0 * 64.0 / 1.0e5) + (z > 1 ? 2.0 : 0.0);
+    if (us < best.us) best = F32Plan{64, z, kc, us};
+  }
+  return best;
+}
+
+void launch_simt_split(nrs_handle* h, const F32Plan& pl, int64_t m, int64_t k, int64_t n, const float* A, int64_t rsa,
+                       int64_t csa, const float* B, int64_t rsb, int64_t csb, float* C, int64_t ldc, int acc,
+                       const uint32_t* unless) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = tiles(m, n, kSplitTile, kSplitTile);
+  cfg.gridDim.z = (unsigned)pl.splits;
+  cfg.blockDim = dim3(SplitTile::NT);
+  cfg.stream = h->stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = (unsigned)pl.splits;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, simt_gemm_split, m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
+}
 
 void launch_simt_f32(nrs_handle* h, bool large, int64_t m, int64_t k, int64_t n, const float* A, int64_t rsa,
                      int64_t csa, const float* B, int64_t rsb, int64_t csb, float* C, int64_t ldc, int acc,
@@ -200,9 +290,21 @@ void launch_simt_f32(nrs_handle* h, bool large, int64_t m, int64_t k, int64_t n,
                                                                                    C, ldc, acc, unless);
 }
 
+void launch_auto_f32(nrs_handle* h, int64_t m, int64_t k, int64_t n, const float* A, int64_t rsa, int64_t csa,
+                     const float* B, int64_t rsb, int64_t csb, float* C, int64_t ldc, int acc,
+                     const uint32_t* unless) {
+  const F32Plan pl = plan_f32(m, n, k);
+  if (pl.tile == 128)
+    launch_simt_f32(h, true, m, k, n, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
+  else
+    launch_simt_split(h, pl, m, k, n, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
+}
+
 bool grid_too_large(int64_t m, int64_t n) { return (n + 31) / 32 > 0x7fffffffLL || (m + 31) / 32 > 65535; }
 
 }  // namespace
+
+double nrs_plain_f32_us(int64_t m, int64_t k, int64_t n) { return plan_f32(m, n, k).us; }
 
 int nrs_dmma_splits(int64_t m, int64_t k, int64_t n) { return plan_dmma(m, n, k, NRS_PLAN_SMS).splits; }
 
@@ -218,8 +320,7 @@ int nrs_plain_gemm_unless(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
       splitk_finish<double><<<finish_grid(h, m, n), 256, 0, h->stream>>>(slab, pl.splits, m, n, (double*)C, ldc, acc,
                                                                          unless, tc_splits);
   } else {
-    launch_simt_f32(h, f32_variant(m, n) == NRS_GEMM_SIMT, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb,
-                    csb, (float*)C, ldc, acc, unless);
+    launch_auto_f32(h, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb, csb, (float*)C, ldc, acc, unless);
     if (tc_splits > 1)
       splitk_finish<float><<<finish_grid(h, m, n), 256, 0, h->stream>>>(slab, 1, m, n, (float*)C, ldc, acc, unless,
                                                                         tc_splits);
@@ -236,8 +337,11 @@ int nrs_plain_gemm_launch(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
   if (grid_too_large(m, n)) variant = NRS_GEMM_GENERIC;
   if (variant == NRS_GEMM_AUTO) {
     if (dtype == NRS_F64) variant = NRS_GEMM_DMMA;
-    else if (dtype == NRS_F32) variant = f32_variant(m, n);
-    else variant = NRS_GEMM_GENERIC;
+    else if (dtype != NRS_F32) variant = NRS_GEMM_GENERIC;
+  }
+  if (variant == NRS_GEMM_AUTO) {
+    launch_auto_f32(h, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb, csb, (float*)C, ldc, acc, nullptr);
+    return nrs_after_launch(h, "simt_gemm<f32>");
   }
   if (variant == NRS_GEMM_DMMA && dtype == NRS_F64) {
     // The k split decides the rounding: plan for a fixed SM count.

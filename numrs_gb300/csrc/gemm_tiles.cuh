@@ -126,10 +126,88 @@ struct Dmma {
 // Either way every C element is the same k-ordered FMA chain, so the mapping
 // does not change a bit of the result.
 // ---------------------------------------------------------------------------
+// One operand's shared tile [BK][ROWS + 4] (k-major): element (row, k) of the
+// operand at p[row * rs + k * ks], rs or ks being 1 (or neither: scalar
+// loads). A thread moves vectors of V elements along whichever dimension is
+// contiguous, so that a warp's loads cover whole sectors for either layout
+// (with the fixed k-fastest mapping an operand that is contiguous along its
+// rows took one sector per element: a 300 x 1000 x 257 f32 product with a
+// transposed B 66 us). Addresses advance by a constant per k tile.
+template <typename T, int ROWS, int BK, int NT>
+struct SimtLoader {
+  static constexpr int PER = ROWS * BK / NT;  // elements per thread
+  static constexpr int V = PER < 16 / (int)sizeof(T) ? PER : 16 / (int)sizeof(T);
+  static constexpr int N = PER / V;
+  static_assert(PER >= 1 && PER % V == 0 && BK % V == 0 && ROWS % V == 0, "tile / thread split");
+  T reg[N][V];
+  const T* p[N];
+  int row[N], kk[N];
+  int64_t step, rstep;  // of a k tile; between a vector's elements along rows
+  int64_t left;         // rows of the operand from the tile's first row on
+  bool kfast, vec;
+
+  __device__ __forceinline__ void init(const T* base, int64_t rs, int64_t ks_, int64_t rows, int64_t r0, int64_t k0) {
+    kfast = ks_ == 1;
+    step = (int64_t)BK * ks_;
+    left = rows - r0;
+    const T* tile = base + r0 * rs + k0 * ks_;
+    // every vector of the tile is aligned when its first one and the pitch are
+    vec = (kfast || rs == 1) && (reinterpret_cast<uintptr_t>(tile) % (V * sizeof(T))) == 0 &&
+          ((kfast ? rs : ks_) % V) == 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int e = threadIdx.x + i * NT;
+      row[i] = kfast ? e / (BK / V) : (e % (ROWS / V)) * V;
+      kk[i] = kfast ? (e % (BK / V)) * V : e / (ROWS / V);
+      p[i] = tile + (int64_t)row[i] * rs + (int64_t)kk[i] * ks_;
+    }
+    rstep = kfast ? 0 : rs;
+  }
+
+  // Loads the k tile whose first k is `kleft` before the end, then moves on.
+  __device__ __forceinline__ void load(int64_t kleft) {
+    const int rl = left < ROWS ? (int)left : ROWS, kl = kleft < BK ? (int)kleft : BK;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const bool whole = kfast ? (row[i] < rl && kk[i] + V <= kl) : (kk[i] < kl && row[i] + V <= rl);
+      if (vec && whole) {
+        if constexpr (V * sizeof(T) == 16) {
+          const uint4 u = *reinterpret_cast<const uint4*>(p[i]);
+          memcpy(reg[i], &u, 16);
+        } else if constexpr (V * sizeof(T) == 8) {
+          const uint2 u = *reinterpret_cast<const uint2*>(p[i]);
+          memcpy(reg[i], &u, 8);
+        } else {
+          reg[i][0] = *p[i];
+        }
+      } else {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const bool in = kfast ? (row[i] < rl && kk[i] + v < kl) : (kk[i] < kl && row[i] + v < rl);
+          reg[i][v] = in ? p[i][kfast ? v : v * rstep] : T(0);
+        }
+      }
+      p[i] += step;
+    }
+  }
+  __device__ __forceinline__ void store(T (*sm)[ROWS + 4]) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (!kfast && V * sizeof(T) == 16) {
+        uint4 u;
+        memcpy(&u, reg[i], 16);
+        *reinterpret_cast<uint4*>(&sm[kk[i]][row[i]]) = u;
+      } else {
+#pragma unroll
+        for (int v = 0; v < V; ++v) sm[kfast ? kk[i] + v : kk[i]][kfast ? row[i] : row[i] + v] = reg[i][v];
+      }
+    }
+  }
+};
+
 template <typename T, int BM, int BN, int BK, int TM, int TN>
 struct Simt {
   static constexpr int NT = (BM / TM) * (BN / TN);
-  static constexpr int LA = BM * BK / NT, LB = BN * BK / NT;
   static constexpr int kSmem = 2 * BK * ((BM + 4) + (BN + 4)) * (int)sizeof(T);
   static constexpr bool kVec = sizeof(T) == 4 && TM % 4 == 0 && TN % 4 == 0;
   T acc[TM][TN];
@@ -153,44 +231,26 @@ struct Simt {
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
-    T ra[LA], rb[LB];
-    auto load = [&](int64_t kt) {
-#pragma unroll
-      for (int i = 0; i < LA; ++i) {
-        int e = tid + i * NT;
-        int r = e / BK, kk = e % BK;
-        int64_t gi = m0 + r, gk = kt + kk;
-        ra[i] = (gi < m && gk < k1) ? A[gi * rsa + gk * csa] : T(0);
-      }
-#pragma unroll
-      for (int i = 0; i < LB; ++i) {
-        int e = tid + i * NT;
-        int kk = e / BN, c = e % BN;
-        int64_t gk = kt + kk, gj = n0 + c;
-        rb[i] = (gk < k1 && gj < n) ? B[gk * rsb + gj * csb] : T(0);
-      }
-    };
-    auto store = [&](int buf) {
-#pragma unroll
-      for (int i = 0; i < LA; ++i) {
-        int e = tid + i * NT;
-        As[buf][e % BK][e / BK] = ra[i];
-      }
-#pragma unroll
-      for (int i = 0; i < LB; ++i) {
-        int e = tid + i * NT;
-        Bs[buf][e / BN][e % BN] = rb[i];
-      }
-    };
+    SimtLoader<T, BM, BK, NT> la;
+    SimtLoader<T, BN, BK, NT> lb;
+    la.init(A, rsa, csa, m, m0, k0);
+    lb.init(B, csb, rsb, n, n0, k0);
     const int64_t ktiles = (k1 - k0 + BK - 1) / BK;
+    int64_t kleft = k1 - k0;
     if (ktiles > 0) {
-      load(k0);
-      store(0);
+      la.load(kleft);
+      lb.load(kleft);
+      la.store(As[0]);
+      lb.store(Bs[0]);
     }
     __syncthreads();
     for (int64_t kt = 0; kt < ktiles; ++kt) {
       const int buf = (int)(kt & 1);
-      if (kt + 1 < ktiles) load(k0 + (kt + 1) * BK);
+      kleft -= BK;
+      if (kt + 1 < ktiles) {
+        la.load(kleft);
+        lb.load(kleft);
+      }
 #pragma unroll
       for (int kk = 0; kk < BK; ++kk) {
         T a[TM], b[TN];
@@ -216,7 +276,10 @@ struct Simt {
 #pragma unroll
           for (int j = 0; j < TN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
       }
-      if (kt + 1 < ktiles) store(buf ^ 1);
+      if (kt + 1 < ktiles) {
+        la.store(As[buf ^ 1]);
+        lb.store(Bs[buf ^ 1]);
+      }
       __syncthreads();
     }
   }

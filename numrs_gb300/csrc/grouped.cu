@@ -187,7 +187,10 @@ __device__ void row_reduce_ops(const nrs_rowreduce_desc& r, uint8_t* smem) {
   }
 }
 
-__global__ void __launch_bounds__(kThreads)
+// Two CTAs per SM (128 registers): the tiles alternate loads and arithmetic,
+// and a row reduction is bound by load latency, so one CTA of 8 warps left
+// the SM idle in between (212 registers, one CTA, before).
+__global__ void __launch_bounds__(kThreads, 2)
     grouped_kernel(const nrs_gemm_desc* __restrict__ gp, const nrs_rowreduce_desc* __restrict__ rp,
                    const WorkItem* __restrict__ items, int n_items, unsigned* queue,
                    unsigned* tile_cnt, uint8_t* partials) {

@@ -2102,21 +2102,29 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
-// f64 GEMMs for which the slice GEMM is the faster form; NRS_ERR_UNSUPPORTED:
+// f64 and f32 GEMMs for which the slice GEMM is the faster form; NRS_ERR_UNSUPPORTED:
 // not one of them (nothing was enqueued). The rule compares both forms'
 // modelled times: the FP64 tensor path's 1.05 TFLOP/s on 32-wide tiles
 // against plan_tc's. Both sides measured (us, DMMA / slices): 256^3 51 / 76,
 // 384^3 124 / 85, 512^3 279 / 84, 1024^3 1983 / 137, 2048^3 15661 / 497,
 // 4096^3 124903 / 2956, 3000 x 2000 x 10 379 / 163, 64 x 4096 x 64 91 / 114.
+// f32 against the FP32 kernels (us): 1024^3 76 / 100, 1536^3 182 / 137,
+// 2048^3 418 / 246, 4096^3 3214 / 1241 (0.11 PFLOP/s; error 4e-9 of
+// (|A||B|)_ij against the FMA chains' 3e-7).
 int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
                      const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate) {
-  if (!h->pool || dtype != NRS_F64) return NRS_ERR_UNSUPPORTED;
+  if (!h->pool || (dtype != NRS_F64 && dtype != NRS_F32)) return NRS_ERR_UNSUPPORTED;
+  const bool f32 = dtype == NRS_F32;
   if (m > (1LL << 24) || n > (1LL << 24) || k > (1LL << 24)) return NRS_ERR_UNSUPPORTED;
   const double mk = (double)m * k, kn = (double)k * n;
-  const double plain_us = (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * 2.0 / 1.05e6 + 10.0;
+  const double plain_us = f32 ? nrs_plain_f32_us(m, k, n)
+                              : (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * 2.0 / 1.05e6 + 10.0;
   if (plain_us < 60.0) return NRS_ERR_UNSUPPORTED;
-  // exponents, estimate, slicing: seven launches, 40 bytes per operand element
-  const double tc_us = 45.0 + (mk + kn) * 40.0 / 3e6 + plan_tc(m, n, (k + 7) / 8 * 8, 7).us * (1.0 + 1.0 / 28.0);
+  // exponents, estimate, slicing: seven launches, 40 (f32: 16) bytes per
+  // operand element
+  const int S = f32 ? 4 : 7;
+  const double tc_us = 45.0 + (mk + kn) * (f32 ? 16.0 : 40.0) / 3e6 +
+                       plan_tc(m, n, (k + 7) / 8 * 8, S).us * (1.0 + 2.0 / (S * (S + 1)));
   if (tc_us > 0.9 * plain_us) return NRS_ERR_UNSUPPORTED;
   // Under stream capture the plain kernel runs, as its launches hold no
   // allocation.
@@ -2128,7 +2136,8 @@ int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, 
   if (cap != cudaStreamCaptureStatusNone) return NRS_ERR_UNSUPPORTED;
   const OzOperand a{A, lda, m, !ta};
   const OzOperand bT{B, ldb, n, tb};
-  return tc_gemm<double>(h, a, bT, m, k, n, C, ldc, accumulate);
+  return f32 ? tc_gemm<float>(h, a, bT, m, k, n, C, ldc, accumulate)
+             : tc_gemm<double>(h, a, bT, m, k, n, C, ldc, accumulate);
 }
 
 extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, const double* A,
