@@ -330,3 +330,23 @@ NRS_HD bool nrs_f64_nan_or_zero(uint64_t u) {
   return ((u & 0x7FFFFFFFFFFFFFFFull) - 1u) >= 0x7FF0000000000000ull;
 }
 NRS_HD bool nrs_f64_is_nan(uint64_t u) { return (u & 0x7FFFFFFFFFFFFFFFull) > 0x7FF0000000000000ull; }
+
+// The bits of x * x rounded once (nearest, ties to even) for the double with
+// bits u, in integer operations: a variance's squared deviations then leave
+// the FP64 pipe to its subtractions and ordered adds. `special`: x or the
+// square is not a normal finite number (zero included); redo it in FP64.
+NRS_HD uint64_t nrs_square(uint64_t u, bool& special) {
+  const int be = (int)((u >> 52) & 0x7FF);
+  const uint32_t hi = 0x80000000u | (uint32_t)(u >> 21), lo = (uint32_t)u << 11;  // significand, left-aligned
+  const uint64_t mid = (uint64_t)hi * lo, ll = (uint64_t)lo * lo;
+  const uint64_t low = ll + (mid << 33);
+  uint64_t high = (uint64_t)hi * hi + (mid >> 31) + (low < ll);  // [2^62, 2^64)
+  const bool top = high >> 63;
+  high = top ? high : high << 1 | low >> 63;
+  const uint64_t rest = top ? low : low << 1;
+  const int e = 2 * be - 1023 + top;  // biased exponent of the leading one
+  special = (be == 0) | (be == 0x7FF) | (e < 1) | (e > 2046);
+  const uint64_t mant = high >> 11;
+  const uint64_t inc = (high >> 10) & (((high & 0x3FF) | rest) != 0 ? 1 : mant) & 1;
+  return ((uint64_t)(uint32_t)(e - 1) << 52) + mant + inc;  // (the leading one adds 1 to the exponent)
+}

@@ -20,8 +20,9 @@
 //                    128 B along the axis x 64 lanes with the 128-byte
 //                    swizzle, so thread t reading its own row with 16-byte
 //                    loads is bank-conflict free.
-//  * fold_generic  : any strides, one thread per lane (small or unaligned
-//                    views).
+//  * fold_ring     : any strides and alignment, and few lanes, through the
+//                    element-copy ring (lane_ring.cuh).
+//  * fold_generic  : any strides, one thread per lane (short axes).
 //
 // Flat reductions (kernels::reduce, src/kernels/reduce.rs:204-444) keep the
 // reference's 8192-element chunking: one warp sums a chunk with a
@@ -35,6 +36,7 @@
 #include <mutex>
 #include <vector>
 
+#include "lane_ring.cuh"
 #include "reduce_common.cuh"
 
 using namespace nrs_red;
@@ -68,8 +70,16 @@ __global__ void fold_generic(const T* __restrict__ x, KeptDims kd, int64_t n_out
     }
     const T* p = x + base;
     const T m = lane_mean ? lane_mean[o] : T(0);
+    // (blocks: eight loads in flight, and the order-free ops' short chains)
     T acc = Fold<T, OP>::init();
-    for (int64_t j = 0; j < alen; ++j) acc = Fold<T, OP>::step(acc, lane_xform<T, OP>(p[j * astride], m));
+    int64_t j = 0;
+    for (; j + 8 <= alen; j += 8) {
+      T v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = p[(j + q) * astride];
+      acc = RunFold<T, OP>::template run<8>(acc, [&](int e) { return lane_xform<T, OP>(v[e], m); });
+    }
+    for (; j < alen; ++j) acc = Fold<T, OP>::step(acc, lane_xform<T, OP>(p[j * astride], m));
     out[o] = finish<T, OP>(acc, alen, div);
   }
 }
@@ -594,6 +604,97 @@ __global__ void __launch_bounds__(64)
 constexpr int kStages = 8;
 
 // ---------------------------------------------------------------------------
+// Views the TMA maps cannot address (lane_ring.cuh)
+// ---------------------------------------------------------------------------
+// d * d rounded once, off the FP64 pipe.
+__device__ __noinline__ double square_fp64(double d) { return __dmul_rn(d, d); }
+__device__ __forceinline__ double square_f64(double d) {
+  bool special;
+  const uint64_t r = nrs_square((uint64_t)__double_as_longlong(d), special);
+  return special ? square_fp64(d) : __longlong_as_double((long long)r);
+}
+
+template <typename T, int OP>
+struct RingFold {
+  static constexpr bool kStore = false;
+  static constexpr bool kXform = std::is_floating_point<T>::value && (OP == NRS_VAR || OP == NRS_STD);
+  typename OutOf<T, OP>::type* out;
+  int64_t alen;
+  T div, acc;
+  // f64: every other square in integers (nrs_square), so that the FP64 and
+  // the integer pipes share the work. Row std of 4864 / 9973 / 19456 x 12001
+  // (us): all in FP64 870 / 1579 / 2006, all in integers 1150 / 1443 / 1632.
+  static __device__ __forceinline__ T xform(T v, T m, int odd) {
+    if constexpr (std::is_same<T, double>::value) {
+      const double d = __dsub_rn(v, m);
+      return odd ? square_f64(d) : __dmul_rn(d, d);
+    } else {
+      return lane_xform<T, OP>(v, m);
+    }
+  }
+  template <int N>
+  __device__ __forceinline__ void block(T (&v)[N], int64_t) {
+    acc = RunFold<T, OP>::template run<N>(acc, [&](int e) { return v[e]; });
+  }
+  __device__ __forceinline__ void one(T& v, int64_t) { acc = Fold<T, OP>::step(acc, v); }
+  __device__ __forceinline__ void finish(int64_t lane) { out[lane] = nrs_red::finish<T, OP>(acc, alen, div); }
+};
+
+template <typename T, bool MAX>
+struct RingArg {
+  static constexpr bool kStore = false, kXform = false;
+  using Ord = ArgOrd<T, MAX>;
+  int64_t* out;
+  typename Ord::K best;
+  int64_t at;
+  static __device__ __forceinline__ T xform(T v, T, int) { return v; }
+  template <int N>
+  __device__ __forceinline__ void block(T (&v)[N], int64_t j) {
+    // (the lane's first element starts it; comparing it with itself then
+    // changes nothing, NaN included)
+    if (j == 0) best = Ord::start(v[0]);
+    int e0 = -1;
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      const typename Ord::K k = Ord::key(v[e]);
+      if (MAX ? (k > best) : (k < best)) {
+        best = k;
+        e0 = e;
+      }
+    }
+    if (e0 >= 0) at = j + e0;
+  }
+  __device__ __forceinline__ void one(T& v, int64_t j) {
+    const typename Ord::K k = Ord::key(v);
+    if (j == 0) {
+      best = Ord::start(v);
+    } else if (MAX ? (k > best) : (k < best)) {
+      best = k;
+      at = j;
+    }
+  }
+  __device__ __forceinline__ void finish(int64_t lane) { out[lane] = at; }
+};
+
+using RingDims = nrs_ring::LaneDims<NRS_UFUNC_MAX_DIMS>;
+
+template <typename T, int OP, bool ROWS>
+__global__ void __launch_bounds__(nrs_ring::kThreads)
+    fold_ring(const T* __restrict__ x, const __grid_constant__ RingDims g, int64_t n_lanes, int64_t alen,
+              int64_t astride, typename OutOf<T, OP>::type* __restrict__ out, const T* __restrict__ lane_mean, T div,
+              int len, uint32_t* err) {
+  RingFold<T, OP> f{out, alen, div, Fold<T, OP>::init()};
+  nrs_ring::run<T, ROWS>(x, g, n_lanes, alen, astride, (T*)nullptr, 0, lane_mean, len, err, 8u, f);
+}
+template <typename T, bool MAX, bool ROWS>
+__global__ void __launch_bounds__(nrs_ring::kThreads)
+    arg_ring(const T* __restrict__ x, const __grid_constant__ RingDims g, int64_t n_lanes, int64_t alen,
+             int64_t astride, int64_t* __restrict__ out, int len, uint32_t* err) {
+  RingArg<T, MAX> f{out, typename ArgOrd<T, MAX>::K(0), 0};
+  nrs_ring::run<T, ROWS>(x, g, n_lanes, alen, astride, (T*)nullptr, 0, (const T*)nullptr, len, err, 9u, f);
+}
+
+// ---------------------------------------------------------------------------
 // Flat reductions
 // ---------------------------------------------------------------------------
 // Per-chunk partials in the lane-striped order of a 256-lane SIMD sum: lane L
@@ -974,6 +1075,48 @@ int launch_generic(nrs_handle* h, const AxisProblem& p) {
   return nrs_after_launch(h, "fold_generic");
 }
 
+RingDims ring_dims(const KeptDims& k) {
+  RingDims g{};
+  g.n = k.n;
+  for (int d = 0; d < k.n; ++d) {
+    g.size[d] = k.size[d];
+    g.xstride[d] = k.stride[d];
+  }
+  return g;
+}
+// Which of the two takes a view that TMA does not: the ring has one warp per
+// 32 lanes fold ahead of three that copy; fold_generic one thread per lane,
+// whose loads are its own. The ring wins while those threads are too few to
+// cover their latency (f64 sums, us, generic / ring: 9973 x 12001 rows 1268 /
+// 591, 1000 x 20001 columns 111 / 121, 1000 x 50001 columns 158 / 234); along
+// contiguous lanes also for many lanes once they are long (a thread's own row
+// takes a sector per few elements: 100001 x 301 f32 60 / 43, x 101 22 / 24).
+bool ring_pays(int64_t alen, int64_t astride, int64_t n_out) {
+  if (n_out < 20000) return alen >= (astride == 1 ? 64 : 256);
+  return astride == 1 && alen >= 256;
+}
+
+template <typename T, typename Kern, typename... Args>
+int launch_ring_kernel(nrs_handle* h, const AxisProblem& p, Kern rows, Kern cols, const char* what, Args... args) {
+  const bool r = p.astride == 1;
+  const int len = nrs_ring::tile_len(sizeof(T), p.n_out, h->hw_sms);
+  const size_t smem = nrs_ring::smem_bytes(sizeof(T), r, len);
+  const Kern kern = r ? rows : cols;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kern<<<(unsigned)((p.n_out + nrs_ring::kLanes - 1) / nrs_ring::kLanes), nrs_ring::kThreads, smem, h->stream>>>(
+      (const T*)p.x, ring_dims(p.kept), p.n_out, p.alen, p.astride, args..., len, h->dev_error);
+  return nrs_after_launch(h, what);
+}
+template <typename T, int OP>
+int launch_ring(nrs_handle* h, const AxisProblem& p) {
+  return launch_ring_kernel<T>(h, p, fold_ring<T, OP, true>, fold_ring<T, OP, false>, "fold_ring",
+                               (typename OutOf<T, OP>::type*)p.out, (const T*)p.lane_mean, (T)p.div);
+}
+template <typename T, bool MAX>
+int launch_arg_ring(nrs_handle* h, const AxisProblem& p) {
+  return launch_ring_kernel<T>(h, p, arg_ring<T, MAX, true>, arg_ring<T, MAX, false>, "arg_ring", (int64_t*)p.out);
+}
+
 template <typename T, bool MAX>
 int launch_arg_tma(nrs_handle* h, const AxisProblem& p);
 
@@ -983,6 +1126,7 @@ int launch_arg(nrs_handle* h, const AxisProblem& p) {
     const int st = launch_arg_tma<T, MAX>(h, p);
     if (st != NRS_ERR_UNSUPPORTED) return st;
   }
+  if (ring_pays(p.alen, p.astride, p.n_out)) return launch_arg_ring<T, MAX>(h, p);
   int64_t blocks = (p.n_out + 255) / 256;
   int grid = (int)(blocks < (int64_t)h->num_sms * 16 ? blocks : (int64_t)h->num_sms * 16);
   if (grid < 1) grid = 1;
@@ -1186,11 +1330,22 @@ int launch_arg_tma(nrs_handle* h, const AxisProblem& p) {
 
 template <typename T, int OP>
 int dispatch_axis_t(nrs_handle* h, const AxisProblem& p) {
-  // The TMA pipelines pay off once lanes are long enough to fill a pipeline.
+  // f64 sums, products and variances: chains of FP64 operations, 64 cycles of
+  // an SM partition each. The ring folds 32 lanes per block on alternating
+  // partitions (the TMA folds 64, on two), and its moving warps subtract and
+  // square for a variance. 9973 x 12000 rows, us, TMA / ring: sum 588 / 485,
+  // std 2070 / 1540; past three (for a variance six) blocks per SM the TMA
+  // form is as fast (19456 rows: sum 593 / 612).
+  if constexpr (std::is_same<T, double>::value && OP != NRS_MAX && OP != NRS_MIN) {
+    const int64_t blocks = (p.n_out + nrs_ring::kLanes - 1) / nrs_ring::kLanes;
+    if (p.alen >= 256 && blocks <= (int64_t)h->hw_sms * (OP == NRS_VAR || OP == NRS_STD ? 6 : 3))
+      return launch_ring<T, OP>(h, p);
+  }
   if (p.alen >= 256 && p.n_out >= 64) {
     int st = launch_tma<T, OP>(h, p);
     if (st != NRS_ERR_UNSUPPORTED) return st;
   }
+  if (ring_pays(p.alen, p.astride, p.n_out)) return launch_ring<T, OP>(h, p);
   return launch_generic<T, OP>(h, p);
 }
 

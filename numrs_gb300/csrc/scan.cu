@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "f64_round.cuh"
+#include "lane_ring.cuh"
 #include "nrs_internal.cuh"
 
 namespace {
@@ -301,6 +302,35 @@ NRS_DEV T fold_row(uint8_t* tile, int t, int cnt, bool first, T acc) {
     }
   }
   return acc;
+}
+
+// Views TMA cannot address, and few lanes: the element-copy ring.
+template <typename T, int OP, bool RUNNING>
+struct RingLane {
+  static constexpr bool kStore = RUNNING, kXform = false;
+  T* out;
+  bool first;
+  T acc;
+  static NRS_DEV T xform(T v, T, int) { return v; }
+  template <int N>
+  NRS_DEV void block(T (&v)[N], int64_t j) {
+    acc = RUNNING ? run_block<T, OP, N>(v, first && j == 0, acc) : reduce_block<T, OP, N>(v, first && j == 0, acc);
+  }
+  NRS_DEV void one(T& v, int64_t j) {
+    acc = first && j == 0 ? v : apply<T, OP>(acc, v);
+    v = acc;
+  }
+  NRS_DEV void finish(int64_t lane) {
+    if (!RUNNING) out[lane] = acc;
+  }
+};
+using RingDims = nrs_ring::LaneDims<kMaxDims>;
+template <typename T, int OP, bool RUNNING, bool ROWS>
+__global__ void __launch_bounds__(nrs_ring::kThreads)
+    lane_ring(const T* __restrict__ x, const __grid_constant__ RingDims g, int64_t n_lanes, int64_t alen,
+              int64_t xastride, T* __restrict__ out, int64_t oastride, Seed seed, int len, uint32_t* err) {
+  RingLane<T, OP, RUNNING> f{out, seed.first != 0, seed.get<T>()};
+  nrs_ring::run<T, ROWS>(x, g, n_lanes, alen, xastride, out, oastride, (const T*)nullptr, len, err, 10u, f);
 }
 
 // Reduction along lanes (one value per lane): the axis-reduction pipeline.
@@ -1196,6 +1226,27 @@ int launch_lanes(nrs_handle* h, const LaneProblem& p) {
   if (p.alen >= 256 && p.n_lanes >= 64) {
     const int st = launch_lane_tma<T, OP, RUNNING>(h, p);
     if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
+  // The element-copy ring or one thread per lane (see ring_pays in the axis
+  // reductions; a running fold along contiguous lanes also writes a sector
+  // per few elements when a thread owns its row: 100001 x 301 f64 329 / 172
+  // us, and 1000 x 50001 columns 225 / 286).
+  const bool rows = p.xastride == 1, few = p.n_lanes < 20000;
+  if (p.alen >= (rows && (few || RUNNING) ? 64 : 256) && (rows || few)) {
+    RingDims g{};
+    g.n = p.lanes.n;
+    for (int d = 0; d < g.n; ++d) {
+      g.size[d] = p.lanes.size[d];
+      g.xstride[d] = p.lanes.xstride[d];
+      g.ostride[d] = p.lanes.ostride[d];
+    }
+    const int len = nrs_ring::tile_len(sizeof(T), p.n_lanes, h->hw_sms);
+    const size_t smem = nrs_ring::smem_bytes(sizeof(T), rows, len);
+    auto kern = rows ? lane_ring<T, OP, RUNNING, true> : lane_ring<T, OP, RUNNING, false>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<(unsigned)((p.n_lanes + nrs_ring::kLanes - 1) / nrs_ring::kLanes), nrs_ring::kThreads, smem, h->stream>>>(
+        (const T*)p.x, g, p.n_lanes, p.alen, p.xastride, (T*)p.out, p.oastride, p.seed, len, h->dev_error);
+    return nrs_after_launch(h, "lane_ring");
   }
   lane_scan_generic<T, OP, RUNNING><<<grid_for(h, p.n_lanes, 256), 256, 0, h->stream>>>(
       (const T*)p.x, p.lanes, p.n_lanes, p.alen, p.xastride, (T*)p.out, p.oastride, p.seed);

@@ -1,7 +1,9 @@
-"""The slice GEMM's three-word rounding of an element's exact total
-(ozaki_round96) and the slicing of f32 operands without a conversion
-(ozaki_decode), compiled for the host: bit-identical to the 128-bit exact
-path wherever it does not defer, and the same digits as the widened value."""
+"""Integer forms of floating-point steps, compiled for the host: the slice
+GEMM's three-word rounding of an element's exact total (ozaki_round96),
+bit-identical to the 128-bit exact path wherever it does not defer; the
+slicing of f32 operands without a conversion (ozaki_decode), the same digits
+as the widened value's; and the squared deviation of f64 variances
+(nrs_square), the same bits as the product."""
 import ctypes
 import os
 import random
@@ -30,6 +32,16 @@ extern "C" int nrs_test_round96(int32_t R, uint64_t lo, int nd, int e, int* defe
   bad += !sp && (uint32_t)r != (uint32_t)int128_to_float_bits<NrsF32Fmt>(neg, mhi, mlo, e / 8);
   return bad;
 }
+extern "C" int nrs_test_square(double x, int* special) {
+  uint64_t u, w;
+  memcpy(&u, &x, 8);
+  bool sp;
+  const uint64_t r = nrs_square(u, sp);
+  *special = sp;
+  const double d = x * x;
+  memcpy(&w, &d, 8);
+  return !sp && r != w;
+}
 extern "C" int nrs_test_f32_digits(float x, int e, int S) {
   const OzakiZ64 a = ozaki_z64(x, e, 8, S, ozaki_offset64(S, 8)), b = ozaki_z64((double)x, e, 8, S, ozaki_offset64(S, 8));
   int bad = 0;
@@ -52,6 +64,7 @@ def lib(tmp_path_factory):
     dll.nrs_test_round96.argtypes = [ctypes.c_int32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int,
                                      ctypes.POINTER(ctypes.c_int)]
     dll.nrs_test_f32_digits.argtypes = [ctypes.c_float, ctypes.c_int, ctypes.c_int]
+    dll.nrs_test_square.argtypes = [ctypes.c_double, ctypes.POINTER(ctypes.c_int)]
     return dll
 
 
@@ -79,3 +92,17 @@ def test_f32_digits_equal_the_widened_value(lib):
         x = ctypes.c_float(r.uniform(-1, 1) * 2.0 ** r.randrange(-150, 100)).value
         e = max(-148, __import__("math").frexp(x)[1] + r.randrange(0, 12)) if x else 3
         assert lib.nrs_test_f32_digits(x, e, r.randrange(1, 9)) == 0, (x, e)
+
+
+def test_square_equals_the_product(lib):
+    r = random.Random(8)
+    sp = ctypes.c_int(0)
+    for _ in range(60000):
+        m = r.getrandbits(53) | (1 << 52)
+        if r.random() < 0.3:
+            m = (m >> r.randrange(52) << r.randrange(52)) or 1
+        x = float(m) * 2.0 ** r.randrange(-600, 400) * r.choice([-1, 1])
+        assert lib.nrs_test_square(x, ctypes.byref(sp)) == 0, x
+    for x, want in ((0.0, 1), (-0.0, 1), (float("inf"), 1), (float("nan"), 1), (1e200, 1), (1e-170, 1), (5e-324, 1),
+                    (1.0, 0), (-1.5, 0), (1.3e154, 0), (1.6e-154, 0), (1.9999999999999998, 0)):
+        assert lib.nrs_test_square(x, ctypes.byref(sp)) == 0 and sp.value == want, x
