@@ -338,7 +338,7 @@ int nrs_npy_write(nrs_handle* h, const char* path, int dtype, int ndim, const in
 #define NRS_GEMM_TRANS_B 4u    /* B is stored n x k (ldb >= k): a transposed view of B  */
 
 typedef enum nrs_gemm_variant {
-  NRS_GEMM_AUTO = 0,     /* autotuner choice (plain kernels only; never Ozaki) */
+  NRS_GEMM_AUTO = 0,     /* the fastest form for the sizes; see nrs_gemm        */
   NRS_GEMM_DMMA = 1,     /* f64: FP64 tensor-core mma.sync m8n8k4 tiles        */
   NRS_GEMM_SIMT = 2,     /* f32 / f64: register-tiled CUDA-core GEMM           */
   NRS_GEMM_GENERIC = 3,  /* any dtype: one thread per C element (ints, checks) */
@@ -349,10 +349,26 @@ typedef enum nrs_gemm_variant {
  * k x n B, m x n C with leading dimensions lda/ldb/ldc.
  * Replaces kernels::gemm::gemm_2d (src/kernels/gemm.rs:246): m == 0 or
  * n == 0 is a no-op, k == 0 zero-fills C (overwrite contract, :294-302);
- * integer dtypes wrap like gemm_generic (:408). */
+ * integer dtypes wrap like gemm_generic (:408).
+ * NRS_GEMM_AUTO: f64 and f32 products large enough for it run as slice
+ * products on the tensor cores (nrs_gemm_ozaki's scheme, with the slice count
+ * decided on the device: nothing is read back, the call stays asynchronous),
+ * with an error no larger than the plain kernels'; everything else, operands
+ * that the slices cannot carry and calls under stream capture run the plain
+ * kernels. Their scratch is stream-ordered and the library's own. */
 int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A,
              int64_t lda, const void* B, int64_t ldb, void* C, int64_t ldc, unsigned flags,
              int variant);
+
+/* A batch of GEMMs with one shape (Array::matmul on N-D operands,
+ * src/array/linalg.rs:153, batched_gemm :56): C is contiguous, [batch..., m,
+ * n]; panel (i0, i1, ...) of A (B) starts at the sum of i_d * a_strides[d]
+ * (b_strides[d]; elements, 0 for a broadcast axis). Row-major panels with
+ * leading dimensions lda / ldb, or NRS_GEMM_TRANS_A / _B. One launch for all
+ * panels, or panel by panel through nrs_gemm where a panel fills the GPU. */
+int nrs_gemm_batched(nrs_handle* h, int dtype, int batch_ndim, const int64_t* batch_shape, int64_t m, int64_t k,
+                     int64_t n, const void* A, const int64_t* a_strides, int64_t lda, const void* B,
+                     const int64_t* b_strides, int64_t ldb, void* C, unsigned flags);
 
 /* Measures a compute pipe's rate on the handle's device (TFLOP/s, best of
  * three timed launches after a warm-up, CUDA events on the handle's stream;

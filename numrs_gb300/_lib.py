@@ -29,6 +29,7 @@ PLAN_F64_DMMA, PLAN_F64_OZAKI = 0, 1
 PLAN_F32_FMA, PLAN_F32_OZAKI = 0, 1
 RNG_UNIFORM, RNG_NORMAL, RNG_INT, RNG_OZAKI = 0, 1, 2, 3
 TILE_VARIANTS = 6
+MAX_DIMS = 8  # NRS_UFUNC_MAX_DIMS
 
 
 class NpyInfo(C.Structure):
@@ -105,6 +106,7 @@ SIGNATURES = {
     "nrs_npy_write": (_i, [_vp, C.c_char_p, _i, _i, _P64, _vp]),
     "nrs_accumulate": (_i, [_vp, _i, _i, _i, _P64, _P64, _i64, _vp, _vp, _P64]),
     "nrs_gemm": (_i, [_vp, _i, _i64, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _u, _i]),
+    "nrs_gemm_batched": (_i, [_vp, _i, _i, _P64, _i64, _i64, _i64, _vp, _P64, _i64, _vp, _P64, _i64, _vp, _u]),
     "nrs_set_sm_budget": (_i, [_vp, _i]),
     "nrs_test_expire_next_wait": (_i, [_vp, _u32]),
     "nrs_probe_peak": (_i, [_vp, _i, C.POINTER(C.c_double)]),

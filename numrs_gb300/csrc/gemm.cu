@@ -5,7 +5,10 @@
 //                  from shared-memory tiles (GB300's FP64 rate is the bound).
 //  * simt_gemm   : f32 / f64 register-tiled CUDA-core GEMM.
 //  * generic_gemm: one thread per C element, any dtype (integers wrap like
-//                  gemm_generic, src/kernels/gemm.rs:408).
+//                  gemm_generic, src/kernels/gemm.rs:408). Integer products of
+//                  a tile or more run on SIMT tiles (the same wrapped sums).
+//  * batched_gemm: every panel of an N-D product in one launch, on the same
+//                  tiles.
 //
 // Operands are addressed with (row, col) element strides, so transposed views
 // need no copy (the reference copies them in kernels::borrow::operand).
@@ -122,33 +125,37 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM * BN >= 128 * 128 ?
   tile_store<T>(t, C, ldc, m, n, m0, n0, accumulate != 0);
 }
 
-// The 64 x 64 f32 tile with K split over a cluster of gridDim.z CTAs: CTA z
+// A 64 x 64 tile with K split over a cluster of gridDim.z CTAs: CTA z
 // takes k-values [z*kc, min(k, (z+1)*kc)) and leaves its product in shared
 // memory; then every CTA adds a share of the tile's elements over the ranks
 // in order (through distributed shared memory) and writes them. One launch
 // and no scratch, so it needs no workspace shared between streams and runs
 // under capture.
 constexpr int kSplitTile = 64;
-using SplitTile = Simt<float, kSplitTile, kSplitTile, 16, 4, 4>;
-static_assert(SplitTile::kSmem >= kSplitTile * kSplitTile * 4, "the partial tile reuses the operand buffers");
-__global__ void __launch_bounds__(SplitTile::NT, 3)
-    simt_gemm_split(int64_t m, int64_t n, int64_t k, int64_t kc, const float* __restrict__ A, int64_t rsa, int64_t csa,
-                    const float* __restrict__ B, int64_t rsb, int64_t csb, float* __restrict__ C, int64_t ldc,
+template <typename T>
+using SplitTile = Simt<T, kSplitTile, kSplitTile, 16, 4, 4>;
+constexpr int kSplitThreads = SplitTile<float>::NT;
+template <typename T>
+__global__ void __launch_bounds__(kSplitThreads, sizeof(T) == 4 ? 3 : 2)
+    simt_gemm_split(int64_t m, int64_t n, int64_t k, int64_t kc, const T* __restrict__ A, int64_t rsa, int64_t csa,
+                    const T* __restrict__ B, int64_t rsb, int64_t csb, T* __restrict__ C, int64_t ldc,
                     int accumulate, const uint32_t* __restrict__ unless) {
+  using Tile = SplitTile<T>;
+  static_assert(Tile::kSmem >= kSplitTile * kSplitTile * (int)sizeof(T), "the partial tile reuses the operand buffers");
   if (unless && *unless) return;  // (the same word for every CTA of the cluster)
-  __shared__ __align__(16) uint8_t smem[SplitTile::kSmem];
-  SplitTile t;
+  __shared__ __align__(16) uint8_t smem[Tile::kSmem];
+  Tile t;
   const int64_t m0 = (int64_t)blockIdx.y * kSplitTile, n0 = (int64_t)blockIdx.x * kSplitTile;
   const int64_t k0 = (int64_t)blockIdx.z * kc, k1 = (k0 + kc < k) ? k0 + kc : k;
   t.run(A, rsa, csa, B, rsb, csb, m, n, m0, n0, k0, k1, smem);
   const int splits = (int)gridDim.z;
   if (splits == 1) {
-    tile_store<float>(t, C, ldc, m, n, m0, n0, accumulate != 0);
+    tile_store<T>(t, C, ldc, m, n, m0, n0, accumulate != 0);
     return;
   }
-  float* part = reinterpret_cast<float*>(smem);  // (run() ends with a barrier)
+  T* part = reinterpret_cast<T*>(smem);  // (run() ends with a barrier)
 #pragma unroll
-  for (int e = 0; e < SplitTile::kPerThread; ++e) {
+  for (int e = 0; e < Tile::kPerThread; ++e) {
     int r, c;
     t.coords(e, r, c);
     part[r * kSplitTile + c] = t.value(e);
@@ -156,14 +163,14 @@ __global__ void __launch_bounds__(SplitTile::NT, 3)
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
   const int share = kSplitTile * kSplitTile / splits;
-  for (int i = threadIdx.x; i < share; i += SplitTile::NT) {
+  for (int i = threadIdx.x; i < share; i += kSplitThreads) {
     const int idx = (int)blockIdx.z * share + i;
     const int64_t gi = m0 + idx / kSplitTile, gj = n0 + idx % kSplitTile;
     if (gi >= m || gj >= n) continue;
-    float v = cluster.map_shared_rank(part, 0)[idx];
-    for (int z = 1; z < splits; ++z) v += cluster.map_shared_rank(part, z)[idx];
-    float* c = C + gi * ldc + gj;
-    *c = accumulate ? *c + v : v;
+    T v = cluster.map_shared_rank(part, 0)[idx];
+    for (int z = 1; z < splits; ++z) v = tile_add(v, cluster.map_shared_rank(part, z)[idx]);
+    T* c = C + gi * ldc + gj;
+    *c = accumulate ? tile_add(*c, v) : v;
   }
   cluster.sync();  // a CTA's shared memory outlives its readers
 }
@@ -201,6 +208,33 @@ __global__ void generic_gemm(int64_t m, int64_t n, int64_t k, const T* __restric
     T* c = C + i * ldc + j;
     *c = accumulate ? gadd(*c, acc) : acc;
   }
+}
+
+// Every panel of a batch: blockIdx.z + z0 is the panel's row-major index
+// over the batch dimensions, whose strides place its operands.
+constexpr int kMaxBatchDims = NRS_UFUNC_MAX_DIMS;
+struct BatchDims {
+  int n;
+  int64_t size[kMaxBatchDims], a[kMaxBatchDims], b[kMaxBatchDims];
+};
+template <typename T, typename Tile, int BM, int BN, int NT>
+__global__ void __launch_bounds__(NT)
+    batched_gemm(const __grid_constant__ BatchDims g, int64_t z0, int64_t m, int64_t n, int64_t k,
+                 const T* __restrict__ A, int64_t rsa, int64_t csa, const T* __restrict__ B, int64_t rsb, int64_t csb,
+                 T* __restrict__ C) {
+  __shared__ __align__(16) uint8_t smem[Tile::kSmem];
+  const int64_t z = z0 + blockIdx.z;
+  int64_t rem = z, ao = 0, bo = 0;
+  for (int d = g.n - 1; d >= 0; --d) {
+    const int64_t c = rem % g.size[d];
+    rem /= g.size[d];
+    ao += c * g.a[d];
+    bo += c * g.b[d];
+  }
+  Tile t;
+  const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
+  t.run(A + ao, rsa, csa, B + bo, rsb, csb, m, n, m0, n0, 0, k, smem);
+  tile_store<T>(t, C + z * m * n, n, m, n, m0, n0, false);
 }
 
 template <typename T>
@@ -247,10 +281,10 @@ struct F32Plan {
   int64_t kc;
   double us;
 };
-F32Plan plan_f32(int64_t m, int64_t n, int64_t k) {
+// 64 x 64 tiles alone; us as for f32.
+F32Plan plan_split(int64_t m, int64_t n, int64_t k) {
   auto waves = [](double ctas) { return std::ceil(ctas / NRS_PLAN_SMS); };
-  const double t128 = (double)((m + 127) / 128) * (double)((n + 127) / 128);
-  F32Plan best{128, 1, k, 4.0 + waves(t128) * (double)k * (128.0 * 128.0 / 1.45e5)};
+  F32Plan best{64, 1, k, 1e300};
   const double t64 = (double)((m + 63) / 64) * (double)((n + 63) / 64);
   for (int z = 1; z <= 8; z *= 2) {
     const int64_t kc = ((k + z - 1) / z + 15) / 16 * 16;
@@ -260,14 +294,21 @@ F32Plan plan_f32(int64_t m, int64_t n, int64_t k) {
   }
   return best;
 }
+F32Plan plan_f32(int64_t m, int64_t n, int64_t k) {
+  const double t128 = (double)((m + 127) / 128) * (double)((n + 127) / 128);
+  const F32Plan large{128, 1, k, 4.0 + std::ceil(t128 / NRS_PLAN_SMS) * (double)k * (128.0 * 128.0 / 1.45e5)};
+  const F32Plan split = plan_split(m, n, k);
+  return split.us < large.us ? split : large;
+}
 
-void launch_simt_split(nrs_handle* h, const F32Plan& pl, int64_t m, int64_t k, int64_t n, const float* A, int64_t rsa,
-                       int64_t csa, const float* B, int64_t rsb, int64_t csb, float* C, int64_t ldc, int acc,
+template <typename T>
+void launch_simt_split(nrs_handle* h, const F32Plan& pl, int64_t m, int64_t k, int64_t n, const T* A, int64_t rsa,
+                       int64_t csa, const T* B, int64_t rsb, int64_t csb, T* C, int64_t ldc, int acc,
                        const uint32_t* unless) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = tiles(m, n, kSplitTile, kSplitTile);
   cfg.gridDim.z = (unsigned)pl.splits;
-  cfg.blockDim = dim3(SplitTile::NT);
+  cfg.blockDim = dim3(kSplitThreads);
   cfg.stream = h->stream;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -276,7 +317,7 @@ void launch_simt_split(nrs_handle* h, const F32Plan& pl, int64_t m, int64_t k, i
   attr.val.clusterDim.z = (unsigned)pl.splits;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, simt_gemm_split, m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
+  cudaLaunchKernelEx(&cfg, simt_gemm_split<T>, m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
 }
 
 void launch_simt_f32(nrs_handle* h, bool large, int64_t m, int64_t k, int64_t n, const float* A, int64_t rsa,
@@ -337,7 +378,21 @@ int nrs_plain_gemm_launch(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
   if (grid_too_large(m, n)) variant = NRS_GEMM_GENERIC;
   if (variant == NRS_GEMM_AUTO) {
     if (dtype == NRS_F64) variant = NRS_GEMM_DMMA;
-    else if (dtype != NRS_F32) variant = NRS_GEMM_GENERIC;
+    else if (dtype != NRS_F32 && m * n < 1024) variant = NRS_GEMM_GENERIC;
+  }
+  // Integers from a 32 x 32 C on: tiles read each operand element once per 64
+  // products, one thread per element reads two per product; a split K fills
+  // the GPU (i64, us, one thread per element / tiles: 1000^3 657 / 308,
+  // 300 x 1000 x 257 174 / 57).
+  if (variant == NRS_GEMM_AUTO && dtype == NRS_I64) {
+    launch_simt_split(h, plan_split(m, n, k), m, k, n, (const int64_t*)A, rsa, csa, (const int64_t*)B, rsb, csb,
+                      (int64_t*)C, ldc, acc, nullptr);
+    return nrs_after_launch(h, "simt_gemm_split<i64>");
+  }
+  if (variant == NRS_GEMM_AUTO && dtype == NRS_I32) {
+    launch_simt_split(h, plan_split(m, n, k), m, k, n, (const int32_t*)A, rsa, csa, (const int32_t*)B, rsb, csb,
+                      (int32_t*)C, ldc, acc, nullptr);
+    return nrs_after_launch(h, "simt_gemm_split<i32>");
   }
   if (variant == NRS_GEMM_AUTO) {
     launch_auto_f32(h, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb, csb, (float*)C, ldc, acc, nullptr);
@@ -433,6 +488,104 @@ extern "C" int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t 
   const int64_t rsb = tb ? 1 : ldb, csb = tb ? ldb : 1;
   return nrs_plain_gemm_launch(h, dtype, m, k, n, A, rsa, csa, B, rsb, csb, C, ldc, accumulate,
                                variant);
+}
+
+namespace {
+
+// 64 x 64 tiles (weight 4) or 32 x 32: the one whose busiest SM has less to do.
+bool large_tiles(int64_t m, int64_t n, int64_t batch) {
+  const double t64 = (double)((m + 63) / 64) * (double)((n + 63) / 64) * (double)batch;
+  const double t32 = (double)((m + 31) / 32) * (double)((n + 31) / 32) * (double)batch;
+  return std::ceil(t64 / NRS_PLAN_SMS) * 4.0 <= std::ceil(t32 / NRS_PLAN_SMS);
+}
+
+template <typename T, typename Tile, int BM, int BN, int NT>
+void launch_batched(nrs_handle* h, const BatchDims& g, int64_t batch, int64_t m, int64_t k, int64_t n, const void* A,
+                    int64_t rsa, int64_t csa, const void* B, int64_t rsb, int64_t csb, void* C) {
+  for (int64_t z0 = 0; z0 < batch; z0 += 65535) {
+    dim3 grid = tiles(m, n, BM, BN);
+    grid.z = (unsigned)(batch - z0 < 65535 ? batch - z0 : 65535);
+    batched_gemm<T, Tile, BM, BN, NT><<<grid, NT, 0, h->stream>>>(g, z0, m, n, k, (const T*)A, rsa, csa, (const T*)B,
+                                                                  rsb, csb, (T*)C);
+  }
+}
+
+}  // namespace
+
+extern "C" int nrs_gemm_batched(nrs_handle* h, int dtype, int batch_ndim, const int64_t* batch_shape, int64_t m,
+                                int64_t k, int64_t n, const void* A, const int64_t* a_strides, int64_t lda,
+                                const void* B, const int64_t* b_strides, int64_t ldb, void* C, unsigned flags) {
+  if (!h) return NRS_ERR_INVALID;
+  h->last_error.clear();
+  if (batch_ndim < 0 || batch_ndim > kMaxBatchDims || (batch_ndim && (!batch_shape || !a_strides || !b_strides)))
+    return nrs_fail(h, NRS_ERR_INVALID, "bad batch dimensions");
+  if (m < 0 || k < 0 || n < 0) return nrs_fail(h, NRS_ERR_SHAPE, "negative GEMM dimension");
+  const size_t es = nrs_dtype_size(dtype);
+  if (!es) return nrs_fail(h, NRS_ERR_DTYPE, "unknown dtype");
+  if (flags & ~(NRS_GEMM_TRANS_A | NRS_GEMM_TRANS_B)) return nrs_fail(h, NRS_ERR_INVALID, "unknown GEMM flag");
+  const bool ta = flags & NRS_GEMM_TRANS_A, tb = flags & NRS_GEMM_TRANS_B;
+  if (lda < ((ta ? m : k) > 0 ? (ta ? m : k) : 1)) return nrs_fail(h, NRS_ERR_SHAPE, "lda too small");
+  if (ldb < ((tb ? k : n) > 0 ? (tb ? k : n) : 1)) return nrs_fail(h, NRS_ERR_SHAPE, "ldb too small");
+  BatchDims g{};
+  g.n = batch_ndim;
+  int64_t batch = 1;
+  for (int d = 0; d < batch_ndim; ++d) {
+    if (batch_shape[d] < 0) return nrs_fail(h, NRS_ERR_SHAPE, "negative dimension");
+    if (a_strides[d] < 0 || b_strides[d] < 0) return nrs_fail(h, NRS_ERR_STRIDE, "negative stride");
+    g.size[d] = batch_shape[d];
+    g.a[d] = a_strides[d];
+    g.b[d] = b_strides[d];
+    batch *= batch_shape[d];
+  }
+  if (batch == 0 || m == 0 || n == 0) return NRS_OK;
+  if (!C || (k > 0 && (!A || !B))) return nrs_fail(h, NRS_ERR_INVALID, "null operand");
+  if (k == 0) return nrs_gemm(h, dtype, batch * m, 0, n, A, 1, B, n, C, n, 0, NRS_GEMM_AUTO);
+  int st = nrs_cuda_check(h, cudaSetDevice(h->device), "cudaSetDevice");
+  if (st) return st;
+  // A panel that fills the GPU by itself has the single product's choice of
+  // kernels (slice products among them).
+  const bool fills = (double)((m + 127) / 128) * (double)((n + 127) / 128) >= NRS_PLAN_SMS ||
+                     (dtype == NRS_F64 && nrs_tc_gemm_pays(NRS_F64, m, k, n));
+  if (batch == 1 || fills || grid_too_large(m, n)) {
+    const size_t panel = (size_t)m * (size_t)n * es;
+    for (int64_t z = 0; z < batch; ++z) {
+      int64_t rem = z, ao = 0, bo = 0;
+      for (int d = batch_ndim - 1; d >= 0; --d) {
+        const int64_t c = rem % g.size[d];
+        rem /= g.size[d];
+        ao += c * g.a[d];
+        bo += c * g.b[d];
+      }
+      if ((st = nrs_gemm(h, dtype, m, k, n, (const uint8_t*)A + ao * (int64_t)es, lda,
+                         (const uint8_t*)B + bo * (int64_t)es, ldb, (uint8_t*)C + z * panel, n, flags, NRS_GEMM_AUTO)))
+        return st;
+    }
+    return NRS_OK;
+  }
+  const int64_t rsa = ta ? 1 : lda, csa = ta ? lda : 1;
+  const int64_t rsb = tb ? 1 : ldb, csb = tb ? ldb : 1;
+  const bool big = large_tiles(m, n, batch);
+  // One launch over (tiles, panels); a 32 x 96 x 80 x 112 f64 batch: 1.45 ms
+  // as a plan built per call from one descriptor per panel, 0.07 ms here (the FP64
+  // pipe takes 0.06 for the padded tiles).
+#define NRS_BATCH(T, TILE, BM, NT) \
+  launch_batched<T, TILE, BM, BM, NT>(h, g, batch, m, k, n, A, rsa, csa, B, rsb, csb, C)
+  using F32L = Simt<float, 64, 64, 16, 4, 4>;
+  using F32S = Simt<float, 32, 32, 16, 2, 2>;
+  using F64L = Dmma<64, 64, 2, 4>;
+  using F64S = Dmma<32, 32, 2, 2>;
+  using I64L = Simt<int64_t, 64, 64, 8, 4, 4>;
+  using I64S = Simt<int64_t, 32, 32, 16, 2, 2>;
+  using I32L = Simt<int32_t, 64, 64, 16, 4, 4>;
+  using I32S = Simt<int32_t, 32, 32, 16, 2, 2>;
+  switch (dtype) {
+    case NRS_F32: big ? NRS_BATCH(float, F32L, 64, 256) : NRS_BATCH(float, F32S, 32, 256); break;
+    case NRS_F64: big ? NRS_BATCH(double, F64L, 64, 256) : NRS_BATCH(double, F64S, 32, 128); break;
+    case NRS_I64: big ? NRS_BATCH(int64_t, I64L, 64, 256) : NRS_BATCH(int64_t, I64S, 32, 256); break;
+    default: big ? NRS_BATCH(int32_t, I32L, 64, 256) : NRS_BATCH(int32_t, I32S, 32, 256); break;
+  }
+#undef NRS_BATCH
+  return nrs_after_launch(h, "batched_gemm");
 }
 
 // ---------------------------------------------------------------------------

@@ -205,6 +205,22 @@ struct SimtLoader {
   }
 };
 
+// a * b + c: one rounding for floats, wrapping for integers.
+__device__ __forceinline__ float tile_fma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double tile_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ int64_t tile_fma(int64_t a, int64_t b, int64_t c) {
+  return (int64_t)((unsigned long long)a * (unsigned long long)b + (unsigned long long)c);
+}
+__device__ __forceinline__ int32_t tile_fma(int32_t a, int32_t b, int32_t c) {
+  return (int32_t)((unsigned)a * (unsigned)b + (unsigned)c);
+}
+__device__ __forceinline__ float tile_add(float a, float b) { return a + b; }
+__device__ __forceinline__ double tile_add(double a, double b) { return a + b; }
+__device__ __forceinline__ int64_t tile_add(int64_t a, int64_t b) {
+  return (int64_t)((unsigned long long)a + (unsigned long long)b);
+}
+__device__ __forceinline__ int32_t tile_add(int32_t a, int32_t b) { return (int32_t)((unsigned)a + (unsigned)b); }
+
 template <typename T, int BM, int BN, int BK, int TM, int TN>
 struct Simt {
   static constexpr int NT = (BM / TM) * (BN / TN);
@@ -257,13 +273,13 @@ struct Simt {
         if constexpr (kVec) {
 #pragma unroll
           for (int g = 0; g < TM / 4; ++g) {
-            const float4 v = *reinterpret_cast<const float4*>(&As[buf][kk][row_of(tr, 4 * g)]);
-            a[4 * g] = v.x, a[4 * g + 1] = v.y, a[4 * g + 2] = v.z, a[4 * g + 3] = v.w;
+            const uint4 v = *reinterpret_cast<const uint4*>(&As[buf][kk][row_of(tr, 4 * g)]);
+            memcpy(&a[4 * g], &v, 16);
           }
 #pragma unroll
           for (int g = 0; g < TN / 4; ++g) {
-            const float4 v = *reinterpret_cast<const float4*>(&Bs[buf][kk][col_of(tc, 4 * g)]);
-            b[4 * g] = v.x, b[4 * g + 1] = v.y, b[4 * g + 2] = v.z, b[4 * g + 3] = v.w;
+            const uint4 v = *reinterpret_cast<const uint4*>(&Bs[buf][kk][col_of(tc, 4 * g)]);
+            memcpy(&b[4 * g], &v, 16);
           }
         } else {
 #pragma unroll
@@ -274,7 +290,7 @@ struct Simt {
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+          for (int j = 0; j < TN; ++j) acc[i][j] = tile_fma(a[i], b[j], acc[i][j]);
       }
       if (kt + 1 < ktiles) {
         la.store(As[buf ^ 1]);
@@ -305,7 +321,7 @@ __device__ __forceinline__ void tile_store(const Tile& t, T* __restrict__ C, int
     if (gi < m && gj < n) {
       T* p = C + gi * ldc + gj;
       const T v = (T)t.value(e);
-      *p = accumulate ? (*p + v) : v;
+      *p = accumulate ? tile_add(*p, v) : v;
     }
   }
 }

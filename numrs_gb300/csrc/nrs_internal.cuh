@@ -106,6 +106,8 @@ int nrs_plain_gemm_unless(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
 int nrs_dmma_splits(int64_t m, int64_t k, int64_t n);
 // Modelled time of the FP32 kernels for a product.
 double nrs_plain_f32_us(int64_t m, int64_t k, int64_t n);
+// Whether a product is faster as slice products (by sizes alone).
+bool nrs_tc_gemm_pays(int dtype, int64_t m, int64_t k, int64_t n);
 int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
                      const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate);
 

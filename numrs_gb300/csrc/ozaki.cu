@@ -2111,21 +2111,25 @@ __global__ void __launch_bounds__(256)
 // f32 against the FP32 kernels (us): 1024^3 76 / 100, 1536^3 182 / 137,
 // 2048^3 418 / 246, 4096^3 3214 / 1241 (0.11 PFLOP/s; error 4e-9 of
 // (|A||B|)_ij against the FMA chains' 3e-7).
-int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
-                     const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate) {
-  if (!h->pool || (dtype != NRS_F64 && dtype != NRS_F32)) return NRS_ERR_UNSUPPORTED;
+bool nrs_tc_gemm_pays(int dtype, int64_t m, int64_t k, int64_t n) {
+  if (dtype != NRS_F64 && dtype != NRS_F32) return false;
   const bool f32 = dtype == NRS_F32;
-  if (m > (1LL << 24) || n > (1LL << 24) || k > (1LL << 24)) return NRS_ERR_UNSUPPORTED;
+  if (m > (1LL << 24) || n > (1LL << 24) || k > (1LL << 24)) return false;
   const double mk = (double)m * k, kn = (double)k * n;
   const double plain_us = f32 ? nrs_plain_f32_us(m, k, n)
                               : (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * 2.0 / 1.05e6 + 10.0;
-  if (plain_us < 60.0) return NRS_ERR_UNSUPPORTED;
+  if (plain_us < 60.0) return false;
   // exponents, estimate, slicing: seven launches, 40 (f32: 16) bytes per
   // operand element
   const int S = f32 ? 4 : 7;
   const double tc_us = 45.0 + (mk + kn) * (f32 ? 16.0 : 40.0) / 3e6 +
                        plan_tc(m, n, (k + 7) / 8 * 8, S).us * (1.0 + 2.0 / (S * (S + 1)));
-  if (tc_us > 0.9 * plain_us) return NRS_ERR_UNSUPPORTED;
+  return tc_us <= 0.9 * plain_us;
+}
+
+int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
+                     const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate) {
+  if (!h->pool || !nrs_tc_gemm_pays(dtype, m, k, n)) return NRS_ERR_UNSUPPORTED;
   // Under stream capture the plain kernel runs, as its launches hold no
   // allocation.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -2136,7 +2140,7 @@ int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, 
   if (cap != cudaStreamCaptureStatusNone) return NRS_ERR_UNSUPPORTED;
   const OzOperand a{A, lda, m, !ta};
   const OzOperand bT{B, ldb, n, tb};
-  return f32 ? tc_gemm<float>(h, a, bT, m, k, n, C, ldc, accumulate)
+  return dtype == NRS_F32 ? tc_gemm<float>(h, a, bT, m, k, n, C, ldc, accumulate)
              : tc_gemm<double>(h, a, bT, m, k, n, C, ldc, accumulate);
 }
 

@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import builtins as _bi
 import ctypes as C
+import itertools
 import threading
 
 import torch
@@ -299,10 +300,10 @@ def save_npy(path: str, t: torch.Tensor) -> None:
 # GEMM
 # ---------------------------------------------------------------------------
 def _mat_strides(t: torch.Tensor):
-    """(leading dim, transposed?) for a 2-D operand, or None if neither
+    """(leading dim, transposed?) for the last two axes, or None if neither
     row- nor column-contiguous."""
-    r, c = t.stride()
-    rows, cols = t.shape
+    r, c = t.stride()[-2:]
+    rows, cols = t.shape[-2:]
     if c == 1 or cols <= 1:
         return (r if rows > 1 else _bi.max(cols, 1)), False
     if r == 1 or rows <= 1:
@@ -322,6 +323,12 @@ def gemm_2d(m: int, k: int, n: int, a: torch.Tensor, b: torch.Tensor, c: torch.T
     st = lib.nrs_gemm(h, dtype_code(c), m, k, n, _ptr(a), _bi.max(k, 1), _ptr(b), _bi.max(n, 1),
                       _ptr(c), _bi.max(n, 1), flags, variant)
     L.check(st, h)
+
+
+def _batch_strides(t: torch.Tensor, batch) -> list[int]:
+    """Strides of the axes before the last two over `batch` (0 where broadcast)."""
+    own = [0 if d == 1 else s for d, s in zip(t.shape[:-2], t.stride())]
+    return [0] * (len(batch) - len(own)) + own
 
 
 def _logical_copy(t: torch.Tensor) -> torch.Tensor:
@@ -363,7 +370,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, variant: int = L.GEMM_AUTO) -> torc
     GEMM; otherwise a 1-D operand becomes [1, k] (left) or [k, 1] (right) and
     stays so in the result (the reference does not squeeze it), the batch
     axes broadcast by NumPy's rules, and every panel is one GEMM of the batch
-    (batched_gemm, :56-136; f32/f64 panels run as one grouped launch).
+    (batched_gemm, :56-136), all in one nrs_gemm_batched call.
     0-D operands raise DimensionMismatch; mismatched inner or batch
     dimensions raise ShapeMismatch."""
     _need_cuda(a, b)
@@ -384,33 +391,38 @@ def matmul(a: torch.Tensor, b: torch.Tensor, variant: int = L.GEMM_AUTO) -> torc
     if a.shape[-1] != b.shape[-2]:
         raise L.ShapeMismatch(L.ERR_SHAPE, f"matmul: {tuple(a.shape)} @ {tuple(b.shape)}")
     m, k, n = a.shape[-2], a.shape[-1], b.shape[-1]
-    try:
-        batch = torch.broadcast_shapes(a.shape[:-2], b.shape[:-2])
-    except RuntimeError:
-        raise L.ShapeMismatch(L.ERR_SHAPE, f"matmul batch axes: {tuple(a.shape)} @ {tuple(b.shape)}") from None
+    batch = []
+    for da, db in itertools.zip_longest(reversed(a.shape[:-2]), reversed(b.shape[:-2]), fillvalue=1):
+        if da != db and da != 1 and db != 1:
+            raise L.ShapeMismatch(L.ERR_SHAPE, f"matmul batch axes: {tuple(a.shape)} @ {tuple(b.shape)}")
+        batch.insert(0, db if da == 1 else da)
     out = torch.empty((*batch, m, n), dtype=a.dtype, device=a.device)
     if len(batch) == 0:
         _gemm_views(a, b, out, False, variant)
         return out
-    # Broadcast operands are stride-0 views, not copies: each panel is a
-    # view of the original operand (the reference materialises them,
-    # Array::broadcast_to, before borrowing the flat panels).
+    if variant == L.GEMM_AUTO and len(batch) <= L.MAX_DIMS:
+        # Row- or column-contiguous panels go as they are (broadcast axes by
+        # a stride of 0, which the reference materialises,
+        # Array::broadcast_to); other operands are copied once.
+        sa, sb = _mat_strides(a), _mat_strides(b)
+        if sa is None:
+            a = _logical_copy(a)
+            sa = (_bi.max(k, 1), False)
+        if sb is None:
+            b = _logical_copy(b)
+            sb = (_bi.max(n, 1), False)
+        lib = L.load()
+        h = handle(out.device.index)
+        flags = (L.GEMM_TRANS_A if sa[1] else 0) | (L.GEMM_TRANS_B if sb[1] else 0)
+        st = lib.nrs_gemm_batched(h, dtype_code(out), len(batch), L.i64_array(batch), m, k, n, _ptr(a),
+                                  L.i64_array(_batch_strides(a, batch)), sa[0], _ptr(b),
+                                  L.i64_array(_batch_strides(b, batch)), sb[0], _ptr(out), flags)
+        L.check(st, h)
+        return out
     ab = a.expand(*batch, m, k)
     bb = b.expand(*batch, k, n)
-    panels = []
-    for idx in range(out[..., 0, 0].numel()):
-        bi = torch.unravel_index(torch.tensor(idx), batch)
-        bi = tuple(int(x) for x in bi)
-        panels.append((ab[bi], bb[bi], out[bi]))
-    grouped_ok = a.dtype in (torch.float32, torch.float64) and variant == L.GEMM_AUTO and all(
-        _mat_strides(p[0]) is not None and _mat_strides(p[1]) is not None for p in panels)
-    if grouped_ok and m > 0 and n > 0:
-        plan = Plan([(pa, pb, pc, False) for pa, pb, pc in panels])
-        plan.run(use_graph=False)
-        plan.close()
-    else:
-        for pa, pb, pc in panels:
-            _gemm_views(pa, pb, pc, False, variant)
+    for idx in itertools.product(*(range(d) for d in batch)):
+        _gemm_views(ab[idx], bb[idx], out[idx], False, variant)
     return out
 
 
