@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(WM * WN * 32)
               int64_t csa, const double* __restrict__ B, int64_t rsb, int64_t csb,
               double* __restrict__ C, int64_t ldc, int accumulate, double* __restrict__ P,
               const uint32_t* __restrict__ unless) {
+  launch_wait();
+  launch_next();
   if (unless && *unless) return;
   using Tile = Dmma<BM, BN, WM, WN>;
   __shared__ __align__(16) uint8_t smem[Tile::kSmem];
@@ -57,6 +59,7 @@ template <typename T>
 __global__ void splitk_finish(const double* __restrict__ P, int splits, int64_t m, int64_t n,
                               T* __restrict__ C, int64_t ldc, int accumulate, const uint32_t* __restrict__ choice,
                               int splits_if) {
+  launch_wait();
   if (choice && *choice) splits = splits_if;
   if (splits <= 1) return;
   const int64_t mn = m * n;
@@ -116,6 +119,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM * BN >= 128 * 128 ?
     simt_gemm(int64_t m, int64_t n, int64_t k, const T* __restrict__ A, int64_t rsa, int64_t csa,
               const T* __restrict__ B, int64_t rsb, int64_t csb, T* __restrict__ C, int64_t ldc,
               int accumulate, const uint32_t* __restrict__ unless) {
+  launch_wait();
+  launch_next();
   if (unless && *unless) return;
   using Tile = Simt<T, BM, BN, BK, TM, TN>;
   __shared__ __align__(16) uint8_t smem[Tile::kSmem];
@@ -142,6 +147,8 @@ __global__ void __launch_bounds__(kSplitThreads, sizeof(T) == 4 ? 3 : 2)
                     int accumulate, const uint32_t* __restrict__ unless) {
   using Tile = SplitTile<T>;
   static_assert(Tile::kSmem >= kSplitTile * kSplitTile * (int)sizeof(T), "the partial tile reuses the operand buffers");
+  launch_wait();
+  launch_next();
   if (unless && *unless) return;  // (the same word for every CTA of the cluster)
   __shared__ __align__(16) uint8_t smem[Tile::kSmem];
   Tile t;
@@ -259,9 +266,11 @@ void launch_dmma(nrs_handle* h, const DmmaPlan& pl, int64_t m, int64_t k, int64_
   dim3 g = tiles(m, n, pl.tile, pl.tile);
   g.z = (unsigned)pl.splits;
   if (pl.tile == 64)
-    dmma_gemm<64, 64, 2, 4><<<g, 256, 0, h->stream>>>(m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, P, unless);
+    nrs_launch_after(unless != nullptr, dmma_gemm<64, 64, 2, 4>, g, 256, 0, h->stream, m, n, k, pl.kc, A, rsa, csa, B,
+                     rsb, csb, C, ldc, acc, P, unless);
   else
-    dmma_gemm<32, 32, 2, 2><<<g, 128, 0, h->stream>>>(m, n, k, pl.kc, A, rsa, csa, B, rsb, csb, C, ldc, acc, P, unless);
+    nrs_launch_after(unless != nullptr, dmma_gemm<32, 32, 2, 2>, g, 128, 0, h->stream, m, n, k, pl.kc, A, rsa, csa, B,
+                     rsb, csb, C, ldc, acc, P, unless);
 }
 
 int finish_grid(nrs_handle* h, int64_t m, int64_t n) {
@@ -324,8 +333,8 @@ void launch_simt_f32(nrs_handle* h, bool large, int64_t m, int64_t k, int64_t n,
                      int64_t csa, const float* B, int64_t rsb, int64_t csb, float* C, int64_t ldc, int acc,
                      const uint32_t* unless) {
   if (large)
-    simt_gemm<float, 128, 128, 8, 8, 8><<<tiles(m, n, 128, 128), 256, 0, h->stream>>>(m, n, k, A, rsa, csa, B, rsb,
-                                                                                      csb, C, ldc, acc, unless);
+    nrs_launch_after(unless != nullptr, simt_gemm<float, 128, 128, 8, 8, 8>, tiles(m, n, 128, 128), 256, 0, h->stream, m,
+                     n, k, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
   else
     simt_gemm<float, 32, 32, 16, 2, 2><<<tiles(m, n, 32, 32), 256, 0, h->stream>>>(m, n, k, A, rsa, csa, B, rsb, csb,
                                                                                    C, ldc, acc, unless);
@@ -358,13 +367,13 @@ int nrs_plain_gemm_unless(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
     launch_dmma(h, pl, m, k, n, (const double*)A, rsa, csa, (const double*)B, rsb, csb, (double*)C, ldc, acc, slab,
                 unless);
     if (pl.splits > 1 || tc_splits > 1)
-      splitk_finish<double><<<finish_grid(h, m, n), 256, 0, h->stream>>>(slab, pl.splits, m, n, (double*)C, ldc, acc,
-                                                                         unless, tc_splits);
+      nrs_launch_after(true, splitk_finish<double>, finish_grid(h, m, n), 256, 0, h->stream, slab, pl.splits, m, n,
+                       (double*)C, ldc, acc, unless, tc_splits);
   } else {
     launch_auto_f32(h, m, k, n, (const float*)A, rsa, csa, (const float*)B, rsb, csb, (float*)C, ldc, acc, unless);
     if (tc_splits > 1)
-      splitk_finish<float><<<finish_grid(h, m, n), 256, 0, h->stream>>>(slab, 1, m, n, (float*)C, ldc, acc, unless,
-                                                                        tc_splits);
+      nrs_launch_after(true, splitk_finish<float>, finish_grid(h, m, n), 256, 0, h->stream, slab, 1, m, n, (float*)C,
+                       ldc, acc, unless, tc_splits);
   }
   return nrs_after_launch(h, "plain GEMM behind the slice products");
 }

@@ -111,6 +111,26 @@ bool nrs_tc_gemm_pays(int dtype, int64_t m, int64_t k, int64_t n);
 int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A, int64_t lda, bool ta,
                      const void* B, int64_t ldb, bool tb, void* C, int64_t ldc, bool accumulate);
 
+// Launches `kern` as a programmatic dependent of the previous kernel on the
+// stream (`after`), or plainly; a captured launch is always a plain one.
+template <typename... KArgs, typename... Args>
+inline cudaError_t nrs_launch_after(bool after, void (*kern)(KArgs...), dim3 grid, unsigned threads, size_t smem,
+                                    cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (after && cudaStreamIsCapturing(s, &cap) != cudaSuccess) return cudaGetLastError();
+  cfg.numAttrs = after && cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // Device helpers: mbarrier and TMA (inline PTX, sm_90+ forms valid on sm_103a)
 // ---------------------------------------------------------------------------
@@ -156,6 +176,14 @@ NRS_DEV void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
 NRS_DEV void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+
+// Programmatic dependent launch: a kernel launched with nrs_launch_after may
+// be scheduled while the one before it on the stream drains; nothing of
+// global memory is touched before launch_wait(), which every thread calls
+// first (so completion stays transitive), and the kernel before it lets the
+// next one in with launch_next().
+NRS_DEV void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+NRS_DEV void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // One try_wait probe on `phase`; true once the phase has completed.
 NRS_DEV bool mbar_try_wait(uint64_t* bar, uint32_t phase) {

@@ -567,9 +567,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   // (warp-uniform, and known to be)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n_tiles = G ? P.n_tiles : P.tiles_m * P.tiles_n;
-  const int S = P.count ? (int)__ldcg(P.count) : P.slices;
-  if (S == 0) return;  // (the same words for every thread)
-  const int final_shift = 2 - 2 * P.digit_bits - P.digit_bits * (S - 1);
+  launch_next();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Geo::STAGES; ++s) {
@@ -594,6 +592,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+
+  // (the barriers and TMEM are set up while the kernel before drains)
+  launch_wait();
+  const int S = P.count ? (int)__ldcg(P.count) : P.slices;
+  if (S == 0) {  // (the same word for every thread)
+    if (warp == 1) tmem_dealloc(tmem_base, OZ_TMEM_COLS);
+    return;
+  }
+  const int final_shift = 2 - 2 * P.digit_bits - P.digit_bits * (S - 1);
 
   auto bounded = [&](uint64_t* bar, uint32_t phase, uint32_t site) -> bool {
     for (uint32_t i = 0; i < NRS_WAIT_LIMIT; ++i) {
@@ -703,6 +710,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     // (ra_i + cb_j) 2^96, the operands' 2^48 scale factors); D = 0 gives
     // +inf unless the numerator is 0 too (every product then has a zero
     // factor and the result is exact). The running max is float bits.
+    __shared__ float est_cb[EST ? 8 : 1][EST ? OZ_BN / 2 : 1];
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     const int row_in_tile = q * 32 + lane;
@@ -719,6 +727,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const int64_t col0 = tc.col0 + half * (OZ_BN / 2);
       const float ra = row_ok ? (float)P.ra[row] : 0.0f;
       const bool pass1 = P.slices == 1;
+      // this warp's column sums, read while the product runs
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < OZ_BN / 2; j += 32) {
+        const int64_t col = col0 + j + lane;
+        est_cb[warp - 2][j + lane] = pass1 && col < tc.n ? (float)P.cb[col] : 0.0f;
+      }
+      __syncwarp();
       PairIter pr;
       pr.start(S);
       for (int u = 0; u < tc.n_pairs; ++u, ++ai, pr.next(1)) {
@@ -747,7 +763,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int64_t col = col0 + c * 16 + e;
             const float D = __uint_as_float(v[e]);
             float num, r;
-            if (pass1) num = (ra + (float)(col < tc.n ? P.cb[col] : 0u)) * (0x1p96f * P.sum_unit);
+            if (pass1) num = (ra + est_cb[warp - 2][c * 16 + e]) * (0x1p96f * P.sum_unit);
             else num = __uint_as_float(w[e]);
             // (the threshold test of the count tolerates the approximate
             // division's two ulp)
@@ -1195,6 +1211,8 @@ __device__ __forceinline__ void load_run(const T* src, bool vec, int64_t left, T
 // the decision words and the column sums that oz_est adds into.
 template <typename T>
 __global__ void __launch_bounds__(256) oz_max(OzPrep<T> a, OzPrep<T> bT, int64_t k, uint32_t* __restrict__ words) {
+  launch_wait();
+  launch_next();
   if (blockIdx.x == 0 && threadIdx.x < OZ_WORDS) words[threadIdx.x] = 0;
   const bool first = blockIdx.x < a.blocks;
   const OzPrep<T>& o = first ? a : bT;
@@ -1311,6 +1329,8 @@ __device__ __forceinline__ void raise_word(uint32_t* w, uint32_t v) {
 template <typename T, bool PASS2>
 __global__ void __launch_bounds__(256)
     oz_est(OzPrep<T> a, OzPrep<T> bT, int64_t k, int64_t kpad, float scale, uint32_t* __restrict__ words) {
+  launch_wait();
+  launch_next();
   __shared__ uint32_t tile[PASS2 ? 2 : 1][kSliceColN][kSliceColPitch];
   __shared__ float csum[8][kSliceColN];
   __shared__ uint32_t cexp[8][32];
@@ -1481,6 +1501,8 @@ __global__ void __launch_bounds__(256)
     oz_slice(OzPrep<T> a, OzPrep<T> bT, int64_t k, int64_t kpad, int S_given, uint32_t* decide, OzRule rule) {
   __shared__ uint32_t tile[kSliceSet * kSliceColN * kSliceColPitch];
   __shared__ uint32_t cexp[8][32];
+  launch_wait();
+  launch_next();
   const int S = decide ? oz_decide(decide, rule) : S_given;
   if (decide && blockIdx.x == 0 && threadIdx.x == 0) decide[OZ_W_COUNT] = (uint32_t)S;
   if (S == 0) return;
@@ -1633,11 +1655,9 @@ int launch_oz_est(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_
   qa.blocks = blocks(qa);
   qb.blocks = blocks(qb);
   const float scale = oz_sum_scale(k);
-  if (pass2)
-    oz_est<T, true><<<qa.blocks + qb.blocks, 256, 0, h->stream>>>(qa, qb, k, kpad, scale, w.words);
-  else
-    oz_est<T, false><<<qa.blocks + qb.blocks, 256, 0, h->stream>>>(qa, qb, k, kpad, scale, w.words);
-  return nrs_after_launch(h, "oz_est");
+  return nrs_cuda_check(h, nrs_launch_after(true, pass2 ? oz_est<T, true> : oz_est<T, false>, qa.blocks + qb.blocks, 256,
+                                            0, h->stream, qa, qb, k, kpad, scale, w.words),
+                        "oz_est");
 }
 
 // decide != null: the count is decided on the device under `rule`.
@@ -1653,13 +1673,9 @@ int launch_oz_slice(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int6
   qa.blocks = blocks(qa);
   qb.blocks = blocks(qb);
   const unsigned grid = qa.blocks + qb.blocks;
-  if (b == 8)
-    oz_slice<T, 8><<<grid, 256, 0, h->stream>>>(qa, qb, k, kpad, S, decide, rule);
-  else if (b == 7)
-    oz_slice<T, 7><<<grid, 256, 0, h->stream>>>(qa, qb, k, kpad, S, decide, rule);
-  else
-    oz_slice<T, 6><<<grid, 256, 0, h->stream>>>(qa, qb, k, kpad, S, decide, rule);
-  return nrs_after_launch(h, "oz_slice");
+  auto kern = b == 8 ? oz_slice<T, 8> : b == 7 ? oz_slice<T, 7> : oz_slice<T, 6>;
+  return nrs_cuda_check(h, nrs_launch_after(true, kern, grid, 256, 0, h->stream, qa, qb, k, kpad, S, decide, rule),
+                        "oz_slice");
 }
 
 // rows_a / rows_b: rows of the (stacked) slice buffers; P.kpad: their pitch.
@@ -1678,8 +1694,15 @@ int launch_tc_b(nrs_handle* h, const void* sa, const void* sb, int S, const OzPa
   const int n_tiles = G ? P.n_tiles : P.tiles_m * P.tiles_n;
   const int ctas = n_tiles < h->num_sms ? n_tiles : h->num_sms;
   if (ctas < 1) return NRS_OK;
-  ozaki_tc_kernel<EST, G, B8><<<ctas, OZ_THREADS, OzGeom<G>::SMEM, stream>>>(mapA, mapB, P);
-  return nrs_after_launch(h, EST ? "ozaki_tc_kernel<est>" : "ozaki_tc_kernel");
+  // In one wave the early start saves ~3 us. CTAs that start early land on
+  // whichever SM has room first, which scatters neighbouring tiles over the
+  // dies: in several waves that costs more (8192^3, 28 slices products: 27.2
+  // -> 27.9 ms; f32 4096^3: 1.24 -> 1.27 ms). Tile lists follow a kernel that
+  // does not let them in early.
+  const bool after = !P.tiles && n_tiles <= h->num_sms;
+  return nrs_cuda_check(h, nrs_launch_after(after, ozaki_tc_kernel<EST, G, B8>, (unsigned)ctas, OZ_THREADS,
+                                            OzGeom<G>::SMEM, stream, mapA, mapB, P),
+                        EST ? "ozaki_tc_kernel<est>" : "ozaki_tc_kernel");
 }
 template <bool EST, bool G>
 int launch_tc(nrs_handle* h, const void* sa, const void* sb, int S, const OzParams& P, int64_t rows_a,
