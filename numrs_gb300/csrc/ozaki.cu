@@ -29,22 +29,25 @@
 //    2^(e_a[i] + e_b[j] + 2 - 2b - b(S-1)).
 //
 // The tensor-core kernel is persistent (one CTA per SM) and warp-specialised:
-//   warp 0      : TMA producer, 4-stage ring of A (128x64) + B (256x64) bf16
-//                 tiles, 128-byte swizzle;
-//   warp 1      : TMEM allocator and single-thread tcgen05.mma issuer,
-//                 M=128 N=256 K=16, FP32 accumulator in TMEM columns 0..255;
+//   warp 0      : TMA producer, ring of A and B bf16 tiles 64 wide in K,
+//                 128-byte swizzle;
+//   warp 1      : TMEM allocator and single-thread tcgen05.mma issuer;
 //   warps 2..9  : epilogue (one TMEM lane = one tile row per thread, two warps
-//                 per lane quarter splitting the 256 columns): copy the
-//                 finished accumulator to registers, hand it back to the MMA
-//                 warp at once, fold the copy into the carried int32 sums R
-//                 kept in TMEM columns 256..511, write each retired digit as
-//                 a byte of the element's record in a per-CTA slot, and
-//                 round every element's exact total once after d = 0.
-// Grouped launches (many small problems, one tile list) use 128 x 128 tiles,
-// a 6-stage ring and two accumulators in turn, and keep the digits in TMEM
-// and registers (the grouped epilogue below describes it).
-// Measured at 8192^3 (clock counters per warp): the MMA warp waits for TMA
-// data ~29% of its time and for the epilogue ~8%.
+//                 per lane quarter splitting the columns): fold the finished
+//                 accumulator into the carried int32 sums R, hand it back to
+//                 the MMA warp, retire the digits, and round every element's
+//                 exact total once after d = 0.
+// One large problem runs on CTA pairs (cta_group::2, M=256 N=256 K=16): each
+// CTA loads 128 rows of A and of B^T, 32 KB per 64-wide K block for the MMA
+// time of 128 x 256 of C, and holds its two 128 x 256 accumulators in all of
+// TMEM. One CTA with a 128 x 256 tile takes 48 KB for the same, and its one
+// accumulator (R filled the other half of TMEM) kept the tensor pipe 63%
+// active: its MMA warp waited for TMA data 29% of its time, for the epilogue
+// 8%. 8192^3 with 28 slice products (30.8 TFLOP): 20.4 -> 18.2 ms, 1.69
+// PFLOP/s, at the power limit.
+// Small problems and grouped launches (many small problems, one tile list)
+// use 128 x 128 tiles, a 6-stage ring and two accumulators in turn, and keep
+// the digits in TMEM and registers (the grouped epilogue below describes it).
 // Every mbarrier wait is bounded; on give-up the kernel records an error
 // word, drains its own copies and MMAs (bounded), frees TMEM and returns.
 #include <mutex>
@@ -79,28 +82,31 @@ constexpr int kChunkOf(int b) { return 1 << (26 - 2 * b); }
 constexpr int kTopOf(int b) { return 127 - b; }  // position of the top digit in X
 constexpr int OZ_MAX_SLICES = 16;
 
-// Tile geometry per launch kind. One large problem: 128 x 256 tiles, one
-// accumulator, 4 stages (the constants above). Grouped launches, mostly
-// small problems: 128 x 128 tiles (less padding for narrow problems), two
-// accumulators in TMEM columns 0..255 so the MMAs of the next group run
-// while the epilogue reads the last one, the diagonal sums in 256..383,
-// and 6 stages of 32 KB.
-template <bool G>
+// Tile geometry per kernel. The estimate: 128 x 256 tiles, 4 stages (the
+// constants above). Grouped launches, mostly small problems: 128 x 128 tiles
+// (less padding for narrow problems), two accumulators in TMEM columns 0..255
+// so the MMAs of the next group run while the epilogue reads the last one,
+// the diagonal sums in 256..383, and 6 stages of 32 KB. One large problem:
+// CTA pairs on 256 x 256 tiles; each CTA loads 128 rows of A and 128 of B^T
+// (32 KB a stage) and holds 128 x 256 of C in two accumulators.
+template <bool EST, bool G>
 struct OzGeom {
-  static constexpr int BN = G ? 128 : OZ_BN;
-  static constexpr int STAGES = G ? 6 : OZ_STAGES;
-  static constexpr int B_BYTES = BN * OZ_BK * 2;
-  static constexpr int STAGE_BYTES = OZ_A_BYTES + B_BYTES;
-  static constexpr int ACC_BUFS = G ? 2 : 1;
-  // Grouped epilogue: the column exponents of each epilogue warp's 64 tile
-  // columns, staged once per tile.
+  static constexpr bool PAIR = !EST && !G;
+  static constexpr int BM = PAIR ? 2 * OZ_BM : OZ_BM;  // tile rows
+  static constexpr int BN = G ? 128 : OZ_BN;           // tile columns, accumulator columns
+  static constexpr int LOAD_N = EST ? OZ_BN : 128;     // B^T rows that a CTA loads
+  static constexpr int STAGES = EST ? OZ_STAGES : PAIR ? 7 : 6;
+  static constexpr int STAGE_BYTES = OZ_A_BYTES + LOAD_N * OZ_BK * 2;
+  // The column exponents of each grouped epilogue warp's 64 tile columns,
+  // staged once per tile.
   static constexpr int EB_BYTES = G ? 8 * 64 * 4 : 0;
   static constexpr int SMEM = STAGES * STAGE_BYTES + EB_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static_assert(SMEM <= 232448, "shared memory of one CTA");
   // Instruction descriptor, kind::f16: D f32 (bits 4-5 = 1), A and B bf16
   // (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits
   // 17-22, M >> 4 at bits 24-28.
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                    ((uint32_t)(OZ_BM >> 4) << 24);
+                                    ((uint32_t)(BM >> 4) << 24);
 };
 // Grouped launches with S > 9 keep digits 8..14 in a per-CTA 128 x 128 slot
 // of 8-byte records (column-major: for one column a warp's 32 rows are 256
@@ -111,36 +117,65 @@ constexpr int OZ_DIGIT_BYTES = 8;
 // ---------------------------------------------------------------------------
 // tcgen05 / TMEM wrappers
 // ---------------------------------------------------------------------------
+// (PAIR: the cta_group::2 forms, which a kernel uses throughout or not at all)
+template <bool PAIR>
 NRS_DEV void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                   smem_u32(dst_smem)),
-               "r"(ncols)
-               : "memory");
+  if constexpr (PAIR) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
+                 "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
+                 "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
 }
-NRS_DEV void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
+template <bool PAIR>
 NRS_DEV void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-               : "memory");
+  if constexpr (PAIR)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  else
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 NRS_DEV void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 NRS_DEV void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+template <bool PAIR>
 NRS_DEV void tc_mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if constexpr (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
-NRS_DEV void tc_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
-      : "memory");
+// Arrives on `bar` (PAIR: in both CTAs, or in this one only) once the MMAs
+// issued so far are done.
+template <bool PAIR>
+NRS_DEV void tc_commit(uint64_t* bar, bool own = false) {
+  if (PAIR && own)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+  else if constexpr (PAIR)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
 }
 
 // One lane of a converged warp (the same one every time).
@@ -186,6 +221,13 @@ NRS_DEV void tmem_ld8_nowait(uint32_t taddr, uint32_t* v) {
                  "=r"(v[7])
                : "r"(taddr)
                : "memory");
+}
+// Waits for every load; `v` (16 registers of one of them) is usable after it.
+NRS_DEV void tmem_wait_ld16(uint32_t* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
+                 "+r"(v[15])::"memory");
 }
 NRS_DEV void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -250,7 +292,7 @@ constexpr float kSumScale = 65536.0f;
 struct OzParams {
   int64_t m, n, k, kpad;
   int slices;
-  int kchunks;
+  int kchunks;     // estimate only, as n_pairs
   int n_pairs;     // pairs x kchunks work units per tile
   int tiles_m, tiles_n;
   int group_m;     // tile rasterisation group height
@@ -274,15 +316,14 @@ struct OzParams {
   // Slice count decided on the device (null: the count is `slices`). A count
   // of 0 makes the launch return at once.
   const uint32_t* count;
-  // One problem on 128 x 128 tiles (grouped geometry, no tile list): K in
-  // `splits` ranges of split_blocks 64-wide blocks. With several, range z
+  // One problem (no tile list): K in `splits` ranges of split_blocks 64-wide blocks. With several, range z
   // writes its product to the f64 slab C + z m n (row pitch n).
   int splits, split_blocks;
   int f32;
+  int n_tiles;  // tiles x splits
   // Grouped launch only: the tile list and the problems it points into.
   const struct OzTile* tiles;
   const struct OzProb* probs;
-  int n_tiles;
 };
 
 // One problem of a grouped launch: its slices are rows [rowoff, rowoff + m)
@@ -375,11 +416,36 @@ __device__ __forceinline__ int group_size(const PairIter& pi, int gm, int kchunk
 }
 
 
+// The first up to 8 of `nd` digit planes (a byte per column, 8 columns at
+// `p`) as one word per column, digit t in byte t.
+__device__ __forceinline__ void digits8(const uint8_t* p, size_t plane, int nd, uint64_t (&out)[8]) {
+  uint2 d[8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+    d[t] = t < nd ? __ldcg(reinterpret_cast<const uint2*>(p + t * plane)) : make_uint2(0, 0);
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    uint32_t h[2][4];  // [digits 0..3 / 4..7][column]
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const uint32_t a = g ? d[4 * t].y : d[4 * t].x, b = g ? d[4 * t + 1].y : d[4 * t + 1].x;
+      const uint32_t c = g ? d[4 * t + 2].y : d[4 * t + 2].x, e = g ? d[4 * t + 3].y : d[4 * t + 3].x;
+      const uint32_t ab0 = __byte_perm(a, b, 0x5140), ab1 = __byte_perm(a, b, 0x7362);  // a0 b0 a1 b1, a2 b2 a3 b3
+      const uint32_t ce0 = __byte_perm(c, e, 0x5140), ce1 = __byte_perm(c, e, 0x7362);
+      h[t][0] = __byte_perm(ab0, ce0, 0x5410);
+      h[t][1] = __byte_perm(ab0, ce0, 0x7632);
+      h[t][2] = __byte_perm(ab1, ce1, 0x5410);
+      h[t][3] = __byte_perm(ab1, ce1, 0x7632);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[g * 4 + q] = (uint64_t)h[1][q] << 32 | h[0][q];
+  }
+}
+
 // Writes 8 consecutive columns of one tile row of C (f64, or f32 when F32):
 // R values w, digits 0..7 of each column in `lo` (digit t = byte t; with B8,
 // i.e. 8-bit digits, and S <= 9 left-aligned instead, digit S-2 on top),
-// digits 8..14 from the 8-byte records `pitch` apart (S > 9 only) and the
-// column exponents; `left` of the 8 columns lie inside the problem; the row
+// digits 8..14 in `hi` (S > 9) and the column exponents; `left` of the 8 columns lie inside the problem; the row
 // starts at element `off` of C. The conversions run straight-line for all 8
 // (the digit width is a template argument and the slice count is tested
 // once, so no branch separates the elements' chains: with both tested per
@@ -387,19 +453,16 @@ __device__ __forceinline__ int group_size(const PairIter& pi, int gm, int kchunk
 // small tile's time); zero, tiny, subnormal and overflowing results are redone by
 // the exact path.
 template <bool F32, bool B8>
-__device__ __forceinline__ void retire8(const uint32_t (&w)[8], const uint64_t (&lo)[8], const uint8_t* rec,
-                                        size_t pitch, const int* eb, int left, int b, int S, int ebase, void* C,
+__device__ __forceinline__ void retire8(const uint32_t (&w)[8], const uint64_t (&lo)[8], const uint64_t (&hi)[8],
+                                        const int* eb, int left, int b, int S, int ebase, void* C,
                                         int64_t off, bool accumulate) {
   using Fmt = typename std::conditional<F32, NrsF32Fmt, NrsF64Fmt>::type;
   const int nd = S - 1;
-  uint64_t hi[8], bits[8];
+  uint64_t bits[8];
   int ex[8];
   unsigned special = 0;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    hi[e] = 0;
-    ex[e] = e < left ? eb[e] : 0;
-  }
+  for (int e = 0; e < 8; ++e) ex[e] = e < left ? eb[e] : 0;
   const bool top = B8 && nd <= 8;
   if (top) {
 #pragma unroll
@@ -409,11 +472,6 @@ __device__ __forceinline__ void retire8(const uint32_t (&w)[8], const uint64_t (
       special |= (unsigned)sp << e;
     }
   } else {
-    if (S > 9) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        if (e < left) hi[e] = __ldcg(reinterpret_cast<const unsigned long long*>(rec + (size_t)e * pitch));
-    }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       bool neg, sp;
@@ -472,19 +530,23 @@ __device__ __forceinline__ void retire8(const uint32_t (&w)[8], const uint64_t (
 }
 
 // `S`: the launch's slice count (tile lists carry their own pair counts).
-template <bool G>
-__device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int S, int tile) {
+// `rank`: the CTA's in its pair, whose tile is 256 rows and loads 128 + 128
+// rows of B^T.
+template <bool EST, bool G>
+__device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int S, int tile, uint32_t rank) {
+  using Geo = OzGeom<EST, G>;
   TileCtx c;
   c.kbase = 0;
-  if (G && !P.tiles) {
+  if (!EST && !(G && P.tiles)) {
     const int per = P.tiles_m * P.tiles_n;
     const int z = tile / per;
     int tm, tn;
     tile_coords(tile - z * per, P, tm, tn);
     c.m = P.m;
     c.n = P.n;
-    c.row0 = c.arow = (int64_t)tm * OZ_BM;
-    c.col0 = c.brow = (int64_t)tn * OzGeom<true>::BN;
+    c.row0 = c.arow = (int64_t)tm * Geo::BM + rank * OZ_BM;
+    c.col0 = (int64_t)tn * Geo::BN;
+    c.brow = c.col0 + rank * OZ_BM;
     c.kbase = z * P.split_blocks;
     const int kb = (int)((P.kpad + OZ_BK - 1) / OZ_BK) - c.kbase;
     c.kblocks = kb < P.split_blocks ? kb : P.split_blocks;
@@ -509,7 +571,7 @@ __device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int S, int tile) 
     c.m = q.m;
     c.n = q.n;
     c.row0 = (int64_t)t.tm * OZ_BM;
-    c.col0 = (int64_t)t.tn * OzGeom<true>::BN;
+    c.col0 = (int64_t)t.tn * Geo::BN;
     c.arow = q.rowoff + c.row0;
     c.brow = q.coloff + c.col0;
     c.kblocks = (int)((q.kpad + OZ_BK - 1) / OZ_BK);
@@ -529,14 +591,8 @@ __device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int S, int tile) 
     c.row0 = c.arow = (int64_t)tm * OZ_BM;
     c.col0 = c.brow = (int64_t)tn * OZ_BN;
     c.kblocks = (int)((P.kpad + OZ_BK - 1) / OZ_BK);
-    c.n_pairs = P.count ? S * (S + 1) / 2 * P.kchunks : P.n_pairs;
+    c.n_pairs = P.n_pairs;
     c.kchunks = P.kchunks;
-    c.ea = P.ea;
-    c.eb = P.eb;
-    c.C = P.C;
-    c.ldc = P.ldc;
-    c.accumulate = P.accumulate;
-    c.f32 = P.f32;
   }
   return c;
 }
@@ -553,7 +609,8 @@ template <bool EST, bool G, bool B8>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     ozaki_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                     OzParams P) {
-  using Geo = OzGeom<G>;
+  using Geo = OzGeom<EST, G>;
+  constexpr bool PAIR = Geo::PAIR;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + Geo::STAGES * Geo::STAGE_BYTES + Geo::EB_BYTES);
@@ -566,7 +623,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 
   // (warp-uniform, and known to be)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int n_tiles = G ? P.n_tiles : P.tiles_m * P.tiles_n;
+  const int n_tiles = P.n_tiles;
+  // A pair works on one tile: its rank 0 issues the MMAs of both.
+  const uint32_t rank = PAIR ? cluster_rank() : 0;
+  const int tile0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  const int tile_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   launch_next();
 
   if (threadIdx.x == 0) {
@@ -576,7 +637,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accf[b], 1);
-      mbar_init(&acce[b], 8);
+      mbar_init(&acce[b], PAIR ? 16 : 8);
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
@@ -585,11 +646,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     prefetch_tensormap(&mapB);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, OZ_TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc<PAIR>(tmem_slot, OZ_TMEM_COLS);
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // both CTAs' barriers are set up
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -597,14 +658,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   launch_wait();
   const int S = P.count ? (int)__ldcg(P.count) : P.slices;
   if (S == 0) {  // (the same word for every thread)
-    if (warp == 1) tmem_dealloc(tmem_base, OZ_TMEM_COLS);
+    if (warp == 1) tmem_dealloc<PAIR>(tmem_base, OZ_TMEM_COLS);
     return;
   }
   const int final_shift = 2 - 2 * P.digit_bits - P.digit_bits * (S - 1);
 
-  auto bounded = [&](uint64_t* bar, uint32_t phase, uint32_t site) -> bool {
+  auto bounded = [&](uint64_t* bar, uint32_t phase, uint32_t site, auto cluster) -> bool {
     for (uint32_t i = 0; i < NRS_WAIT_LIMIT; ++i) {
-      if (mbar_try_wait(bar, phase)) return true;
+      if (cluster ? mbar_try_wait_cluster(bar, phase) : mbar_try_wait(bar, phase)) return true;
       if (*abort_flag) return false;
     }
     *abort_flag = 1;
@@ -618,8 +679,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       uint32_t s = 0, ph = 1, it = 0;  // ring slot, its empty phase, loads issued
       bool ok = true;
       const int chunk_blocks = P.kchunk / OZ_BK;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const TileCtx c = tile_ctx<G>(P, S, tile);
+      for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+        const TileCtx c = tile_ctx<EST, G>(P, S, tile, rank);
         const int32_t arow = (int32_t)c.arow, brow = (int32_t)c.brow;
         PairIter pr;
         pr.start(S);
@@ -629,11 +690,19 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           const int32_t sa = pr.s, sb = pr.t();
           int32_t x = (c.kbase + kb0) * OZ_BK;
           for (int kb = kb0; kb < kb1; ++kb, ++it, x += OZ_BK) {
-            if (!bounded(&empty[s], ph, 1)) { ok = false; break; }
+            if (!bounded(&empty[s], ph, 1, std::false_type{})) { ok = false; break; }
             uint8_t* st = smem + s * Geo::STAGE_BYTES;
-            mbar_arrive_expect_tx(&full[s], Geo::STAGE_BYTES);
-            tma_load_3d(st, &mapA, &full[s], x, arow, sa);
-            tma_load_3d(st + OZ_A_BYTES, &mapB, &full[s], x, brow, sb);
+            if constexpr (PAIR) {
+              // both CTAs' bytes are counted by rank 0's barrier
+              if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * Geo::STAGE_BYTES);
+              const uint32_t bar = cluster_addr(&full[s], 0);
+              tma_load_3d_pair(st, &mapA, bar, x, arow, sa);
+              tma_load_3d_pair(st + OZ_A_BYTES, &mapB, bar, x, brow, sb);
+            } else {
+              mbar_arrive_expect_tx(&full[s], Geo::STAGE_BYTES);
+              tma_load_3d(st, &mapA, &full[s], x, arow, sa);
+              tma_load_3d(st + OZ_A_BYTES, &mapB, &full[s], x, brow, sb);
+            }
             if (++s == Geo::STAGES) {
               s = 0;
               ph ^= 1;
@@ -641,7 +710,22 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           }
         }
       }
-      if (!ok) {
+      if (PAIR && ok) {
+        // rank 0's MMAs release this CTA's stages too: let the last of those
+        // arrivals land before the CTA can exit
+        for (int j = 0; j < Geo::STAGES && ok; ++j) {
+          ok = bounded(&empty[s], ph, 1, std::false_type{});
+          if (++s == Geo::STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (PAIR && !ok && rank != 0) {
+        // Rank 0's barriers, which this CTA cannot wait on, count its copies
+        // in flight: they take microseconds, this a millisecond.
+        for (int j = 0; j < 100; ++j) __nanosleep(10000);
+      } else if (!ok) {
         // Drain: wait (bounded) for the copies still in flight.
         for (uint32_t j = (it >= Geo::STAGES ? it - Geo::STAGES : 0); j < it; ++j)
           mbar_wait_bounded(&full[j % Geo::STAGES], (j / Geo::STAGES) & 1, 1u << 16);
@@ -649,27 +733,27 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (elect_one()) {
+    if (rank == 0 && elect_one()) {
       uint32_t s = 0, ph = 0, ai = 0;  // ring slot, its full phase, accumulation groups
       bool ok = true;
-      const bool two = EST ? P.slices == 1 : Geo::ACC_BUFS == 2;
+      const bool two = !EST || P.slices == 1;
       const int chunk_blocks = P.kchunk / OZ_BK;
       const uint64_t adesc0 = smem_desc_sw128(smem_u32(smem));
       const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem) + OZ_A_BYTES);
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        const TileCtx c = tile_ctx<G>(P, S, tile);
+      for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+        const TileCtx c = tile_ctx<EST, G>(P, S, tile, rank);
         const int gm = merge_count(c, P, EST);
         PairIter pr;
         pr.start(S);
         for (int u = 0; u < c.n_pairs && ok; ++ai) {
           const int g = group_size(pr, gm, c.kchunks);
-          // One accumulator (TMEM columns 0..255) or two (0..127, 128..255 in
-          // grouped launches, 0..255, 256..511 in the estimate's first
-          // pass), used in turn; the epilogue frees one as soon as it has
-          // read it.
+          // Two accumulators (TMEM columns 0..127, 128..255 in grouped
+          // launches, else 0..255, 256..511; the estimate's second pass has
+          // only the first), used in turn; the epilogue frees one as soon as
+          // it has read it.
           const int buf = two ? (int)(ai & 1) : 0;
           const uint32_t aph = (two ? ai >> 1 : ai) & 1;
-          if (!bounded(&acce[buf], aph ^ 1, 2)) { ok = false; break; }
+          if (!bounded(&acce[buf], aph ^ 1, 2, std::bool_constant<PAIR>{})) { ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(buf * Geo::BN);
           uint32_t accum = 0;
@@ -677,16 +761,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int kb0 = pr.chunk * chunk_blocks;
             const int kb1 = kb0 + chunk_blocks < c.kblocks ? kb0 + chunk_blocks : c.kblocks;
             for (int kb = kb0; kb < kb1; ++kb) {
-              if (!bounded(&full[s], ph, 3)) { ok = false; break; }
+              if (!bounded(&full[s], ph, 3, std::false_type{})) { ok = false; break; }
               tc_fence_after();
               // (a stage or K step moves the descriptors' 16-byte address field)
               const uint64_t off = (uint64_t)(s * (Geo::STAGE_BYTES / 16));
 #pragma unroll
               for (int kk = 0; kk < OZ_BK / 16; ++kk) {
-                tc_mma_bf16(d_tmem, adesc0 + off + kk * 2, bdesc0 + off + kk * 2, Geo::IDESC, accum);
+                tc_mma_bf16<PAIR>(d_tmem, adesc0 + off + kk * 2, bdesc0 + off + kk * 2, Geo::IDESC, accum);
                 accum = 1;
               }
-              tc_commit(&empty[s]);  // frees the stage once these MMAs have read it
+              tc_commit<PAIR>(&empty[s]);  // frees the stage once these MMAs have read it
               if (++s == Geo::STAGES) {
                 s = 0;
                 ph ^= 1;
@@ -694,12 +778,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             }
           }
           if (!ok) break;
-          tc_commit(&accf[buf]);  // accumulator ready once every MMA above completes
+          tc_commit<PAIR>(&accf[buf]);  // accumulator ready once every MMA above completes
           u += g;
         }
       }
       // Make sure no MMA is still running before TMEM is released.
-      tc_commit(drain);
+      tc_commit<PAIR>(drain, true);
       mbar_wait_bounded(drain, 0, 1u << 20);
     }
   } else if (EST) {
@@ -720,8 +804,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint32_t ai = 0;
     float rmax = 0.0f;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileCtx tc = tile_ctx<G>(P, S, tile);
+    for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+      const TileCtx tc = tile_ctx<EST, G>(P, S, tile, rank);
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int64_t col0 = tc.col0 + half * (OZ_BN / 2);
@@ -739,7 +823,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       pr.start(S);
       for (int u = 0; u < tc.n_pairs; ++u, ++ai, pr.next(1)) {
         const int buf = pass1 ? (int)(ai & 1) : 0;
-        if (!bounded(&accf[buf], (pass1 ? ai >> 1 : ai) & 1, 4)) { ok = false; break; }
+        if (!bounded(&accf[buf], (pass1 ? ai >> 1 : ai) & 1, 4, std::false_type{})) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < OZ_BN / 32; ++c) {
@@ -817,8 +901,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     int* const sm_eb = reinterpret_cast<int*>(smem + Geo::STAGES * Geo::STAGE_BYTES) + (warp - 2) * 64;
     uint32_t ai = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileCtx tc = tile_ctx<G>(P, S, tile);
+    for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+      const TileCtx tc = tile_ctx<EST, G>(P, S, tile, rank);
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int ncols = (int)(tc.n - tc.col0 < BN ? tc.n - tc.col0 : BN);
@@ -850,7 +934,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         for (int j = 0; j < g; ++j) pr.next(tc.kchunks);
         const bool final_group = u == tc.n_pairs;  // the last group of d = 0
         const int buf = (int)(ai & 1);
-        if (!bounded(&accf[buf], (ai >> 1) & 1, 4)) { ok = false; break; }
+        if (!bounded(&accf[buf], (ai >> 1) & 1, 4, std::false_type{})) { ok = false; break; }
         tc_fence_after();
         // Chunk by chunk: the accumulator and R in flight together, R
         // updated and stored back; the accumulator goes back to the MMA warp
@@ -942,11 +1026,20 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           }
           const int64_t off = row * tc.ldc + tc.col0 + col_t;
           const uint8_t* rec = slot + (size_t)col_t * kColPitch;
+          uint64_t hi[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) hi[e] = 0;
+          if (S > 9) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (col_t + e < ncols)
+                hi[e] = __ldcg(reinterpret_cast<const unsigned long long*>(rec + (size_t)e * kColPitch));
+          }
           if (tc.f32)
-            retire8<true, B8>(w, lo, rec, kColPitch, sm_eb + i * 16 + h8, ncols - col_t, b, S, ecol_base, tc.C, off,
+            retire8<true, B8>(w, lo, hi, sm_eb + i * 16 + h8, ncols - col_t, b, S, ecol_base, tc.C, off,
                               tc.accumulate);
           else
-            retire8<false, B8>(w, lo, rec, kColPitch, sm_eb + i * 16 + h8, ncols - col_t, b, S, ecol_base, tc.C, off,
+            retire8<false, B8>(w, lo, hi, sm_eb + i * 16 + h8, ncols - col_t, b, S, ecol_base, tc.C, off,
                                tc.accumulate);
           }
           __syncwarp();  // (the loads above are warp-wide)
@@ -957,33 +1050,39 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       if (lane == 0) mbar_arrive(&acce[last_buf]);
     }
   } else {
-    // ---------------- epilogue (warps 2..9) ----------------
+    // ---------------- epilogue of a pair (warps 2..9) ----------------
     // Warp w reads TMEM lane quarter w % 4 (one tile row per thread) and
     // column half (w - 2) / 4 (128 columns). As in the grouped epilogue, one
-    // int32 per element, R (TMEM columns 256..511), carries the exact
-    // diagonal sums from d = S-1 to d = 0 (R <- floor(R / 2^b) + D_d) and
-    // the low b bits retire as digit S-2-d, here as a byte of the element's
-    // 16-byte record in this CTA's slot (column-major 128 x 256; written once
-    // per diagonal, read once).
-    // No global read-modify-write per diagonal; after d = 0 each element's
-    // exact total R 2^(b(S-1)) + sum_t digit_t 2^(bt) is rounded once to
-    // f64. Per group: copy the accumulator to registers, hand it back to the
-    // MMA warp at once, fold the copy into R.
+    // int32 per element, R, carries the exact diagonal sums from d = S-1 to
+    // d = 0 (R <- floor(R / 2^b) + D_d); the two accumulators take all of
+    // TMEM, so R stays in this thread's registers. The low b bits retire as
+    // digit S-2-d: a thread packs its 128 into eight 16-byte stores to the
+    // digit's plane of this CTA's slot ([digit][column / 16][row][16]: a
+    // warp's store is 512 contiguous bytes), each read once by the retire
+    // pass, which transposes the bytes of 8 columns back. (Byte stores into
+    // 16-byte records per element: 4096 x 64 x 4096 516 us, 249 us.)
+    // After d = 0 each element's exact total R 2^(b(S-1)) + sum_t digit_t
+    // 2^(bt) is rounded once to f64.
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     const int row_in_tile = q * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + half * (OZ_BN / 2);
-    const uint32_t acc_t = lane_base;           // accumulator columns
-    const uint32_t dsum_t = lane_base + OZ_BN;  // R
     const int b = B8 ? 8 : P.digit_bits, nd = S - 1;
-    const uint32_t dmask = (1u << b) - 1;
-    constexpr size_t pitch = (size_t)OZ_BM * 16;  // record bytes between tile columns
-    uint8_t* const slot = reinterpret_cast<uint8_t*>(P.acc) + (size_t)blockIdx.x * (OZ_BM * OZ_BN * 16) +
-                          (size_t)(half * (OZ_BN / 2)) * pitch + (size_t)row_in_tile * 16;
+    constexpr size_t kChunk = (size_t)OZ_BM * 16;        // bytes of 16 columns of a digit
+    constexpr size_t kPlane = (size_t)OZ_BM * OZ_BN;      // bytes of a digit
+    uint8_t* const slot = reinterpret_cast<uint8_t*>(P.acc) + (size_t)blockIdx.x * (kPlane * 16) +
+                          (size_t)(half * (OZ_BN / 32)) * kChunk + (size_t)row_in_tile * 16;
+    const uint32_t acce0 = cluster_addr(&acce[0], 0);  // rank 0's barriers
+    auto release = [&](int buf) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(acce0 + buf * (uint32_t)sizeof(uint64_t));
+    };
+    uint32_t R[OZ_BN / 2];
     uint32_t ai = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-      const TileCtx tc = tile_ctx<G>(P, S, tile);
+    for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+      const TileCtx tc = tile_ctx<EST, G>(P, S, tile, rank);
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int64_t col0 = tc.col0 + half * (OZ_BN / 2);
@@ -992,92 +1091,97 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const int gm = merge_count(tc, P, false);
       PairIter pr;
       pr.start(S);
+      int last_buf = 0;
+#pragma unroll
+      for (int e = 0; e < OZ_BN / 2; ++e) R[e] = 0;
       for (int u = 0; u < tc.n_pairs && ok; ++ai) {
         const int g = group_size(pr, gm, tc.kchunks);
         const int d = pr.d;
-        const bool diag_start = pr.diag_first();
-        const bool tile_first = u == 0;
+        const bool push = pr.diag_first() && u != 0;
         u += g;
         for (int j = 0; j < g; ++j) pr.next(tc.kchunks);
-        const uint32_t aph = ai & 1;
-        if (!bounded(&accf[0], aph, 4)) { ok = false; break; }
-        tc_fence_after();
-        // Copy this warp's 128 accumulator columns to registers (eight loads,
-        // one wait) and hand the accumulator back at once, so the next unit's
-        // MMAs run while the copy is folded into R.
-        uint32_t v[OZ_BN / 2];
+        const int buf = (int)(ai & 1);
+        last_buf = buf;
+        if (push) {  // digit of diagonal d + 1
+          uint8_t* const sp = slot + (size_t)(nd - 1 - d) * kPlane;
+          const uint32_t dmask = ((1u << b) - 1) * 0x01010101u;
 #pragma unroll
-        for (int c = 0; c < OZ_BN / 32; ++c) tmem_ld16_nowait(acc_t + c * 16, v + c * 16);
-        tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[0]);
-        const int dig_i = nd - 1 - d;  // digit index of diagonal d + 1
-        const bool push = diag_start && !tile_first;
-        const int rsh = push ? b : 0;
+          for (int c = 0; c < OZ_BN / 32; ++c) {
+            uint32_t u4[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t* r = R + c * 16 + j * 4;
+              u4[j] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410) & dmask;
+            }
+            *reinterpret_cast<uint4*>(sp + c * kChunk) = make_uint4(u4[0], u4[1], u4[2], u4[3]);
+          }
+#pragma unroll
+          for (int e = 0; e < OZ_BN / 2; ++e) R[e] = (uint32_t)((int32_t)R[e] >> b);
+        }
+        if (!bounded(&accf[buf], (ai >> 1) & 1, 4, std::false_type{})) { ok = false; break; }
+        tc_fence_after();
+        // 16 columns are folded into R while the next 16 load
+        uint32_t v[2][16];
+        tmem_ld16_nowait(lane_base + buf * OZ_BN, v[0]);
 #pragma unroll
         for (int c = 0; c < OZ_BN / 32; ++c) {
-          uint32_t w[16];
-          if (tile_first) {
+          tmem_wait_ld16(v[c & 1]);
+          if (c + 1 < OZ_BN / 32) tmem_ld16_nowait(lane_base + buf * OZ_BN + (c + 1) * 16, v[(c + 1) & 1]);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) w[e] = 0;
-          } else {
-            tmem_ld16(dsum_t + c * 16, w);
-          }
-          if (push) {
-            uint8_t* sp = slot + (size_t)(c * 16) * pitch + dig_i;
-            const int nv = row_ok ? ncols - c * 16 : 0;  // columns of this chunk inside the problem
-#pragma unroll
-            for (int e = 0; e < 16; ++e)
-              if (e < nv) sp[(size_t)e * pitch] = (uint8_t)(w[e] & dmask);
-          }
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            w[e] = (uint32_t)(((int32_t)w[e] >> rsh) + __float2int_rn(__uint_as_float(v[c * 16 + e])));
-          tmem_st16(dsum_t + c * 16, w);
+          for (int e = 0; e < 16; ++e) R[c * 16 + e] += (uint32_t)__float2int_rn(__uint_as_float(v[c & 1][e]));
         }
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
+        if (u < tc.n_pairs) release(buf);
       }
       if (!ok) break;
-      // After the last group of d = 0: R and the records of 8 columns at a
+      // The last group's accumulator is still held: R goes through it to the
+      // retire pass, which runs as a loop.
+#pragma unroll
+      for (int c = 0; c < OZ_BN / 32; ++c)
+        tmem_st16(lane_base + last_buf * OZ_BN + c * 16, *reinterpret_cast<const uint32_t(*)[16]>(R + c * 16));
+      tmem_wait_st();
+      const uint32_t dsum_t = lane_base + last_buf * OZ_BN;
+      // After the last group of d = 0: R and the digits of 8 columns at a
       // time (loads in flight together), rounded once, written to C.
 #pragma unroll 1
       for (int c8 = 0; c8 < OZ_BN / 2; c8 += 8) {
         if (c8 >= ncols) break;  // warp-uniform
         uint32_t w[8];
-        uint64_t lo[8];
+        uint64_t lo[8], hi[8];
         tmem_ld8_nowait(dsum_t + c8, w);
+        const uint8_t* dp = slot + (size_t)(c8 >> 4) * kChunk + (c8 & 8);
+        digits8(dp, kPlane, nd, lo);
+        if (S > 9) {
+          digits8(dp + 8 * kPlane, kPlane, nd - 8, hi);
+        } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          lo[e] = row_ok && c8 + e < ncols
-                      ? __ldcg(reinterpret_cast<const unsigned long long*>(slot + (size_t)(c8 + e) * pitch))
-                      : 0;
+          for (int e = 0; e < 8; ++e) hi[e] = 0;
+        }
         tmem_wait_ld();
         if (row_ok) {
         if (B8 && nd <= 8) {  // left-aligned; bytes the digits do not reach drop out
 #pragma unroll
           for (int e = 0; e < 8; ++e) lo[e] = nd ? lo[e] << (64 - 8 * nd) : 0;
         }
-        const uint8_t* rec = slot + (size_t)c8 * pitch + 8;
         const int64_t off = row * tc.ldc + col0 + c8;
         if (tc.f32)
-          retire8<true, B8>(w, lo, rec, pitch, tc.eb + col0 + c8, ncols - c8, b, S, ecol_base, tc.C, off,
+          retire8<true, B8>(w, lo, hi, tc.eb + col0 + c8, ncols - c8, b, S, ecol_base, tc.C, off,
                             tc.accumulate);
         else
-          retire8<false, B8>(w, lo, rec, pitch, tc.eb + col0 + c8, ncols - c8, b, S, ecol_base, tc.C, off,
+          retire8<false, B8>(w, lo, hi, tc.eb + col0 + c8, ncols - c8, b, S, ecol_base, tc.C, off,
                              tc.accumulate);
         }
         __syncwarp();  // (the loads above are warp-wide)
       }
+      release(last_buf);
     }
   }
   tc_fence_before();
   __syncthreads();
+  // (a pair's CTAs reach into each other until both are done)
+  if constexpr (PAIR) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, OZ_TMEM_COLS);
+    tmem_dealloc<PAIR>(tmem_base, OZ_TMEM_COLS);
   }
 }
 
@@ -1678,30 +1782,48 @@ int launch_oz_slice(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int6
                         "oz_slice");
 }
 
+// CTAs of a pair launch (and its digit slots).
+int pair_ctas(nrs_handle* h, int64_t tiles) { return 2 * (int)std::max<int64_t>(1, std::min<int64_t>(tiles, h->num_sms / 2)); }
+
 // rows_a / rows_b: rows of the (stacked) slice buffers; P.kpad: their pitch.
 template <bool EST, bool G, bool B8>
 int launch_tc_b(nrs_handle* h, const void* sa, const void* sb, int S, const OzParams& P, int64_t rows_a,
                 int64_t rows_b, cudaStream_t stream) {
+  using Geo = OzGeom<EST, G>;
   CUtensorMap mapA, mapB;
   if (!make_slice_map(&mapA, sa, P.kpad, rows_a, S, OZ_BM) ||
-      !make_slice_map(&mapB, sb, P.kpad, rows_b, S, OzGeom<G>::BN))
+      !make_slice_map(&mapB, sb, P.kpad, rows_b, S, Geo::LOAD_N))
     return nrs_fail(h, NRS_ERR_CUDA, "cuTensorMapEncodeTiled failed for the slices");
   // Set on every call: the attribute belongs to the current device's context.
   int st = nrs_cuda_check(h, cudaFuncSetAttribute(ozaki_tc_kernel<EST, G, B8>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, OzGeom<G>::SMEM),
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM),
                           "cudaFuncSetAttribute(ozaki)");
   if (st) return st;
-  const int n_tiles = G ? P.n_tiles : P.tiles_m * P.tiles_n;
+  const int n_tiles = P.n_tiles;
+  if (n_tiles < 1) return NRS_OK;
+  if constexpr (Geo::PAIR) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)pair_ctas(h, n_tiles));
+    cfg.blockDim = dim3(OZ_THREADS);
+    cfg.dynamicSmemBytes = Geo::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return nrs_cuda_check(h, cudaLaunchKernelEx(&cfg, ozaki_tc_kernel<EST, G, B8>, mapA, mapB, P), "ozaki_tc_kernel");
+  }
   const int ctas = n_tiles < h->num_sms ? n_tiles : h->num_sms;
-  if (ctas < 1) return NRS_OK;
   // In one wave the early start saves ~3 us. CTAs that start early land on
   // whichever SM has room first, which scatters neighbouring tiles over the
-  // dies: in several waves that costs more (8192^3, 28 slices products: 27.2
-  // -> 27.9 ms; f32 4096^3: 1.24 -> 1.27 ms). Tile lists follow a kernel that
+  // dies: in several waves that costs more (f32 4096^3 on these tiles: 1.24
+  // -> 1.27 ms). Tile lists follow a kernel that
   // does not let them in early.
   const bool after = !P.tiles && n_tiles <= h->num_sms;
   return nrs_cuda_check(h, nrs_launch_after(after, ozaki_tc_kernel<EST, G, B8>, (unsigned)ctas, OZ_THREADS,
-                                            OzGeom<G>::SMEM, stream, mapA, mapB, P),
+                                            Geo::SMEM, stream, mapA, mapB, P),
                         EST ? "ozaki_tc_kernel<est>" : "ozaki_tc_kernel");
 }
 template <bool EST, bool G>
@@ -1720,9 +1842,19 @@ OzParams base_params(nrs_handle* h, int64_t m, int64_t n, int64_t k, int64_t kpa
   P.tiles_m = (int)((m + OZ_BM - 1) / OZ_BM);
   P.tiles_n = (int)((n + OZ_BN - 1) / OZ_BN);
   P.group_m = 12;
+  P.n_tiles = P.tiles_m * P.tiles_n;
+  P.splits = 1;
+  P.split_blocks = (int)((kpad + OZ_BK - 1) / OZ_BK);
   P.err = h->dev_error;
   return P;
 }
+
+// Elements between the rows of a slice: TMA needs multiples of 8; from 256 on
+// of 64, so that the 128-byte rows of its boxes do not straddle sectors and
+// lines (f64 5000^3: 6.82 ms with rows of 10000 bytes, 4.95 of 10112;
+// 1999 x 1537 x 3001: 0.73 and 0.56). The
+// pad is zero, and within the 64-wide K block that is computed anyway.
+int64_t slice_pitch(int64_t k) { return k < 256 ? (k + 7) / 8 * 8 : (k + 63) / 64 * 64; }
 
 // Limits of b-bit digits with S slices over kpad: S <= 16, every digit
 // inside the 126 fraction bits (b S <= 126), int32-exact diagonal sums (at
@@ -1815,17 +1947,71 @@ int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, bool
   return NRS_OK;
 }
 
-// Digit slots of the 128 x 256 kernel: 16 bytes per element and CTA.
-size_t oz_slot_bytes(nrs_handle* h, int64_t m, int64_t n) {
-  const int64_t tiles = ((m + OZ_BM - 1) / OZ_BM) * ((n + OZ_BN - 1) / OZ_BN);
-  return (size_t)std::min<int64_t>(tiles, h->hw_sms) * OZ_BM * OZ_BN * 16;
+// One problem runs either on CTA pairs with 256 x 256 tiles (the least panel
+// traffic per flop) or on the grouped 128 x 128 geometry, either with K split
+// into ranges whose f64 products are added in order, which fills the GPU at
+// small sizes.
+struct TcPlan {
+  bool pair;
+  int splits, split_blocks;
+  double us;
+};
+
+// The form with the least modelled time (us). A 64-wide K block of one slice
+// pair takes 0.22 us on a 128 x 128 tile and 0.34 us on a pair's 256 x 256
+// one; a tile's fold and rounding 30 and 40 us; the ranges' slabs move at 3
+// TB/s. Measured whole calls, us (128 x 128 tiles in 1, 2, 4 ranges / pairs in
+// 1, 2, 4): f64 512^3 96, 79, 72 / 129, 103, 92; 1024^3 161, 134, 155 / 211,
+// 163, 146; 1536^3 252, 276, 315 / 333, 244, 288; 2048^3 504, 547, 557 / 405,
+// 458, 531; 4096^3 3006, 3088, - / 2544, 2524, -; 1024 x 8192 x 1024 981, 660,
+// 682 / 1258, 796, 581; f32 2048^3 252, 305 / 223, 274.
+TcPlan plan_tc(int64_t m, int64_t n, int64_t kpad, int S, int max_splits) {
+  const double pairs = 0.5 * S * (S + 1);
+  const int kb = (int)((kpad + OZ_BK - 1) / OZ_BK);
+  const int64_t t128 = (m + 127) / 128 * ((n + 127) / 128), t256 = (m + 255) / 256 * ((n + 255) / 256);
+  auto waves = [](int64_t tiles, int64_t at_once) { return (double)((tiles + at_once - 1) / at_once); };
+  TcPlan best{true, 0, 0, 0.0};
+  for (int z = 1; z <= max_splits && z <= kb; ++z) {
+    const int blocks = (kb + z - 1) / z;
+    const int splits = (kb + blocks - 1) / blocks;
+    if (splits != z || (z > 1 && (double)z * (double)(m * n) * 8.0 > 256.0 * (1 << 20))) continue;
+    const double join = z > 1 ? 3.0 + (double)z * (double)(m * n) * 8.0 / 3e6 : 0.0;
+    const double one = waves(t128 * z, NRS_PLAN_SMS) * (pairs * blocks * 0.22 + 30.0) + join;
+    const double two = waves(t256 * z, NRS_PLAN_SMS / 2) * (pairs * blocks * 0.34 + 40.0) + join;
+    if (!best.splits || two < best.us) best = TcPlan{true, splits, blocks, two};
+    if (one < best.us) best = TcPlan{false, splits, blocks, one};
+  }
+  return best;
+}
+
+// Digit slots of the slice products: a pair launch 16 bytes per element and
+// CTA, the grouped geometry 8 (used beyond 9 slices).
+size_t oz_slot_bytes(nrs_handle* h, const TcPlan& pl, int64_t m, int64_t n) {
+  if (pl.pair) return (size_t)pair_ctas(h, (m + 255) / 256 * ((n + 255) / 256) * pl.splits) * OZ_BM * OZ_BN * 16;
+  return (size_t)h->hw_sms * OZ_BM * OzGeom<false, true>::BN * OZ_DIGIT_BYTES;
+}
+
+// The slice products of one problem in the planned form (P from base_params).
+int launch_products(nrs_handle* h, const TcPlan& pl, int S, OzParams P, const OzScratch& w) {
+  using Pair = OzGeom<false, false>;
+  const int bm = pl.pair ? Pair::BM : OZ_BM, bn = pl.pair ? Pair::BN : OzGeom<false, true>::BN;
+  P.tiles_m = (int)((P.m + bm - 1) / bm);
+  P.tiles_n = (int)((P.n + bn - 1) / bn);
+  P.group_m = pl.pair ? 8 : 12;
+  P.splits = pl.splits;
+  P.split_blocks = pl.split_blocks;
+  P.n_tiles = P.tiles_m * P.tiles_n * pl.splits;
+  return pl.pair ? launch_tc<false, false>(h, w.area_a, w.area_b, S, P, P.m, P.n, h->stream)
+                 : launch_tc<false, true>(h, w.area_a, w.area_b, S, P, P.m, P.n, h->stream);
 }
 
 int ozaki_run(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, int64_t n, int64_t k,
-              int64_t kpad, int b, int S, int kchunks, double* C, int64_t ldc, bool accumulate) {
+              int64_t kpad, int b, int S, double* C, int64_t ldc, bool accumulate) {
   int st;
   OzScratch w;
-  const size_t slots = oz_slot_bytes(h, m, n);
+  TcPlan pl = plan_tc(m, n, kpad, S, 1);
+  if (!digits_fit(b, S, kpad, kMaxChunkSlicesGrouped)) pl.pair = true;
+  const size_t slots = oz_slot_bytes(h, pl, m, n);
   uint8_t* ws = (uint8_t*)nrs_workspace(h, oz_scratch(m, n, kpad, S, slots, nullptr, nullptr), &st);
   if (!ws) return st;
   oz_scratch(m, n, kpad, S, slots, ws, &w);
@@ -1833,8 +2019,6 @@ int ozaki_run(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m,
   if ((st = launch_oz_slice<double>(h, a, bT, k, kpad, b, S, nullptr, OzRule{}, w))) return st;
   OzParams P = base_params(h, m, n, k, kpad);
   P.slices = S;
-  P.kchunks = kchunks;
-  P.n_pairs = S * (S + 1) / 2 * (kchunks > 0 ? kchunks : 1);
   P.ea = w.ea;
   P.eb = w.eb;
   P.acc = reinterpret_cast<__int128*>(w.tail);
@@ -1843,7 +2027,7 @@ int ozaki_run(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m,
   P.digit_bits = b;
   P.kchunk = kChunkOf(b);
   P.accumulate = accumulate ? 1 : 0;
-  return launch_tc<false, false>(h, w.area_a, w.area_b, S, P, m, n, h->stream);
+  return launch_products(h, pl, S, P, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -1856,46 +2040,13 @@ int ozaki_run(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m,
 // products, and the plain FP64 / FP32 kernel, whose blocks return at once
 // unless the count is 0 (Inf / NaN operands, sums that could overflow, or a
 // spread beyond the slice limit).
-//
-// One problem runs either on 128 x 256 tiles (the least panel traffic per
-// flop) or on the grouped 128 x 128 geometry with K split into ranges whose
-// f64 products are added in order, which fills the GPU at small sizes.
-struct TcPlan {
-  bool big;
-  int splits, split_blocks;
-  double us;
-};
 constexpr int kAutoMaxSlices = 12;
-
-// The form with the least modelled time (us). A 64-wide K block of one slice
-// pair takes 0.21 us on a 128 x 128 tile and 0.37 us on a 128 x 256 one; a
-// tile's fold and rounding 25 and 90 us. Measured against it (f64, S = 7):
-// 4096^3 2956 us (128 x 128) and 3389 us (128 x 256), 2048^3 497 and 544,
-// 1999 x 3001 x 1537 705, 623 with two K ranges, 709 on 128 x 256 tiles;
-// 1024^3 166 whole, 137 in two; 512^3 111, 94, 84, 84 in 1, 2, 4, 8.
-TcPlan plan_tc(int64_t m, int64_t n, int64_t kpad, int S) {
-  const double pairs = 0.5 * S * (S + 1);
-  const int kb = (int)((kpad + OZ_BK - 1) / OZ_BK);
-  const int64_t tm = (m + OZ_BM - 1) / OZ_BM;
-  auto waves = [](int64_t tiles) { return (double)((tiles + NRS_PLAN_SMS - 1) / NRS_PLAN_SMS); };
-  TcPlan best{true, 1, kb, waves(tm * ((n + OZ_BN - 1) / OZ_BN)) * (pairs * kb * 0.37 + 90.0)};
-  const int64_t t128 = tm * ((n + 127) / 128);
-  for (int z = 1; z <= 16 && z <= kb; z *= 2) {
-    const int blocks = (kb + z - 1) / z;
-    const int splits = (kb + blocks - 1) / blocks;
-    if (splits != z || (z > 1 && (double)z * (double)(m * n) * 8.0 > 256.0 * (1 << 20))) continue;
-    double us = waves(t128 * z) * (pairs * blocks * 0.21 + 25.0);
-    if (z > 1) us += 3.0 + (double)z * (double)(m * n) * 8.0 / 4e6;
-    if (us < best.us) best = TcPlan{false, splits, blocks, us};
-  }
-  return best;
-}
 
 template <typename T>
 int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, int64_t k, int64_t n, void* C,
             int64_t ldc, bool accumulate) {
   constexpr bool F32 = sizeof(T) == 4;
-  const int64_t kpad = (k + 7) / 8 * 8;
+  const int64_t kpad = slice_pitch(k);
   // 8-bit digits up to K = 10240, then 7-bit (exact int32 diagonal sums for
   // every count up to the limit)
   const int b = digits_fit(8, kAutoMaxSlices, kpad, kMaxChunkSlicesGrouped) ? 8 : 7;
@@ -1903,13 +2054,11 @@ int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, i
   int klog = 0;
   while (((int64_t)1 << klog) < k) ++klog;
   const OzRule rule{F32 ? 26 : 53, b, kAutoMaxSlices, (F32 ? 127 : 1023) - klog - 1};
-  const TcPlan pl = plan_tc(m, n, kpad, F32 ? 4 : 7);
+  const TcPlan pl = plan_tc(m, n, kpad, F32 ? 4 : 7, 16);
   const int plain_splits = F32 ? 1 : nrs_dmma_splits(m, k, n);
   const int slabs = std::max(pl.splits > 1 ? pl.splits : 0, plain_splits > 1 ? plain_splits : 0);
-  // Behind the slices: the kernel's digit slots (the grouped geometry needs
-  // them beyond 9 slices only), then the partial slabs.
-  const size_t slots = oz_al(pl.big ? oz_slot_bytes(h, m, n)
-                                    : (size_t)h->hw_sms * OZ_BM * OzGeom<true>::BN * OZ_DIGIT_BYTES);
+  // Behind the slices: the digit slots, then the partial slabs.
+  const size_t slots = oz_al(oz_slot_bytes(h, pl, m, n));
   const size_t tail = slots + (size_t)slabs * (size_t)(m * n) * 8;
   cudaStream_t s = h->stream;
   const size_t bytes = oz_scratch(m, n, kpad, kAutoMaxSlices, tail, nullptr, nullptr);
@@ -1927,7 +2076,6 @@ int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, i
     if ((st = launch_oz_slice<T>(h, a, bT, k, kpad, b, 0, w.words, rule, w))) return st;
     OzParams P = base_params(h, m, n, k, kpad);
     P.count = w.words + OZ_W_COUNT;
-    P.kchunks = (int)((kpad + kChunkOf(b) - 1) / kChunkOf(b));
     P.ea = w.ea;
     P.eb = w.eb;
     P.acc = reinterpret_cast<__int128*>(w.tail);
@@ -1937,15 +2085,7 @@ int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, i
     P.kchunk = kChunkOf(b);
     P.accumulate = accumulate ? 1 : 0;
     P.f32 = F32 ? 1 : 0;
-    if (pl.big) {
-      st = launch_tc<false, false>(h, w.area_a, w.area_b, kAutoMaxSlices, P, m, n, s);
-    } else {
-      P.tiles_n = (int)((n + OzGeom<true>::BN - 1) / OzGeom<true>::BN);
-      P.splits = pl.splits;
-      P.split_blocks = pl.split_blocks;
-      P.n_tiles = P.tiles_m * P.tiles_n * pl.splits;
-      st = launch_tc<false, true>(h, w.area_a, w.area_b, kAutoMaxSlices, P, m, n, s);
-    }
+    st = launch_products(h, pl, kAutoMaxSlices, P, w);
     if (st) return st;
     const int64_t rsa = a.rows_contig ? a.ld : 1, csa = a.rows_contig ? 1 : a.ld;
     const int64_t rsb = bT.rows_contig ? 1 : bT.ld, csb = bT.rows_contig ? bT.ld : 1;
@@ -2128,11 +2268,11 @@ __global__ void __launch_bounds__(256)
 // f64 and f32 GEMMs for which the slice GEMM is the faster form; NRS_ERR_UNSUPPORTED:
 // not one of them (nothing was enqueued). The rule compares both forms'
 // modelled times: the FP64 tensor path's 1.05 TFLOP/s on 32-wide tiles
-// against plan_tc's. Both sides measured (us, DMMA / slices): 256^3 51 / 76,
-// 384^3 124 / 85, 512^3 279 / 84, 1024^3 1983 / 137, 2048^3 15661 / 497,
-// 4096^3 124903 / 2956, 3000 x 2000 x 10 379 / 163, 64 x 4096 x 64 91 / 114.
-// f32 against the FP32 kernels (us): 1024^3 76 / 100, 1536^3 182 / 137,
-// 2048^3 418 / 246, 4096^3 3214 / 1241 (0.11 PFLOP/s; error 4e-9 of
+// against plan_tc's. Both sides measured (us, DMMA / slices): 256^3 47 / 62,
+// 384^3 124 / 65, 512^3 279 / 70, 1024^3 1983 / 130, 2048^3 15661 / 405,
+// 4096^3 124903 / 2560, 3000 x 2000 x 10 379 / 148, 64 x 4096 x 64 91 / 100.
+// f32 against the FP32 kernels (us): 1024^3 77 / 90, 1280^3 155 / 112,
+// 1536^3 184 / 134, 2048^3 418 / 222, 4096^3 3214 / 1120 (error 4e-9 of
 // (|A||B|)_ij against the FMA chains' 3e-7).
 bool nrs_tc_gemm_pays(int dtype, int64_t m, int64_t k, int64_t n) {
   if (dtype != NRS_F64 && dtype != NRS_F32) return false;
@@ -2142,11 +2282,11 @@ bool nrs_tc_gemm_pays(int dtype, int64_t m, int64_t k, int64_t n) {
   const double plain_us = f32 ? nrs_plain_f32_us(m, k, n)
                               : (double)((m + 31) / 32 * 32) * (double)((n + 31) / 32 * 32) * (double)k * 2.0 / 1.05e6 + 10.0;
   if (plain_us < 60.0) return false;
-  // exponents, estimate, slicing: seven launches, 40 (f32: 16) bytes per
+  // exponents, estimate, slicing: six launches, 40 (f32: 16) bytes per
   // operand element
   const int S = f32 ? 4 : 7;
-  const double tc_us = 45.0 + (mk + kn) * (f32 ? 16.0 : 40.0) / 3e6 +
-                       plan_tc(m, n, (k + 7) / 8 * 8, S).us * (1.0 + 2.0 / (S * (S + 1)));
+  const double tc_us = 30.0 + (mk + kn) * (f32 ? 16.0 : 40.0) / 3e6 +
+                       plan_tc(m, n, slice_pitch(k), S, 16).us * (1.0 + 2.0 / (S * (S + 1)));
   return tc_us <= 0.9 * plain_us;
 }
 
@@ -2182,7 +2322,7 @@ extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, co
   if (ldb < ((tb ? k : n) > 0 ? (tb ? k : n) : 1)) return nrs_fail(h, NRS_ERR_SHAPE, "ldb too small");
   if (slices < 0 || slices > OZ_MAX_SLICES)
     return nrs_fail(h, NRS_ERR_INVALID, "slices must be 0 (auto) or 1..16");
-  const int64_t kpad = ((k + 7) / 8) * 8;
+  const int64_t kpad = slice_pitch(k);
   if (info) std::memset(info, 0, sizeof(*info));
   int b = 0, S = 0, kchunks = 0;
   if (slices > 0) {
@@ -2252,7 +2392,7 @@ extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, co
     info->est_rel_error = slices == 0 ? std::ldexp(std::max(spread, 1.0), -b * S) + std::ldexp(1.0, -53)
                                       : std::ldexp(2.0, -b * S);
   }
-  return ozaki_run(h, a, bT, m, n, k, kpad, b, S, kchunks, C, ldc, accumulate);
+  return ozaki_run(h, a, bT, m, n, k, kpad, b, S, C, ldc, accumulate);
 }
 
 // ---------------------------------------------------------------------------
@@ -2323,16 +2463,16 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
       keep.push_back(i);
       continue;
     }
-    const int64_t kpad8 = (g.k + 7) / 8 * 8;
+    const int64_t kpad1 = slice_pitch(g.k);
     SpreadResult r{};
     const OzOperand a{g.A, g.lda, g.m, true}, bT{g.B, g.ldb, g.n, false};
-    int st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad8, 1, &r);
+    int st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad1, 1, &r);
     if (st) return st;
     if (r.flags & 1u) continue;
     double need = target + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
     int bb, SS, kc;
     if (!(std::isfinite((double)r.rmax) && choose_digits(kp_max, need, &bb, &SS, &kc, kMaxChunkSlicesGrouped))) {
-      if ((st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad8, 2, &r))) return st;
+      if ((st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad1, 2, &r))) return st;
       need = target + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
       if (!(std::isfinite((double)r.rmax) && choose_digits(kp_max, need, &bb, &SS, &kc, kMaxChunkSlicesGrouped)))
         continue;
@@ -2389,7 +2529,7 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
       for (int64_t k0 = 0; k0 < g.k; k0 += kColStrip) colch.push_back(OzChunk{p, (int32_t)c0, (int32_t)k0, 0});
     for (int64_t c0 = 0; c0 < g.n; c0 += kSliceColN)
       for (int64_t k0 = 0; k0 < kpad; k0 += kSliceColK) slcol.push_back(OzChunk{p, (int32_t)c0, (int32_t)k0, 0});
-    constexpr int kBN = OzGeom<true>::BN;
+    constexpr int kBN = OzGeom<false, true>::BN;
     const int tm_n = (int)((g.m + OZ_BM - 1) / OZ_BM), tn_n = (int)((g.n + kBN - 1) / kBN);
     for (int a = 0; a < tm_n; ++a)
       for (int c = 0; c < tn_n; ++c) tiles.push_back({(double)kpad * (S * (S + 1) / 2), OzTile{p, a, c, 0}});
@@ -2407,7 +2547,7 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
                b_pr = al(probs.size() * sizeof(OzProb)), b_tl = al(tl.size() * sizeof(OzTile)),
                b_ea = al((size_t)rowoff * 4), b_eb = al((size_t)coloff * 4), b_cm = al((size_t)coloff * 8),
                b_sa = al((size_t)S * rowoff * kp_max * 2), b_sb = al((size_t)S * coloff * kp_max * 2),
-               b_acc = al((size_t)h->hw_sms * OZ_BM * OzGeom<true>::BN * OZ_DIGIT_BYTES);  // a digit slot per CTA
+               b_acc = al((size_t)h->hw_sms * OZ_BM * OzGeom<false, true>::BN * OZ_DIGIT_BYTES);  // a digit slot per CTA
   const size_t total = b_in + b_rc + b_cc + b_sc + b_pr + b_tl + b_ea + b_eb + b_cm + b_sa + b_sb + b_acc;
   nrs_ozaki_group* G = new nrs_ozaki_group();
   if (cudaMalloc(&G->arena, total) != cudaSuccess) {
