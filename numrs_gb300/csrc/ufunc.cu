@@ -624,9 +624,12 @@ __global__ void __launch_bounds__(256)
       const V v = __ldcs(xv + i + u * stride);
       memcpy(e + u * PER, &v, 16);
     }
-    ea_vec(e, a, b);
+    // (f64: one group of chains for all vectors; f32 stores each as it is
+    // ready: 3480 x 4050 21.9 -> 21.5 us)
+    if constexpr (sizeof(T) == 8) ea_vec(e, a, b);
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u) {
+      if constexpr (sizeof(T) == 4) ea_vec(reinterpret_cast<T(&)[PER]>(e[u * PER]), a, b);
       V v;
       memcpy(&v, e + u * PER, 16);
       __stcs(yv + i + u * stride, v);
