@@ -2118,70 +2118,92 @@ struct OzChunk {
   int32_t prob, r0, k0, pad;  // problem, first row (column), first k
 };
 
-// Row exponents of every A: one warp per row, 8 rows per block. T (double or
-// float) is the group's element type; floats widen to double exactly.
+// The high word of |x| as a double, whose top bits are the exponent (T: double
+// or float, the group's element type; floats widen exactly).
 template <typename T>
-__global__ void __launch_bounds__(256)
-    g_row_exponents(const OzIn* __restrict__ in, const OzChunk* __restrict__ ch, int* __restrict__ ea) {
-  const OzChunk c = ch[blockIdx.x];
-  const OzIn q = in[c.prob];
-  const int64_t row = (int64_t)c.r0 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= q.m) return;
-  uint64_t mx = 0;
-  for (int64_t j = lane; j < q.k; j += 32) {
-    const uint64_t v =
-        (uint64_t)__double_as_longlong((double)static_cast<const T*>(q.A)[row * q.lda + j]) & 0x7FFFFFFFFFFFFFFFULL;
-    mx = v > mx ? v : mx;
-  }
-  for (int off = 16; off; off >>= 1) {
-    const uint64_t o = __shfl_xor_sync(0xffffffffu, mx, off);
-    mx = o > mx ? o : mx;
-  }
-  if (lane == 0) ea[q.rowoff + row] = ((mx >> 52) == 0) ? -1021 : (int)(mx >> 52) - 1022;
+__device__ __forceinline__ uint32_t g_high_bits(T x) {
+  return (uint32_t)__double2hiint((double)x) & 0x7FFFFFFFu;
 }
 
-// Column maxima of every B: 256 columns x 256 k per block, atomicMax on the
-// bit patterns (of the values widened to double) into a zeroed array.
+// Column maxima of every B: 32 columns x 256 k per block, 8 threads per column
+// (2048 problems of 16..512: 85 us with 256-column blocks, half of whose
+// threads had no column, 70 so), atomicMax into a zeroed array.
 template <typename T>
 __global__ void __launch_bounds__(256)
     g_col_max_bits(const OzIn* __restrict__ in, const OzChunk* __restrict__ ch, unsigned long long* __restrict__ colmax) {
+  __shared__ uint32_t part[8][32];
   const OzChunk c = ch[blockIdx.x];
   const OzIn q = in[c.prob];
-  const int64_t col = (int64_t)c.r0 + threadIdx.x;
-  if (col >= q.n) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t col = (int64_t)c.r0 + tx;
   const int64_t r1 = (c.k0 + kColStrip) < q.k ? (c.k0 + kColStrip) : q.k;
-  unsigned long long mx = 0;
-  for (int64_t i = c.k0; i < r1; ++i) {
-    const unsigned long long v =
-        (unsigned long long)__double_as_longlong((double)static_cast<const T*>(q.B)[i * q.ldb + col]) &
-        0x7FFFFFFFFFFFFFFFULL;
-    mx = v > mx ? v : mx;
+  uint32_t mx = 0;
+  if (col < q.n) {
+    const T* p = static_cast<const T*>(q.B) + col;
+#pragma unroll 8
+    for (int64_t i = c.k0 + ty; i < r1; i += 8) mx = max(mx, g_high_bits(p[i * q.ldb]));
   }
-  atomicMax(&colmax[q.coloff + col], mx);
+  part[ty][tx] = mx;
+  __syncthreads();
+  if (ty == 0 && col < q.n) {
+#pragma unroll
+    for (int r = 1; r < 8; ++r) mx = max(mx, part[r][tx]);
+    atomicMax(&colmax[q.coloff + col], (unsigned long long)mx << 32);
+  }
 }
 
-// A slices of every problem: a block takes 8 rows of one problem, a thread 8
-// consecutive k of one row (zero beyond k, up to the problem's kpad).
+// Row exponents and slices of every A: a block takes 8 rows of one problem.
+// Each warp finds two rows' exponents; then a thread slices 8 consecutive k of
+// one row (zero beyond k, up to the problem's kpad), whose second read hits
+// the caches. A block's chain of dependent loads (chunk, problem, row, slices)
+// bounds it, so blocks are small and nine fit an SM. (2048 problems of 16..512:
+// 97 + 263 us with the exponents in their own launch, 357 fused in blocks of
+// 256 threads, 261 in blocks of 128.)
 template <typename T, int b, bool SMALL>
-__global__ void __launch_bounds__(256)
-    g_slice_rows(const OzIn* __restrict__ in, const OzChunk* __restrict__ ch, const int* __restrict__ ea, int S,
+__global__ void __launch_bounds__(128)
+    g_slice_rows(const OzIn* __restrict__ in, const OzChunk* __restrict__ ch, int* __restrict__ ea, int S,
                  int64_t pitch, int64_t plane, uint16_t* __restrict__ out) {
+  __shared__ int row_e[8];
   const OzChunk c = ch[blockIdx.x];
   const OzIn q = in[c.prob];
-  const int64_t groups = q.kpad / 8;
+  const T* const Aq = static_cast<const T*>(q.A) + (int64_t)c.r0 * q.lda;
+  {
+    const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool ok[2] = {c.r0 + r < q.m, c.r0 + r + 4 < q.m};
+    uint32_t mx[2] = {0, 0};
+#pragma unroll 4
+    for (int64_t j = lane; j < q.k; j += 32) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (ok[i]) mx[i] = max(mx[i], g_high_bits(Aq[(r + 4 * i) * q.lda + j]));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t m = __reduce_max_sync(0xffffffffu, mx[i]);
+      if (lane == 0 && ok[i]) {
+        const int e = (m >> 20) == 0 ? -1021 : (int)(m >> 20) - 1022;
+        row_e[r + 4 * i] = e;
+        ea[q.rowoff + c.r0 + r + 4 * i] = e;
+      }
+    }
+  }
+  __syncthreads();
+  const bool vec = (reinterpret_cast<uintptr_t>(q.A) & 15) == 0 && (q.lda * sizeof(T)) % 16 == 0;
+  const uint32_t groups = (uint32_t)(q.kpad / 8);
   const unsigned __int128 C = digit_offset(S, b);
   const uint64_t C64 = ozaki_offset64(S, b);
-  for (int64_t w = threadIdx.x; w < 8 * groups; w += blockDim.x) {
-    const int64_t row = (int64_t)c.r0 + w / groups, j0 = (w % groups) * 8;
+  for (uint32_t w = threadIdx.x; w < 8 * groups; w += blockDim.x) {
+    const uint32_t r = w / groups;
+    const int64_t row = (int64_t)c.r0 + r, j0 = (int64_t)(w - r * groups) * 8;
     if (row >= q.m) break;  // w only grows: every later item is beyond m too
-    const int e = ea[q.rowoff + row];
-    const T* src = static_cast<const T*>(q.A) + row * q.lda + j0;
+    const int e = row_e[r];
+    T x[8];
+    load_run(Aq + r * q.lda + j0, vec, q.k - j0, x);
     uint16_t* o = out + (q.rowoff + row) * pitch + j0;
     if constexpr (SMALL) {
       OzakiZ64 Z[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) Z[t] = ozaki_z64(j0 + t < q.k ? src[t] : T(0), e, b, S, C64);
+      for (int t = 0; t < 8; ++t) Z[t] = ozaki_z64(x[t], e, b, S, C64);
 #pragma unroll
       for (int t = 0; t < OZ_MAX_SLICES; ++t) {
         if (t < S) {
@@ -2196,7 +2218,7 @@ __global__ void __launch_bounds__(256)
     } else {
       unsigned __int128 Z[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) Z[t] = (unsigned __int128)fixed126(j0 + t < q.k ? src[t] : T(0), e) + C;
+      for (int t = 0; t < 8; ++t) Z[t] = (unsigned __int128)fixed126(x[t], e) + C;
 #pragma unroll
       for (int t = 0; t < OZ_MAX_SLICES; ++t) {
         if (t < S) {
@@ -2525,7 +2547,7 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
     probs.push_back(OzProb{g.m, g.n, kpad, rowoff, coloff, g.C, g.ldc, kc, S * (S + 1) / 2 * kc,
                            (g.flags & NRS_GEMM_ACCUMULATE) ? 1 : 0, f32 ? 1 : 0});
     for (int64_t r = 0; r < g.m; r += 8) rowch.push_back(OzChunk{p, (int32_t)r, 0, 0});
-    for (int64_t c0 = 0; c0 < g.n; c0 += 256)
+    for (int64_t c0 = 0; c0 < g.n; c0 += 32)
       for (int64_t k0 = 0; k0 < g.k; k0 += kColStrip) colch.push_back(OzChunk{p, (int32_t)c0, (int32_t)k0, 0});
     for (int64_t c0 = 0; c0 < g.n; c0 += kSliceColN)
       for (int64_t k0 = 0; k0 < kpad; k0 += kSliceColK) slcol.push_back(OzChunk{p, (int32_t)c0, (int32_t)k0, 0});
@@ -2605,7 +2627,7 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
 template <typename T, int b, bool SMALL>
 int group_slices_s(nrs_handle* h, nrs_ozaki_group* G, cudaStream_t s) {
   const int64_t plane_a = G->rows_a * G->pitch, plane_b = G->rows_b * G->pitch;
-  g_slice_rows<T, b, SMALL><<<(unsigned)G->n_rowch, 256, 0, s>>>(G->d_in, G->d_rowch, G->d_ea, G->S, G->pitch,
+  g_slice_rows<T, b, SMALL><<<(unsigned)G->n_rowch, 128, 0, s>>>(G->d_in, G->d_rowch, G->d_ea, G->S, G->pitch,
                                                                  plane_a, G->d_sa);
   const int smem = (int)((size_t)G->S * kSliceColN * kSliceColPitch * 4);
   int st = nrs_cuda_check(
@@ -2623,7 +2645,6 @@ int group_slices(nrs_handle* h, nrs_ozaki_group* G, cudaStream_t s) {
 
 template <typename T>
 int group_prepare(nrs_handle* h, nrs_ozaki_group* G, cudaStream_t s) {
-  g_row_exponents<T><<<(unsigned)G->n_rowch, 256, 0, s>>>(G->d_in, G->d_rowch, G->d_ea);
   g_col_max_bits<T><<<(unsigned)G->n_colch, 256, 0, s>>>(G->d_in, G->d_colch, G->d_colmax);
   exponents_from_bits<<<(unsigned)((G->rows_b + 255) / 256), 256, 0, s>>>(G->d_colmax, G->rows_b, G->d_eb);
   int st = nrs_after_launch(h, "grouped ozaki exponents");
