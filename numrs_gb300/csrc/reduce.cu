@@ -28,7 +28,8 @@
 // reference's 8192-element chunking: one warp sums a chunk with a
 // lane-striped tree (256 lanes, eight per thread, 16-byte loads), chunk
 // partials go to workspace, and a single CTA folds them (in chunk order up to
-// 1024 chunks, else as 1024 interleaved runs folded in order).
+// 1024 chunks, else as 1024 interleaved runs folded in order); at most 32
+// chunks of at most 512 KB go through both steps in one launch.
 #include <cfloat>
 #include <type_traits>
 #include <climits>
