@@ -179,7 +179,7 @@ NRS_DEV void mbar_arrive(uint64_t* bar) {
 
 // Thread-block clusters: the CTA's rank, the address of its shared memory's
 // counterpart in another CTA, arrivals on a barrier there, and the barrier
-// over all threads of the cluster (convergent warps).
+// over all threads of the cluster.
 NRS_DEV uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -194,6 +194,7 @@ NRS_DEV void mbar_arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
 NRS_DEV void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -9,6 +9,8 @@ inner edges.
 import pytest
 import torch
 
+from numrs_gb300 import _lib as L
+
 pytestmark = pytest.mark.gpu
 
 
@@ -48,10 +50,20 @@ def test_pair_accumulates_into_a_pitched_view(K):
 
 
 # several K ranges on pairs (the slabs are added in order): the error bar of 16 ranges
-@pytest.mark.parametrize("m,k,n", [(1536, 1536, 1536), (1000, 8192, 1030), (1999, 1537, 3001)])
+@pytest.mark.parametrize("m,k,n", [(1536, 1536, 1536), (1000, 8192, 1000), (1999, 1537, 3001)])
 def test_pair_with_k_ranges(K, m, k, n):
     a, b = _operand(m, k, 5), _operand(k, n, 6)
     c = K.matmul(a, b)
     ref, _ = K.gemm_ozaki(a, b, slices=12)  # 2^-96 of the scaled operands: its own rounding of C only
     bar = 2e-15 * (a.abs() @ b.abs())
     assert bool(((c - ref).abs() <= bar).all())
+
+
+def test_pair_launch_returns_at_once_for_operands_it_cannot_carry(K):
+    a, b = _operand(2048, 700, 7), _operand(700, 2100, 8)
+    a[5, 9], b[3, 77] = float("inf"), float("nan")
+    c, d = K.matmul(a, b), K.matmul(a, b, variant=L.GEMM_DMMA)
+    assert torch.equal(c.isnan(), d.isnan())
+    assert torch.equal(torch.nan_to_num(c, nan=7.0), torch.nan_to_num(d, nan=7.0))
+    a[5, 9], b[3, 77] = 1.0, 1.0  # and the next call on the stream is served
+    assert bool(((K.matmul(a, b) - a @ b).abs() <= 1e-12 * (a.abs() @ b.abs())).all())
