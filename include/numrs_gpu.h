@@ -352,10 +352,13 @@ typedef enum nrs_gemm_variant {
  * integer dtypes wrap like gemm_generic (:408).
  * NRS_GEMM_AUTO: f64 and f32 products large enough for it run as slice
  * products on the tensor cores (nrs_gemm_ozaki's scheme, with the slice count
- * decided on the device: nothing is read back, the call stays asynchronous),
- * with an error no larger than the plain kernels'; everything else, operands
- * that the slices cannot carry and calls under stream capture run the plain
- * kernels. Their scratch is stream-ordered and the library's own. */
+ * decided on the device: nothing is read back, the call stays asynchronous).
+ * Whatever the operands, |C - AB|_ij is then at most 10 units of the element
+ * type (2^-53, 2^-24) of (|A||B|)_ij, for f64 one more per further range when
+ * K runs in up to 16 ranges; a K-long FMA chain's bound is K units. Everything
+ * else, operands that the slices cannot carry to that and calls under stream
+ * capture run the plain kernels. Their scratch is stream-ordered and the
+ * library's own. */
 int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A,
              int64_t lda, const void* B, int64_t ldb, void* C, int64_t ldc, unsigned flags,
              int variant);
@@ -410,7 +413,10 @@ typedef struct nrs_ozaki_info {
  * tensor-core product of |A'| and |B'| and the row / column sums; if some
  * (|A'||B'|)_ij is 0, a second pass counts only the k where the other factor
  * is nonzero). Each operand is then carried to 53 + log2(max R) bits, which
- * keeps max_ij |C - AB|_ij / (|A||B|)_ij at about 2^-53. If no count within
+ * keeps the error of its rounding at 2^-53 of (|A||B|)_ij, and to as many more
+ * as keep the slice pairs that are not multiplied (at most (S - 1) 2^-(bS) per
+ * k, whatever the entries) within (K / 4 + 4) 2^-53, a quarter of a K-long FP64
+ * chain's bound; entries that do not repeat along K stay far below it. If no count within
  * the limits (16 slices, 126 bits, exact int32 sums for this K, an exact
  * total within 128 bits: b (S - 1) <= 95 for b-bit digits) reaches that, or an operand holds Inf or NaN, the call runs the native FP64 DMMA
  * GEMM and reports slices = 0. The automatic mode reads the measured spread

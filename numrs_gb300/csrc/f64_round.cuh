@@ -229,6 +229,41 @@ NRS_HD uint64_t ozaki_round96(int32_t R, uint32_t fhi, uint32_t flo, int e, bool
 }
 
 // ---------------------------------------------------------------------------
+// The slice count
+// ---------------------------------------------------------------------------
+// Two things separate the slices' sum from C_ij = sum_k a'_ik b'_kj (scaled
+// operands, D_ij = sum_k |a'_ik||b'_kj|):
+//  * each operand's rounding, at most 2^-(bS) sum_k (|a'_ik| + |b'_kj|), i.e.
+//    2^-(bS) D_ij times the spread R_ij;
+//  * the slice pairs with s + t >= S, which are not multiplied. For one k, digit
+//    s of a' is at most 2^-(bs) and the tail of b' that it misses, the digits
+//    from S - s on, at most 2^-(b(S-s)): together at most (S - 1) 2^-(bS),
+//    however small the entries are, and of one sign when the entries repeat.
+// So S holds when 2^-(bS) R <= 2^-target and (S - 1) 2^-(bS) K / min D is at
+// most `tau` times that: spread = max R, drop = K / (tau min D).
+NRS_HD float nrs_exp2i(int e) {  // -126 <= e <= 127
+  const uint32_t u = (uint32_t)(e + 127) << 23;
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+}
+NRS_HD bool ozaki_count_holds(int S, int b, int target, float spread, float drop) {
+  const float room = nrs_exp2i(b * S - target);
+  return spread <= room && (float)(S - 1) * drop <= room;
+}
+// The tau of a product that stands in for a plain kernel unasked: 7 units of
+// the element type (2^-53; 2^-24, i.e. four times the target 2^-26), so that all
+// is within 10 with the operands' and the result's rounding and the percent or
+// two of an estimated D. A plain chain's own error is of that size (8 units at
+// K = 8192), and the dense cases keep the count that the spread gives.
+NRS_HD float ozaki_drop_units(int target) { return target >= 53 ? 7.0f : 28.0f; }
+// The tau of a call that asks for the slices: a quarter of the bound K of a
+// K-long chain of the element type, and 4 units.
+NRS_HD float ozaki_drop_units_asked(int target, double k) {
+  return (float)((k * 0.24 + 4.0) * (target >= 53 ? 1.0 : 4.0));
+}
+
+// ---------------------------------------------------------------------------
 // Slicing with 64-bit integers when b S <= 64
 // ---------------------------------------------------------------------------
 // The slicers round X = x 2^(126-e) (exact for |x| < 2^e) to a multiple of

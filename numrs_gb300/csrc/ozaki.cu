@@ -15,8 +15,9 @@
 //    exactly representable in BF16, and x = sum_t digit_t * 2^-(b - 1 + bt)
 //    up to 2^-(bS). Slices are stored K-major ([S][rows][kpad] bf16) for A
 //    and for B^T (the B slicer transposes through shared memory).
-// 3. Products: for every slice pair (s, t) with s + t <= S-1 (the pairs
-//    whose weight 2^-(2b - 2 + b(s+t)) matters), P = A_s * B_t^T on the
+// 3. Products: for every slice pair (s, t) with s + t <= S-1 (what the others
+//    can add up to counts in the choice of S: ozaki_count_holds in
+//    f64_round.cuh), P = A_s * B_t^T on the
 //    tensor cores with FP32 accumulation. |digit products| <= 2^(2b-2), so
 //    every partial sum of a K <= 2^(26-2b) chunk (4096 for b = 7) is an
 //    integer of at most 2^24: the FP32 accumulation is EXACT.
@@ -259,6 +260,7 @@ struct OzRule {
   int target_bits;  // operand bits wanted at spread 1 (53 for f64, 26 for f32)
   int digit_bits;
   int max_slices;   // beyond: 0 (the caller's FP64 / FP32 kernel runs instead)
+  float drop_scale; // K / tau of ozaki_count_holds
   int exp_limit;    // max row + column exponent whose dot products cannot overflow T
 };
 
@@ -266,22 +268,23 @@ struct OzRule {
 // estimate product.
 // OZ_W_COUNT: the slice count that oz_slice decided on, read by the launches
 // behind it.
-enum { OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_EXP_A = 2, OZ_W_EXP_B = 3, OZ_W_COUNT = 4, OZ_WORDS = 5 };
+// OZ_W_DROP: 1 / min_ij (|A'||B'|)_ij over its nonzero entries, as float bits.
+enum { OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_DROP = 2, OZ_W_EXP_A = 3, OZ_W_EXP_B = 4, OZ_W_COUNT = 5, OZ_WORDS = 6 };
 constexpr int kExpBias = 4096;  // exponents are collected biased, as unsigned maxima
 
-// The slice count for the measured spread R (float bits): the smallest S with
-// R <= 2^(b S - target), so that 2^-(bS) R stays at the target; 0 when no
-// count up to the limit reaches it, an operand holds Inf or NaN, or a partial
-// sum could overflow the element type (the plain kernel then gives its own
-// Inf / NaN).
+// The slice count for the measured spread and smallest (|A'||B'|)_ij: the
+// smallest S for which ozaki_count_holds; 0 when no count up to the limit
+// does, an operand holds Inf or NaN, or a partial sum could overflow the
+// element type (the plain kernel then gives its own Inf / NaN).
 __device__ __forceinline__ int oz_decide(const uint32_t* w, const OzRule& r) {
-  const uint32_t spread = __ldcg(w + OZ_W_SPREAD);
+  const float spread = __uint_as_float(__ldcg(w + OZ_W_SPREAD));
+  const float drop = __uint_as_float(__ldcg(w + OZ_W_DROP)) * r.drop_scale;
   if (__ldcg(w + OZ_W_NONFINITE)) return 0;
   const int e = (int)__ldcg(w + OZ_W_EXP_A) + (int)__ldcg(w + OZ_W_EXP_B) - 2 * kExpBias;
   if (e > r.exp_limit) return 0;
   int S = (r.target_bits + r.digit_bits - 1) / r.digit_bits;
   for (; S <= r.max_slices; ++S)
-    if (spread <= (uint32_t)(127 + r.digit_bits * S - r.target_bits) << 23) return S;
+    if (ozaki_count_holds(S, r.digit_bits, r.target_bits, spread, drop)) return S;
   return 0;
 }
 
@@ -307,8 +310,9 @@ struct OzParams {
   uint32_t* err;
   // Spread estimate only (EST kernel): row sums of |A'| and column sums of
   // |B'| (operands scaled by their row / column exponents; fixed point, in
-  // units of sum_unit), and the word that collects max_ij of the ratio as
-  // float bits.
+  // units of sum_unit), and the decision words, of which it raises the spread
+  // (max_ij of the ratio) and the inverse of the smallest nonzero D, as float
+  // bits.
   const uint32_t* ra;
   const uint32_t* cb;
   float sum_unit;
@@ -603,7 +607,8 @@ __device__ __forceinline__ TileCtx tile_ctx(const OzParams& P, int S, int tile, 
 //              D = |A'| |B'|^T; pass 2 (slices = 2) also runs the two cross
 //              products N = |A'| 1_B^T + 1_A |B'|^T of slices 0 and 1 (|x'|
 //              and the nonzero indicator). The epilogue folds
-//              max_ij (numerator_ij / D_ij) into P.est instead of writing C.
+//              max_ij (numerator_ij / D_ij) and the smallest nonzero D_ij into
+//              P.est instead of writing C.
 // B8: 8-bit digits (else 7 or 6, P.digit_bits).
 template <bool EST, bool G, bool B8>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
@@ -802,7 +807,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const uint32_t acc_t = lane_base;
     const uint32_t dsum_t = lane_base + OZ_BN;
     uint32_t ai = 0;
-    float rmax = 0.0f;
+    const float inf = __uint_as_float(0x7f800000u);
+    float rmax = 0.0f, dmin = inf;
     bool ok = true;
     for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
       const TileCtx tc = tile_ctx<EST, G>(P, S, tile, rank);
@@ -851,8 +857,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             else num = __uint_as_float(w[e]);
             // (the threshold test of the count tolerates the approximate
             // division's two ulp)
-            r = D > 0.0f ? __fdividef(num, D) : num > 0.0f ? __uint_as_float(0x7f800000u) : 0.0f;
-            if (row_ok && col < tc.n) rmax = fmaxf(rmax, r);
+            r = D > 0.0f ? __fdividef(num, D) : num > 0.0f ? inf : 0.0f;
+            if (row_ok && col < tc.n) {
+              rmax = fmaxf(rmax, r);
+              if (D > 0.0f) dmin = fminf(dmin, D);
+            }
           }
         }
         tmem_wait_st();
@@ -861,8 +870,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         if (lane == 0) mbar_arrive(&acce[buf]);
       }
     }
-    for (int off = 16; off; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
-    if (lane == 0 && ok) atomicMax(P.est, __float_as_uint(rmax));
+    for (int off = 16; off; off >>= 1) {
+      rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
+      dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, off));
+    }
+    if (lane == 0 && ok) {
+      atomicMax(P.est + OZ_W_SPREAD, __float_as_uint(rmax));
+      if (dmin < inf) atomicMax(P.est + OZ_W_DROP, __float_as_uint(0x1p96f / dmin));
+    }
   } else if (G) {
     // ---------------- grouped epilogue (warps 2..9) ----------------
     // Warp w reads TMEM lane quarter w % 4 (one tile row per thread); the
@@ -1869,14 +1884,25 @@ bool digits_fit(int b, int S, int64_t kpad, int64_t max_kcs) {
   return S >= 1 && S <= OZ_MAX_SLICES && b * S <= 126 && b * (S - 1) <= 95 && kc * S <= max_kcs;
 }
 
-// Digit width and count for `bits` bits of each operand's fixed-point value:
-// the widest b (8, 7, 6) with S = ceil(bits / b) inside digits_fit's limits.
-// false if no width qualifies.
-bool choose_digits(int64_t kpad, double bits, int* b, int* S, int* kchunks,
+// What a call's operands ask of a slice count (ozaki_count_holds): the bits
+// that the spread needs and, for the pairs left out, target + log2 drop.
+struct OzNeed {
+  double bits, drop_bits;
+};
+
+// The least count for digits of b bits.
+int slices_for(int b, const OzNeed& need) {
+  int S = std::max(1, (int)std::ceil(need.bits / b - 1e-9));
+  while (S <= OZ_MAX_SLICES && S > 1 && b * S < need.drop_bits + std::log2((double)(S - 1))) ++S;
+  return S;
+}
+
+// Digit width and count: the widest b (8, 7, 6) whose least count is inside
+// digits_fit's limits. false if no width qualifies.
+bool choose_digits(int64_t kpad, const OzNeed& need, int* b, int* S, int* kchunks,
                    int64_t max_kcs = kMaxChunkSlices) {
   for (int cand = 8; cand >= 6; --cand) {
-    int s_c = (int)std::ceil(bits / cand - 1e-9);
-    if (s_c < 1) s_c = 1;
+    const int s_c = slices_for(cand, need);
     const int64_t kc = (kpad + kChunkOf(cand) - 1) / kChunkOf(cand);
     if (digits_fit(cand, s_c, kpad, max_kcs)) {
       *b = cand;
@@ -1888,15 +1914,20 @@ bool choose_digits(int64_t kpad, double bits, int* b, int* S, int* kchunks,
   return false;
 }
 
-// Bits of the fixed-point operands that keep the slicing error at FP64's
-// unit roundoff relative to (|A||B|)_ij: each operand element is rounded at
-// 2^-(bS) (scaled units), so |C - AB|_ij <~ 2^-(bS) (sum_k |a'_ik| + |b'_kj|)
-// = 2^-(bS) R_ij (|A'||B'|)_ij, and bS >= 53 + log2 max_ij R_ij.
-constexpr double kTargetBits = 53.0;
+// Bits of the fixed-point operands that keep their rounding at FP64's unit
+// roundoff relative to (|A||B|)_ij: bS >= 53 + log2 max_ij R_ij; 26 (24 and two
+// guard bits) for f32.
+constexpr int kTargetBits = 53, kTargetBits32 = 26;
 
 struct SpreadResult {
   float rmax;
   uint32_t flags;  // bit 0: an operand holds Inf or NaN
+  float dinv;      // 1 / the smallest nonzero (|A'||B'|)_ij
+  bool finite() const { return std::isfinite((double)rmax) && std::isfinite((double)dinv); }
+  OzNeed need(int target, int64_t k) const {
+    const double drop = (double)dinv * (double)k / ozaki_drop_units_asked(target, (double)k);
+    return OzNeed{target + (rmax > 1.0f ? std::log2((double)rmax) : 0.0), drop > 0.0 ? target + std::log2(drop) : 0.0};
+  }
 };
 
 // Enqueues the spread estimate: exponents, estimate operands and one (pass
@@ -1915,7 +1946,7 @@ int launch_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int6
   P.ra = w.ra;
   P.cb = w.cb;
   P.sum_unit = 1.0f / oz_sum_scale(k);
-  P.est = w.words + OZ_W_SPREAD;
+  P.est = w.words;
   return launch_tc<true, false>(h, w.area_a, w.area_b, pass, P, m, n, h->stream);
 }
 
@@ -1931,19 +1962,18 @@ int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, bool
            : launch_estimate<double>(h, a, bT, m, n, k, kpad, pass, w);
   if (st) return st;
   cudaStream_t s = h->stream;
-  uint32_t host[2] = {0, 0};
-  static_assert(OZ_W_SPREAD == 0 && OZ_W_NONFINITE == 1, "the two words read back");
-  if ((st = nrs_cuda_check(h, cudaMemcpyAsync(host, w.words, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync")))
+  uint32_t host[3] = {0, 0, 0};
+  static_assert(OZ_W_SPREAD == 0 && OZ_W_NONFINITE == 1 && OZ_W_DROP == 2, "the words read back");
+  if ((st = nrs_cuda_check(h, cudaMemcpyAsync(host, w.words, sizeof(host), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync")))
     return st;
   if ((st = nrs_cuda_check(h, cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return st;
   uint32_t derr = 0;
   if ((st = nrs_cuda_check(h, cudaMemcpy(&derr, h->dev_error, 4, cudaMemcpyDeviceToHost), "cudaMemcpy")))
     return st;
   if (derr) return nrs_fail(h, NRS_ERR_TIMEOUT, "ozaki spread estimate: a device-side bounded wait gave up");
-  float r;
-  std::memcpy(&r, &host[0], 4);
-  res->rmax = r;
-  res->flags = host[1];
+  std::memcpy(&res->rmax, &host[OZ_W_SPREAD], 4);
+  std::memcpy(&res->dinv, &host[OZ_W_DROP], 4);
+  res->flags = host[OZ_W_NONFINITE];
   return NRS_OK;
 }
 
@@ -2053,7 +2083,8 @@ int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, i
   if (!digits_fit(b, kAutoMaxSlices, kpad, kMaxChunkSlicesGrouped)) return NRS_ERR_UNSUPPORTED;
   int klog = 0;
   while (((int64_t)1 << klog) < k) ++klog;
-  const OzRule rule{F32 ? 26 : 53, b, kAutoMaxSlices, (F32 ? 127 : 1023) - klog - 1};
+  constexpr int target = F32 ? kTargetBits32 : kTargetBits;
+  const OzRule rule{target, b, kAutoMaxSlices, (float)((double)k / ozaki_drop_units(target)), (F32 ? 127 : 1023) - klog - 1};
   const TcPlan pl = plan_tc(m, n, kpad, F32 ? 4 : 7, 16);
   const int plain_splits = F32 ? 1 : nrs_dmma_splits(m, k, n);
   const int slabs = std::max(pl.splits > 1 ? pl.splits : 0, plain_splits > 1 ? plain_splits : 0);
@@ -2385,23 +2416,22 @@ extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, co
     return nrs_gemm(h, NRS_F64, m, k, n, A, lda, B, ldb, C, ldc, flags, NRS_GEMM_DMMA);
   };
 
-  double spread = 0.0;
+  double spread = 0.0, dropped = 0.0;
   if (slices == 0) {
     SpreadResult r{};
     if ((st = spread_estimate(h, a, bT, false, m, n, k, kpad, 1, &r))) return st;
     if (r.flags & 1u) return fallback("non-finite operand");
-    double need = kTargetBits + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
-    if (!(std::isfinite((double)r.rmax) && choose_digits(kpad, need, &b, &S, &kchunks))) {
+    if (!(r.finite() && choose_digits(kpad, r.need(kTargetBits, k), &b, &S, &kchunks))) {
       // The pass-1 numerator counts every k; pass 2 counts only the k where
       // the other operand is nonzero (sparse and structured operands).
       if ((st = spread_estimate(h, a, bT, false, m, n, k, kpad, 2, &r))) return st;
-      need = kTargetBits + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
-      if (!(std::isfinite((double)r.rmax) && choose_digits(kpad, need, &b, &S, &kchunks))) {
+      if (!(r.finite() && choose_digits(kpad, r.need(kTargetBits, k), &b, &S, &kchunks))) {
         if (info) info->spread = std::isfinite((double)r.rmax) ? (double)r.rmax : HUGE_VAL;
         return fallback("spread beyond the slice limits");
       }
     }
     spread = r.rmax;
+    dropped = (double)(S - 1) * (double)k * (double)r.dinv;
   }
   if (info) {
     info->slices = S;
@@ -2409,10 +2439,10 @@ extern "C" int nrs_gemm_ozaki(nrs_handle* h, int64_t m, int64_t k, int64_t n, co
     info->slice_bits = b;
     info->k_chunk = kChunkOf(b);
     info->spread = spread;
-    // auto: 2^-(bS) R_max (+ the final rounding); explicit: relative to
-    // rowmax|A| colmax|B| k, as no spread was measured
-    info->est_rel_error = slices == 0 ? std::ldexp(std::max(spread, 1.0), -b * S) + std::ldexp(1.0, -53)
-                                      : std::ldexp(2.0, -b * S);
+    // auto: 2^-(bS) (R_max and the pairs left out), and the final rounding;
+    // explicit: relative to rowmax|A| colmax|B| k, as no spread was measured
+    info->est_rel_error = slices == 0 ? std::ldexp(std::max(spread, 1.0) + dropped, -b * S) + std::ldexp(1.0, -53)
+                                      : std::ldexp(S + 1.0, -b * S);
   }
   return ozaki_run(h, a, bT, m, n, k, kpad, b, S, C, ldc, accumulate);
 }
@@ -2452,12 +2482,10 @@ int nrs_ozaki_group_info(const nrs_ozaki_group* g, int* slices, int* bits, int64
 
 // The row-major GEMMs of element type `dtype` (NRS_F64 or NRS_F32) as one
 // group. Slice count for `slices` = 0: each problem's spread measured now
-// (one read-back each); the group takes the largest count, carrying each
-// operand to 53 + log2(max R) bits for f64 and 26 + log2(max R) (f32's 24
-// and two guard bits) for f32. Problems whose spread no count covers, or
+// (one read-back each); the group takes the largest count that one of them
+// needs. Problems whose spread no count covers, or
 // with Inf / NaN, are left out (they stay on the persistent kernel's DMMA or
 // FP32 tiles). digit_bits 0 = the widest width the group's K allows.
-constexpr double kTargetBits32 = 26.0;
 int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, int dtype, int slices,
                           int digit_bits, int* accepted, nrs_ozaki_group** out) {
   *out = nullptr;
@@ -2476,8 +2504,8 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
   }
   if (idx.empty()) return NRS_OK;
   const bool f32 = dtype == NRS_F32;
-  const double target = f32 ? kTargetBits32 : kTargetBits;
-  double bits_max = target;
+  const int target = f32 ? kTargetBits32 : kTargetBits;
+  OzNeed most{(double)target, 0.0};
   std::vector<int64_t> keep;
   for (int64_t i : idx) {
     const nrs_gemm_desc& g = d[i];
@@ -2491,22 +2519,22 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
     int st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad1, 1, &r);
     if (st) return st;
     if (r.flags & 1u) continue;
-    double need = target + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
     int bb, SS, kc;
-    if (!(std::isfinite((double)r.rmax) && choose_digits(kp_max, need, &bb, &SS, &kc, kMaxChunkSlicesGrouped))) {
+    if (!(r.finite() && choose_digits(kp_max, r.need(target, g.k), &bb, &SS, &kc, kMaxChunkSlicesGrouped))) {
       if ((st = spread_estimate(h, a, bT, f32, g.m, g.n, g.k, kpad1, 2, &r))) return st;
-      need = target + (r.rmax > 1.0f ? std::log2((double)r.rmax) : 0.0);
-      if (!(std::isfinite((double)r.rmax) && choose_digits(kp_max, need, &bb, &SS, &kc, kMaxChunkSlicesGrouped)))
+      if (!(r.finite() && choose_digits(kp_max, r.need(target, g.k), &bb, &SS, &kc, kMaxChunkSlicesGrouped)))
         continue;
     }
-    bits_max = std::max(bits_max, need);
+    const OzNeed need = r.need(target, g.k);
+    most.bits = std::max(most.bits, need.bits);
+    most.drop_bits = std::max(most.drop_bits, need.drop_bits);
     keep.push_back(i);
   }
   if (keep.empty()) return NRS_OK;
   int b = 0, S = 0, kc_max = 0;
   if (digit_bits) {
     // a given width: S from the bits (or as given), if the width's limits hold
-    const int s_c = slices > 0 ? slices : std::max(1, (int)std::ceil(bits_max / digit_bits - 1e-9));
+    const int s_c = slices > 0 ? slices : slices_for(digit_bits, most);
     if (digits_fit(digit_bits, s_c, kp_max, kMaxChunkSlicesGrouped)) {
       b = digit_bits;
       S = s_c;
@@ -2523,7 +2551,7 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
       }
     }
     if (!b) return nrs_fail(h, NRS_ERR_TOO_LARGE, "k too large for this slice count");
-  } else if (!choose_digits(kp_max, bits_max, &b, &S, &kc_max, kMaxChunkSlicesGrouped)) {
+  } else if (!choose_digits(kp_max, most, &b, &S, &kc_max, kMaxChunkSlicesGrouped)) {
     return NRS_OK;  // nothing qualifies together: all stay on DMMA
   }
   (void)kc_max;
