@@ -356,9 +356,10 @@ typedef enum nrs_gemm_variant {
  * Whatever the operands, |C - AB|_ij is then at most 10 units of the element
  * type (2^-53, 2^-24) of (|A||B|)_ij, for f64 one more per further range when
  * K runs in up to 16 ranges; a K-long FMA chain's bound is K units. Everything
- * else, operands that the slices cannot carry to that and calls under stream
- * capture run the plain kernels. Their scratch is stream-ordered and the
- * library's own. */
+ * else and calls under stream capture run the plain kernels, and so do operands
+ * that the slices cannot carry to that (Inf or NaN, sums that may overflow,
+ * entries too far apart for 12 slices), after the measurement that finds them.
+ * Their scratch is stream-ordered and the library's own. */
 int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A,
              int64_t lda, const void* B, int64_t ldb, void* C, int64_t ldc, unsigned flags,
              int variant);

@@ -269,17 +269,30 @@ struct OzRule {
 // OZ_W_COUNT: the slice count that oz_slice decided on, read by the launches
 // behind it.
 // OZ_W_DROP: 1 / min_ij (|A'||B'|)_ij over its nonzero entries, as float bits.
-enum { OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_DROP = 2, OZ_W_EXP_A = 3, OZ_W_EXP_B = 4, OZ_W_COUNT = 5, OZ_WORDS = 6 };
+// OZ_W_HOLE: pass 1 met a (|A'||B'|)_ij of 0 whose row or column is not zero.
+// OZ_W_TINY: an operand holds a nonzero entry so small (est_bits) that its
+// products with another can be lost in |A'||B'|.
+enum {
+  OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_DROP = 2, OZ_W_HOLE = 3, OZ_W_EXP_A = 4, OZ_W_EXP_B = 5, OZ_W_COUNT = 6,
+  OZ_W_TINY = 7, OZ_WORDS = 8
+};
+// Raises a word to at least v; most callers find it there already.
+__device__ __forceinline__ void raise_word(uint32_t* w, uint32_t v) {
+  if (__ldcg(w) < v) atomicMax(w, v);
+}
 constexpr int kExpBias = 4096;  // exponents are collected biased, as unsigned maxima
 
 // The slice count for the measured spread and smallest (|A'||B'|)_ij: the
 // smallest S for which ozaki_count_holds; 0 when no count up to the limit
 // does, an operand holds Inf or NaN, or a partial sum could overflow the
-// element type (the plain kernel then gives its own Inf / NaN).
+// element type (the plain kernel then gives its own Inf / NaN). Where
+// (|A'||B'|)_ij is 0 (zero rows and columns, identity, block-diagonal and
+// one-hot operands) every product of the sum has a zero factor, whose digits are
+// zeros: C_ij is exact at any count. Only tiny entries make that uncertain.
 __device__ __forceinline__ int oz_decide(const uint32_t* w, const OzRule& r) {
   const float spread = __uint_as_float(__ldcg(w + OZ_W_SPREAD));
   const float drop = __uint_as_float(__ldcg(w + OZ_W_DROP)) * r.drop_scale;
-  if (__ldcg(w + OZ_W_NONFINITE)) return 0;
+  if (__ldcg(w + OZ_W_NONFINITE) || (__ldcg(w + OZ_W_HOLE) && __ldcg(w + OZ_W_TINY))) return 0;
   const int e = (int)__ldcg(w + OZ_W_EXP_A) + (int)__ldcg(w + OZ_W_EXP_B) - 2 * kExpBias;
   if (e > r.exp_limit) return 0;
   int S = (r.target_bits + r.digit_bits - 1) / r.digit_bits;
@@ -796,9 +809,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     // Same TMEM geometry as below. Units of a tile: pass 1: (0,0) = D;
     // pass 2: (0,1), (1,0) summed in fp32 into columns 256..511 = N, then
     // (0,0) = D. Per element r = numerator / D (pass 1: numerator =
-    // (ra_i + cb_j) 2^96, the operands' 2^48 scale factors); D = 0 gives
-    // +inf unless the numerator is 0 too (every product then has a zero
-    // factor and the result is exact). The running max is float bits.
+    // (ra_i + cb_j) 2^96, the operands' 2^48 scale factors). D = 0 with a
+    // nonzero numerator: pass 1 notes a hole; in pass 2 a product was lost,
+    // which gives +inf. The running max is float bits.
     __shared__ float est_cb[EST ? 8 : 1][EST ? OZ_BN / 2 : 1];
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
@@ -809,6 +822,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint32_t ai = 0;
     const float inf = __uint_as_float(0x7f800000u);
     float rmax = 0.0f, dmin = inf;
+    bool hole = false;
     bool ok = true;
     for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
       const TileCtx tc = tile_ctx<EST, G>(P, S, tile, rank);
@@ -857,10 +871,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             else num = __uint_as_float(w[e]);
             // (the threshold test of the count tolerates the approximate
             // division's two ulp)
-            r = D > 0.0f ? __fdividef(num, D) : num > 0.0f ? inf : 0.0f;
+            r = D > 0.0f ? __fdividef(num, D) : num > 0.0f && !pass1 ? inf : 0.0f;
             if (row_ok && col < tc.n) {
               rmax = fmaxf(rmax, r);
               if (D > 0.0f) dmin = fminf(dmin, D);
+              else hole |= num > 0.0f;
             }
           }
         }
@@ -874,7 +889,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
       dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, off));
     }
+    hole = __any_sync(0xffffffffu, hole);
     if (lane == 0 && ok) {
+      if (hole) raise_word(P.est + OZ_W_HOLE, 1);
       atomicMax(P.est + OZ_W_SPREAD, __float_as_uint(rmax));
       if (dmin < inf) atomicMax(P.est + OZ_W_DROP, __float_as_uint(0x1p96f / dmin));
     }
@@ -1400,12 +1417,16 @@ constexpr uint32_t kBf16Two48 = 0x5780u;  // 2^48 in BF16
 // |x| 2^-e from the bit pattern alone (no FP64 arithmetic: GB300's FP64 pipe
 // is slow): *f = |x'| as fp32 (mantissa truncated), return value = |x'| 2^48
 // as BF16 (round to nearest even). Subnormal x and values below the formats'
-// normal ranges give 0 (the estimate then only grows).
-__device__ __forceinline__ uint32_t est_bits(double x, int e, float* f) {
+// normal ranges give 0 (the estimate then only grows). `tiny`: x is not 0 and
+// 0 here or below 2^-110 (two entries from there on have a product of 2^-124,
+// scaled, which fp32 holds).
+constexpr int kTinyExp = -110;
+__device__ __forceinline__ uint32_t est_bits(double x, int e, float* f, bool& tiny) {
   const uint64_t u = (uint64_t)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL;
   const int be = (int)(u >> 52);
   const uint64_t mant = u & 0xFFFFFFFFFFFFFULL;
   const int fe = be - 1023 - e;  // unbiased exponent of |x'| (<= -1)
+  tiny |= u != 0 && (be == 0 || fe < kTinyExp);
   if (be == 0) {
     *f = 0.0f;
     return 0u;
@@ -1417,11 +1438,12 @@ __device__ __forceinline__ uint32_t est_bits(double x, int e, float* f) {
   if (rem > half || (rem == half && (h & 1u))) ++h;
   return h;
 }
-__device__ __forceinline__ uint32_t est_bits(float x, int e, float* f) {
+__device__ __forceinline__ uint32_t est_bits(float x, int e, float* f, bool& tiny) {
   const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
   const int be = (int)(u >> 23);
   const uint32_t mant = u & 0x7FFFFFu;
   const int fe = be - 127 - e;
+  tiny |= u != 0 && (be == 0 || fe < kTinyExp);
   if (be == 0) {
     *f = 0.0f;
     return 0u;
@@ -1438,10 +1460,6 @@ __device__ __forceinline__ uint32_t two48_if(double x) {
   return ((uint64_t)__double_as_longlong(x) << 1) != 0 ? kBf16Two48 : 0u;
 }
 __device__ __forceinline__ uint32_t two48_if(float x) { return x != 0.0f ? kBf16Two48 : 0u; }
-// Raises a word to at least v; most callers find it there already.
-__device__ __forceinline__ void raise_word(uint32_t* w, uint32_t v) {
-  if (__ldcg(w) < v) atomicMax(w, v);
-}
 
 // Both operands' estimate slices, sums and exponent maxima. `kside`: the
 // decision word of the operand's exponent maximum.
@@ -1464,6 +1482,7 @@ __global__ void __launch_bounds__(256)
     const int er = o.e[row];
     const T* xr = o.p + row * o.ld;
     float s = 0.0f;
+    bool tiny = false;
     for (int64_t j0 = (int64_t)tx * 8; j0 < kpad; j0 += 256) {
       T x[8];
       load_run(xr + j0, o.vec, k - j0, x);
@@ -1471,7 +1490,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         float f0, f1;
-        const uint32_t b0 = est_bits(x[2 * h], er, &f0), b1 = est_bits(x[2 * h + 1], er, &f1);
+        const uint32_t b0 = est_bits(x[2 * h], er, &f0, tiny), b1 = est_bits(x[2 * h + 1], er, &f1, tiny);
         s += f0;
         s += f1;
         pa[h] = b0 | (b1 << 16);
@@ -1482,7 +1501,9 @@ __global__ void __launch_bounds__(256)
       if (PASS2) *reinterpret_cast<uint4*>(q + o.rows * kpad) = make_uint4(pi[0], pi[1], pi[2], pi[3]);
     }
     for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    tiny = __any_sync(0xffffffffu, tiny);
     if (tx == 0) {
+      if (tiny) raise_word(&words[OZ_W_TINY], 1);
       o.sums[row] = __float2uint_ru(s * scale);
       raise_word(&words[word], (uint32_t)(er + kExpBias));
       if (er == kNonFinite<T>) words[OZ_W_NONFINITE] = 1;
@@ -1503,17 +1524,20 @@ __global__ void __launch_bounds__(256)
   }
   const int ec = block_col_exps(o, n0, ky == 0, cexp);
   float s = 0.0f;
+  bool tiny = false;
 #pragma unroll
   for (int r = 0; r < kSliceColK / 16; ++r) {
     const int w = ty + 8 * r;
     float f0, f1;
-    const uint32_t b0 = est_bits(x0[r], ec, &f0), b1 = est_bits(x1[r], ec, &f1);
+    const uint32_t b0 = est_bits(x0[r], ec, &f0, tiny), b1 = est_bits(x1[r], ec, &f1, tiny);
     s += f0;
     s += f1;
     tile[0][tx][w] = b0 | (b1 << 16);
     if (PASS2) tile[PASS2 ? 1 : 0][tx][w] = two48_if(x0[r]) | (two48_if(x1[r]) << 16);
   }
   csum[ty][tx] = s;
+  tiny = __any_sync(0xffffffffu, tiny);
+  if (tiny && tx == 0) raise_word(&words[OZ_W_TINY], 1);
   __syncthreads();
   if (ty == 0 && nn < o.rows) {
     float t = 0.0f;
@@ -1962,8 +1986,8 @@ int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, bool
            : launch_estimate<double>(h, a, bT, m, n, k, kpad, pass, w);
   if (st) return st;
   cudaStream_t s = h->stream;
-  uint32_t host[3] = {0, 0, 0};
-  static_assert(OZ_W_SPREAD == 0 && OZ_W_NONFINITE == 1 && OZ_W_DROP == 2, "the words read back");
+  uint32_t host[4] = {0, 0, 0, 0};
+  static_assert(OZ_W_SPREAD == 0 && OZ_W_NONFINITE == 1 && OZ_W_DROP == 2 && OZ_W_HOLE == 3, "the words read back");
   if ((st = nrs_cuda_check(h, cudaMemcpyAsync(host, w.words, sizeof(host), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync")))
     return st;
   if ((st = nrs_cuda_check(h, cudaStreamSynchronize(s), "cudaStreamSynchronize"))) return st;
@@ -1972,6 +1996,7 @@ int spread_estimate(nrs_handle* h, const OzOperand& a, const OzOperand& bT, bool
     return st;
   if (derr) return nrs_fail(h, NRS_ERR_TIMEOUT, "ozaki spread estimate: a device-side bounded wait gave up");
   std::memcpy(&res->rmax, &host[OZ_W_SPREAD], 4);
+  if (pass == 1 && host[OZ_W_HOLE]) res->rmax = HUGE_VALF;  // pass 2 counts only the k of nonzero products
   std::memcpy(&res->dinv, &host[OZ_W_DROP], 4);
   res->flags = host[OZ_W_NONFINITE];
   return NRS_OK;
