@@ -273,8 +273,8 @@ struct OzRule {
 // OZ_W_TINY: an operand holds a nonzero entry so small (est_bits) that its
 // products with another can be lost in |A'||B'|.
 enum {
-  OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_DROP = 2, OZ_W_HOLE = 3, OZ_W_EXP_A = 4, OZ_W_EXP_B = 5, OZ_W_COUNT = 6,
-  OZ_W_TINY = 7, OZ_WORDS = 8
+  OZ_W_SPREAD = 0, OZ_W_NONFINITE = 1, OZ_W_DROP = 2, OZ_W_HOLE = 3, OZ_W_EXP_A = 4, OZ_W_EXP_B = 5, OZ_W_TINY = 6,
+  OZ_W_COUNT = 8, OZ_WORDS = 9
 };
 // Raises a word to at least v; most callers find it there already.
 __device__ __forceinline__ void raise_word(uint32_t* w, uint32_t v) {
@@ -290,10 +290,13 @@ constexpr int kExpBias = 4096;  // exponents are collected biased, as unsigned m
 // one-hot operands) every product of the sum has a zero factor, whose digits are
 // zeros: C_ij is exact at any count. Only tiny entries make that uncertain.
 __device__ __forceinline__ int oz_decide(const uint32_t* w, const OzRule& r) {
-  const float spread = __uint_as_float(__ldcg(w + OZ_W_SPREAD));
-  const float drop = __uint_as_float(__ldcg(w + OZ_W_DROP)) * r.drop_scale;
-  if (__ldcg(w + OZ_W_NONFINITE) || (__ldcg(w + OZ_W_HOLE) && __ldcg(w + OZ_W_TINY))) return 0;
-  const int e = (int)__ldcg(w + OZ_W_EXP_A) + (int)__ldcg(w + OZ_W_EXP_B) - 2 * kExpBias;
+  // (two loads in flight together: every block of oz_slice starts with them, and
+  // one load after another cost 13 us at 4096^3)
+  const uint4 lo = __ldcg(reinterpret_cast<const uint4*>(w)), hi = __ldcg(reinterpret_cast<const uint4*>(w) + 1);
+  static_assert(OZ_W_HOLE == 3 && OZ_W_EXP_A == 4 && OZ_W_EXP_B == 5 && OZ_W_TINY == 6, "the words' places");
+  const float spread = __uint_as_float(lo.x), drop = __uint_as_float(lo.z) * r.drop_scale;
+  if (lo.y | (lo.w & hi.z)) return 0;  // (both 0 or 1)
+  const int e = (int)hi.x + (int)hi.y - 2 * kExpBias;
   if (e > r.exp_limit) return 0;
   int S = (r.target_bits + r.digit_bits - 1) / r.digit_bits;
   for (; S <= r.max_slices; ++S)
@@ -821,6 +824,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const uint32_t dsum_t = lane_base + OZ_BN;
     uint32_t ai = 0;
     const float inf = __uint_as_float(0x7f800000u);
+    // (the numerators' scale, in the sums already: 2^31 2^96 2^-16 at most)
+    const float unit = 0x1p96f * P.sum_unit;
     float rmax = 0.0f, dmin = inf;
     bool hole = false;
     bool ok = true;
@@ -829,14 +834,17 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       const int64_t row = tc.row0 + row_in_tile;
       const bool row_ok = row < tc.m;
       const int64_t col0 = tc.col0 + half * (OZ_BN / 2);
-      const float ra = row_ok ? (float)P.ra[row] : 0.0f;
+      // Rows and columns outside the problem have D = 0 (the loads fill with
+      // zeros) and here a numerator of -inf: no ratio and no hole. Pass 2's is
+      // 0 there.
+      const float ra = row_ok ? (float)P.ra[row] * unit : -inf;
       const bool pass1 = P.slices == 1;
       // this warp's column sums, read while the product runs
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < OZ_BN / 2; j += 32) {
         const int64_t col = col0 + j + lane;
-        est_cb[warp - 2][j + lane] = pass1 && col < tc.n ? (float)P.cb[col] : 0.0f;
+        est_cb[warp - 2][j + lane] = pass1 && col < tc.n ? (float)P.cb[col] * unit : -inf;
       }
       __syncwarp();
       PairIter pr;
@@ -864,19 +872,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           }
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const int64_t col = col0 + c * 16 + e;
+            // (straight-line: with a mask and a branch per element 1024^3 took
+            // 12 us more)
             const float D = __uint_as_float(v[e]);
-            float num, r;
-            if (pass1) num = (ra + est_cb[warp - 2][c * 16 + e]) * (0x1p96f * P.sum_unit);
-            else num = __uint_as_float(w[e]);
+            const float num = pass1 ? ra + est_cb[warp - 2][c * 16 + e] : __uint_as_float(w[e]);
+            const bool some = D > 0.0f;
             // (the threshold test of the count tolerates the approximate
             // division's two ulp)
-            r = D > 0.0f ? __fdividef(num, D) : num > 0.0f && !pass1 ? inf : 0.0f;
-            if (row_ok && col < tc.n) {
-              rmax = fmaxf(rmax, r);
-              if (D > 0.0f) dmin = fminf(dmin, D);
-              else hole |= num > 0.0f;
-            }
+            rmax = fmaxf(rmax, some ? __fdividef(num, D) : 0.0f);
+            dmin = fminf(dmin, some ? D : inf);
+            hole |= !some & (num > 0.0f);
           }
         }
         tmem_wait_st();
@@ -891,7 +896,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
     hole = __any_sync(0xffffffffu, hole);
     if (lane == 0 && ok) {
-      if (hole) raise_word(P.est + OZ_W_HOLE, 1);
+      if (hole && P.slices == 1) raise_word(P.est + OZ_W_HOLE, 1);
+      if (hole && P.slices != 1) rmax = inf;
       atomicMax(P.est + OZ_W_SPREAD, __float_as_uint(rmax));
       if (dmin < inf) atomicMax(P.est + OZ_W_DROP, __float_as_uint(0x1p96f / dmin));
     }
@@ -1421,12 +1427,25 @@ constexpr uint32_t kBf16Two48 = 0x5780u;  // 2^48 in BF16
 // 0 here or below 2^-110 (two entries from there on have a product of 2^-124,
 // scaled, which fp32 holds).
 constexpr int kTinyExp = -110;
-__device__ __forceinline__ uint32_t est_bits(double x, int e, float* f, bool& tiny) {
+// With e's limit, tiny is one comparison of |x|'s bits.
+template <typename T>
+struct TinyLimit;
+template <>
+struct TinyLimit<double> {
+  uint64_t v;
+  __device__ __forceinline__ explicit TinyLimit(int e) : v(((uint64_t)max(1, 1023 + e + kTinyExp) << 52) - 1) {}
+};
+template <>
+struct TinyLimit<float> {
+  uint32_t v;
+  __device__ __forceinline__ explicit TinyLimit(int e) : v(((uint32_t)max(1, 127 + e + kTinyExp) << 23) - 1) {}
+};
+__device__ __forceinline__ uint32_t est_bits(double x, int e, TinyLimit<double> lim, float* f, bool& tiny) {
   const uint64_t u = (uint64_t)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL;
   const int be = (int)(u >> 52);
   const uint64_t mant = u & 0xFFFFFFFFFFFFFULL;
   const int fe = be - 1023 - e;  // unbiased exponent of |x'| (<= -1)
-  tiny |= u != 0 && (be == 0 || fe < kTinyExp);
+  tiny |= u - 1 < lim.v;
   if (be == 0) {
     *f = 0.0f;
     return 0u;
@@ -1438,12 +1457,12 @@ __device__ __forceinline__ uint32_t est_bits(double x, int e, float* f, bool& ti
   if (rem > half || (rem == half && (h & 1u))) ++h;
   return h;
 }
-__device__ __forceinline__ uint32_t est_bits(float x, int e, float* f, bool& tiny) {
+__device__ __forceinline__ uint32_t est_bits(float x, int e, TinyLimit<float> lim, float* f, bool& tiny) {
   const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
   const int be = (int)(u >> 23);
   const uint32_t mant = u & 0x7FFFFFu;
   const int fe = be - 127 - e;
-  tiny |= u != 0 && (be == 0 || fe < kTinyExp);
+  tiny |= u - 1 < lim.v;
   if (be == 0) {
     *f = 0.0f;
     return 0u;
@@ -1483,6 +1502,7 @@ __global__ void __launch_bounds__(256)
     const T* xr = o.p + row * o.ld;
     float s = 0.0f;
     bool tiny = false;
+    const TinyLimit<T> lim(er);
     for (int64_t j0 = (int64_t)tx * 8; j0 < kpad; j0 += 256) {
       T x[8];
       load_run(xr + j0, o.vec, k - j0, x);
@@ -1490,7 +1510,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         float f0, f1;
-        const uint32_t b0 = est_bits(x[2 * h], er, &f0, tiny), b1 = est_bits(x[2 * h + 1], er, &f1, tiny);
+        const uint32_t b0 = est_bits(x[2 * h], er, lim, &f0, tiny), b1 = est_bits(x[2 * h + 1], er, lim, &f1, tiny);
         s += f0;
         s += f1;
         pa[h] = b0 | (b1 << 16);
@@ -1525,11 +1545,12 @@ __global__ void __launch_bounds__(256)
   const int ec = block_col_exps(o, n0, ky == 0, cexp);
   float s = 0.0f;
   bool tiny = false;
+  const TinyLimit<T> lim(ec);
 #pragma unroll
   for (int r = 0; r < kSliceColK / 16; ++r) {
     const int w = ty + 8 * r;
     float f0, f1;
-    const uint32_t b0 = est_bits(x0[r], ec, &f0, tiny), b1 = est_bits(x1[r], ec, &f1, tiny);
+    const uint32_t b0 = est_bits(x0[r], ec, lim, &f0, tiny), b1 = est_bits(x1[r], ec, lim, &f1, tiny);
     s += f0;
     s += f1;
     tile[0][tx][w] = b0 | (b1 << 16);
