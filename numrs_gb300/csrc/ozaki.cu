@@ -2400,6 +2400,14 @@ int nrs_tc_gemm_auto(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, 
     return NRS_ERR_UNSUPPORTED;
   }
   if (cap != cudaStreamCaptureStatusNone) return NRS_ERR_UNSUPPORTED;
+  // A workspace cannot grow during a capture: a call outside one leaves the
+  // room that the FP64 kernel's K ranges take when the same call is captured
+  // (no room: only that capture is refused).
+  const int splits = dtype == NRS_F64 ? nrs_dmma_splits(m, k, n) : 1;
+  if (splits > 1) {
+    int st;
+    if (!nrs_workspace(h, (size_t)splits * (size_t)(m * n) * sizeof(double), &st)) h->last_error.clear();
+  }
   const OzOperand a{A, lda, m, !ta};
   const OzOperand bT{B, ldb, n, tb};
   return dtype == NRS_F32 ? tc_gemm<float>(h, a, bT, m, k, n, C, ldc, accumulate)

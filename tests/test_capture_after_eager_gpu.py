@@ -1,0 +1,50 @@
+"""A call that has run once outside a stream capture can be captured: what it
+needs of the handle's workspace, which cannot grow during a capture, is there.
+Each test has a handle of its own, so that no other call has made the room.
+"""
+import ctypes as C
+
+import pytest
+import torch
+
+from numrs_gb300 import _lib as L
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def call(K):
+    lib, h = L.load(), C.c_void_p()
+    L.check(lib.nrs_create(0, C.byref(h)))
+
+    def f(name, *args):
+        lib.nrs_set_stream(h, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        L.check(getattr(lib, name)(h, *args), h)
+    yield f
+    torch.cuda.synchronize()
+    lib.nrs_destroy(h)
+
+
+def _p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("n", [512, 1000, 1024])
+def test_f64_product(K, call, n):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a, b = (torch.rand((n, n), dtype=torch.float64, device="cuda", generator=g) - 0.5 for _ in range(2))
+    c = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+
+    def product():
+        call("nrs_gemm", L.F64, n, n, n, _p(a), n, _p(b), n, _p(c), n, 0, L.GEMM_AUTO)
+    product()
+    torch.cuda.synchronize()
+    assert not torch.equal(c, K.matmul(a, b, variant=L.GEMM_DMMA))  # (the slices ran)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        product()
+    a.mul_(-3.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(c, K.matmul(a, b, variant=L.GEMM_DMMA))
