@@ -124,6 +124,12 @@ extern "C" int nrs_create(int device, nrs_handle** out) {
     if (h->pool) cudaMemPoolDestroy(h->pool);
     h->pool = nullptr;
   }
+  // The workspace's smallest size from the start: a short flat reduction runs
+  // without it, and a longer one that is captured next could not get it then.
+  // (No room now: the first call that needs it asks again.)
+  int ws = NRS_OK;
+  nrs_workspace(h, 1, &ws);
+  h->last_error.clear();
   h->hw_sms = h->num_sms;
   h->stream = h->own_stream;
   *out = h;

@@ -48,3 +48,22 @@ def test_f64_product(K, call, n):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(c, K.matmul(a, b, variant=L.GEMM_DMMA))
+
+
+def test_flat_reduction_after_a_short_one(K, call):
+    """(300,000 elements: 37 chunk partials; 1000 run in one launch without any)"""
+    x = torch.randn(300_000, dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+
+    def total(n):
+        call("nrs_reduce", L.F64, L.SUM, 1, L.i64_array([n]), L.i64_array([1]), L.AXIS_NONE, 0, _p(x), _p(out))
+    total(1000)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        total(300_000)
+    x.mul_(2.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, K.sum(x))
