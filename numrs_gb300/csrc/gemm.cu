@@ -130,12 +130,37 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), (BM * BN >= 128 * 128 ?
   tile_store<T>(t, C, ldc, m, n, m0, n0, accumulate != 0);
 }
 
-// A 64 x 64 tile with K split over a cluster of gridDim.z CTAs: CTA z
-// takes k-values [z*kc, min(k, (z+1)*kc)) and leaves its product in shared
-// memory; then every CTA adds a share of the tile's elements over the ranks
-// in order (through distributed shared memory) and writes them. One launch
-// and no scratch, so it needs no workspace shared between streams and runs
-// under capture.
+// K split over a cluster of `splits` CTAs: CTA `rank` takes k-values
+// [rank*kc, min(k, (rank+1)*kc)) and leaves its product in shared memory; then
+// every CTA adds a share of the tile's elements over the ranks in order
+// (through distributed shared memory) and writes them. One launch and no
+// scratch, so it needs no workspace shared between streams and runs under
+// capture.
+template <typename T, int BM, int NT, typename Tile>
+__device__ __forceinline__ void cluster_sum_store(const Tile& t, T* part, int rank, int splits, T* C, int64_t ldc,
+                                                  int64_t m, int64_t n, int64_t m0, int64_t n0, bool accumulate) {
+#pragma unroll
+  for (int e = 0; e < Tile::kPerThread; ++e) {
+    int r, c;
+    t.coords(e, r, c);
+    part[r * BM + c] = t.value(e);
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  const int share = BM * BM / splits;
+  for (int i = threadIdx.x; i < share; i += NT) {
+    const int idx = rank * share + i;
+    const int64_t gi = m0 + idx / BM, gj = n0 + idx % BM;
+    if (gi >= m || gj >= n) continue;
+    T v = cluster.map_shared_rank(part, 0)[idx];
+    for (int z = 1; z < splits; ++z) v = tile_add(v, cluster.map_shared_rank(part, z)[idx]);
+    T* c = C + gi * ldc + gj;
+    *c = accumulate ? tile_add(*c, v) : v;
+  }
+  cluster.sync();  // a CTA's shared memory outlives its readers
+}
+
+// A 64 x 64 tile with K split over a cluster of gridDim.z CTAs.
 constexpr int kSplitTile = 64;
 template <typename T>
 using SplitTile = Simt<T, kSplitTile, kSplitTile, 16, 4, 4>;
@@ -160,26 +185,9 @@ __global__ void __launch_bounds__(kSplitThreads, sizeof(T) == 4 ? 3 : 2)
     tile_store<T>(t, C, ldc, m, n, m0, n0, accumulate != 0);
     return;
   }
-  T* part = reinterpret_cast<T*>(smem);  // (run() ends with a barrier)
-#pragma unroll
-  for (int e = 0; e < Tile::kPerThread; ++e) {
-    int r, c;
-    t.coords(e, r, c);
-    part[r * kSplitTile + c] = t.value(e);
-  }
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  const int share = kSplitTile * kSplitTile / splits;
-  for (int i = threadIdx.x; i < share; i += kSplitThreads) {
-    const int idx = (int)blockIdx.z * share + i;
-    const int64_t gi = m0 + idx / kSplitTile, gj = n0 + idx % kSplitTile;
-    if (gi >= m || gj >= n) continue;
-    T v = cluster.map_shared_rank(part, 0)[idx];
-    for (int z = 1; z < splits; ++z) v = tile_add(v, cluster.map_shared_rank(part, z)[idx]);
-    T* c = C + gi * ldc + gj;
-    *c = accumulate ? tile_add(*c, v) : v;
-  }
-  cluster.sync();  // a CTA's shared memory outlives its readers
+  // (run() ends with a barrier)
+  cluster_sum_store<T, kSplitTile, kSplitThreads>(t, reinterpret_cast<T*>(smem), (int)blockIdx.z, splits, C, ldc, m, n,
+                                                  m0, n0, accumulate != 0);
 }
 
 // Generic GEMM: one thread per C element, k ascending, one rounding per op.
@@ -224,12 +232,16 @@ struct BatchDims {
   int n;
   int64_t size[kMaxBatchDims], a[kMaxBatchDims], b[kMaxBatchDims];
 };
-template <typename T, typename Tile, int BM, int BN, int NT>
+// SPLIT: K over clusters of `splits` CTAs along x (few panels with long sums:
+// 2 x (64 x 4096 x 64) f64 1239 -> 159 us, which one CTA per tile adds 256
+// k tiles for).
+template <typename T, typename Tile, int BM, int NT, bool SPLIT>
 __global__ void __launch_bounds__(NT)
-    batched_gemm(const __grid_constant__ BatchDims g, int64_t z0, int64_t m, int64_t n, int64_t k,
-                 const T* __restrict__ A, int64_t rsa, int64_t csa, const T* __restrict__ B, int64_t rsb, int64_t csb,
-                 T* __restrict__ C) {
-  __shared__ __align__(16) uint8_t smem[Tile::kSmem];
+    batched_gemm(const __grid_constant__ BatchDims g, int64_t z0, int64_t m, int64_t n, int64_t k, int splits,
+                 int64_t kc, const T* __restrict__ A, int64_t rsa, int64_t csa, const T* __restrict__ B, int64_t rsb,
+                 int64_t csb, T* __restrict__ C) {
+  constexpr int kPart = SPLIT ? BM * BM * (int)sizeof(T) : 0;  // the partial tile reuses the operand buffers
+  __shared__ __align__(16) uint8_t smem[Tile::kSmem > kPart ? Tile::kSmem : kPart];
   const int64_t z = z0 + blockIdx.z;
   int64_t rem = z, ao = 0, bo = 0;
   for (int d = g.n - 1; d >= 0; --d) {
@@ -239,9 +251,15 @@ __global__ void __launch_bounds__(NT)
     bo += c * g.b[d];
   }
   Tile t;
-  const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-  t.run(A + ao, rsa, csa, B + bo, rsb, csb, m, n, m0, n0, 0, k, smem);
-  tile_store<T>(t, C + z * m * n, n, m, n, m0, n0, false);
+  const int rank = SPLIT ? (int)(blockIdx.x % (unsigned)splits) : 0;
+  const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)(SPLIT ? blockIdx.x / (unsigned)splits : blockIdx.x) * BM;
+  const int64_t k0 = rank * kc, k1 = SPLIT && k0 + kc < k ? k0 + kc : k;
+  t.run(A + ao, rsa, csa, B + bo, rsb, csb, m, n, m0, n0, k0, k1, smem);
+  T* const Cz = C + z * m * n;
+  if constexpr (SPLIT)
+    cluster_sum_store<T, BM, NT>(t, reinterpret_cast<T*>(smem), rank, splits, Cz, n, m, n, m0, n0, false);
+  else
+    tile_store<T>(t, Cz, n, m, n, m0, n0, false);
 }
 
 template <typename T>
@@ -501,21 +519,52 @@ extern "C" int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t 
 
 namespace {
 
-// 64 x 64 tiles (weight 4) or 32 x 32: the one whose busiest SM has less to do.
-bool large_tiles(int64_t m, int64_t n, int64_t batch) {
-  const double t64 = (double)((m + 63) / 64) * (double)((n + 63) / 64) * (double)batch;
-  const double t32 = (double)((m + 31) / 32) * (double)((n + 31) / 32) * (double)batch;
-  return std::ceil(t64 / NRS_PLAN_SMS) * 4.0 <= std::ceil(t32 / NRS_PLAN_SMS);
+// 64 x 64 tiles (weight 4) or 32 x 32, and K in ranges of at least 64 values
+// over clusters of up to 8 CTAs while the batch does not fill the GPU: the form
+// whose busiest SM has less to do (a split costs about 32 k-values of a tile).
+struct BatchPlan {
+  bool large;
+  int splits;
+  int64_t kc;
+};
+BatchPlan plan_batched(int64_t m, int64_t n, int64_t k, int64_t batch) {
+  BatchPlan best{true, 1, k};
+  double least = 1e300;
+  for (int tile : {64, 32}) {
+    const double ctas = (double)((m + tile - 1) / tile) * (double)((n + tile - 1) / tile) * (double)batch;
+    for (int z = 1; z <= 8; z *= 2) {
+      const int64_t kc = z > 1 ? ((k + z - 1) / z + 15) / 16 * 16 : k;
+      if (z > 1 && (kc < 64 || (k + kc - 1) / kc != z || ctas * z >= 2.0 * NRS_PLAN_SMS)) break;
+      const double cost = std::ceil(ctas * z / NRS_PLAN_SMS) * (tile == 64 ? 4.0 : 1.0) * ((double)kc + (z > 1 ? 32.0 : 0.0));
+      if (cost < least) {
+        least = cost;
+        best = BatchPlan{tile == 64, z, kc};
+      }
+    }
+  }
+  return best;
 }
 
-template <typename T, typename Tile, int BM, int BN, int NT>
-void launch_batched(nrs_handle* h, const BatchDims& g, int64_t batch, int64_t m, int64_t k, int64_t n, const void* A,
-                    int64_t rsa, int64_t csa, const void* B, int64_t rsb, int64_t csb, void* C) {
+template <typename T, typename Tile, int BM, int NT>
+void launch_batched(nrs_handle* h, const BatchDims& g, const BatchPlan& pl, int64_t batch, int64_t m, int64_t k,
+                    int64_t n, const void* A, int64_t rsa, int64_t csa, const void* B, int64_t rsb, int64_t csb,
+                    void* C) {
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(NT);
+  cfg.stream = h->stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)pl.splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pl.splits > 1 ? 1 : 0;
+  auto kern = pl.splits > 1 ? batched_gemm<T, Tile, BM, NT, true> : batched_gemm<T, Tile, BM, NT, false>;
   for (int64_t z0 = 0; z0 < batch; z0 += 65535) {
-    dim3 grid = tiles(m, n, BM, BN);
-    grid.z = (unsigned)(batch - z0 < 65535 ? batch - z0 : 65535);
-    batched_gemm<T, Tile, BM, BN, NT><<<grid, NT, 0, h->stream>>>(g, z0, m, n, k, (const T*)A, rsa, csa, (const T*)B,
-                                                                  rsb, csb, (T*)C);
+    cfg.gridDim = tiles(m, n, BM, BM);
+    cfg.gridDim.x *= (unsigned)pl.splits;
+    cfg.gridDim.z = (unsigned)(batch - z0 < 65535 ? batch - z0 : 65535);
+    cudaLaunchKernelEx(&cfg, kern, g, z0, m, n, k, pl.splits, pl.kc, (const T*)A, rsa, csa, (const T*)B, rsb, csb,
+                       (T*)C);
   }
 }
 
@@ -573,12 +622,12 @@ extern "C" int nrs_gemm_batched(nrs_handle* h, int dtype, int batch_ndim, const 
   }
   const int64_t rsa = ta ? 1 : lda, csa = ta ? lda : 1;
   const int64_t rsb = tb ? 1 : ldb, csb = tb ? ldb : 1;
-  const bool big = large_tiles(m, n, batch);
+  const BatchPlan pl = plan_batched(m, n, k, batch);
   // One launch over (tiles, panels); a 32 x 96 x 80 x 112 f64 batch: 1.45 ms
   // as a plan built per call from one descriptor per panel, 0.07 ms here (the FP64
   // pipe takes 0.06 for the padded tiles).
 #define NRS_BATCH(T, TILE, BM, NT) \
-  launch_batched<T, TILE, BM, BM, NT>(h, g, batch, m, k, n, A, rsa, csa, B, rsb, csb, C)
+  launch_batched<T, TILE, BM, NT>(h, g, pl, batch, m, k, n, A, rsa, csa, B, rsb, csb, C)
   using F32L = Simt<float, 64, 64, 16, 4, 4>;
   using F32S = Simt<float, 32, 32, 16, 2, 2>;
   using F64L = Dmma<64, 64, 2, 4>;
@@ -588,10 +637,10 @@ extern "C" int nrs_gemm_batched(nrs_handle* h, int dtype, int batch_ndim, const 
   using I32L = Simt<int32_t, 64, 64, 16, 4, 4>;
   using I32S = Simt<int32_t, 32, 32, 16, 2, 2>;
   switch (dtype) {
-    case NRS_F32: big ? NRS_BATCH(float, F32L, 64, 256) : NRS_BATCH(float, F32S, 32, 256); break;
-    case NRS_F64: big ? NRS_BATCH(double, F64L, 64, 256) : NRS_BATCH(double, F64S, 32, 128); break;
-    case NRS_I64: big ? NRS_BATCH(int64_t, I64L, 64, 256) : NRS_BATCH(int64_t, I64S, 32, 256); break;
-    default: big ? NRS_BATCH(int32_t, I32L, 64, 256) : NRS_BATCH(int32_t, I32S, 32, 256); break;
+    case NRS_F32: pl.large ? NRS_BATCH(float, F32L, 64, 256) : NRS_BATCH(float, F32S, 32, 256); break;
+    case NRS_F64: pl.large ? NRS_BATCH(double, F64L, 64, 256) : NRS_BATCH(double, F64S, 32, 128); break;
+    case NRS_I64: pl.large ? NRS_BATCH(int64_t, I64L, 64, 256) : NRS_BATCH(int64_t, I64S, 32, 256); break;
+    default: pl.large ? NRS_BATCH(int32_t, I32L, 64, 256) : NRS_BATCH(int32_t, I32S, 32, 256); break;
   }
 #undef NRS_BATCH
   return nrs_after_launch(h, "batched_gemm");
