@@ -15,6 +15,7 @@
 // Overwrite contract: C is written, never read, unless ACCUMULATE is set, in
 // which case C += (A*B) with the product rounded first (matmul_to computes a
 // temporary and adds it, src/array/operations_optimized.rs:385).
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -368,6 +369,21 @@ void launch_auto_f32(nrs_handle* h, int64_t m, int64_t k, int64_t n, const float
     launch_simt_split(h, pl, m, k, n, A, rsa, csa, B, rsb, csb, C, ldc, acc, unless);
 }
 
+// i64 products of row-major operands, modelled (us). One thread per element:
+// 1.98 products per ns and 0.33 elements per ns, or 0.17 us per k of one
+// thread's chain; 64 x 64 tiles 0.17 us per k and wave, K padded to 16.
+// Measured (us, one thread per element / tiles): 64 x 20000 x 64 3313 / 479,
+// 512^3 92 / 55, 8000 x 16 x 8000 714 / 381, 20000 x 100 x 100 106 / 100.
+double generic_i64_us(int64_t m, int64_t n, int64_t k) {
+  const double mn = (double)m * (double)n;
+  return 4.0 + std::max(mn * (double)k / 1.98e6 + mn / 3.3e5, 0.17 * (double)k);
+}
+double tiled_i64_us(int64_t m, int64_t n, int64_t k) {
+  const F32Plan pl = plan_split(m, n, k);
+  const double ctas = (double)((m + 63) / 64) * (double)((n + 63) / 64) * pl.splits;
+  return 4.0 + std::ceil(ctas / NRS_PLAN_SMS) * (double)((pl.kc + 15) / 16 * 16) * 0.17;
+}
+
 bool grid_too_large(int64_t m, int64_t n) { return (n + 31) / 32 > 0x7fffffffLL || (m + 31) / 32 > 65535; }
 
 }  // namespace
@@ -410,7 +426,11 @@ int nrs_plain_gemm_launch(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_
   // Integers from a 32 x 32 C on: tiles read each operand element once per 64
   // products, one thread per element reads two per product; a split K fills
   // the GPU (i64, us, one thread per element / tiles: 1000^3 657 / 308,
-  // 300 x 1000 x 257 174 / 57).
+  // 300 x 1000 x 257 174 / 57). For i64 the padding of narrow and of shallow
+  // products can cost more than that (2^20 x 64 x 16 542 / 1189,
+  // 4096 x 1 x 4096 64 / 99).
+  if (variant == NRS_GEMM_AUTO && dtype == NRS_I64 && csa == 1 && csb == 1 && generic_i64_us(m, n, k) < tiled_i64_us(m, n, k))
+    variant = NRS_GEMM_GENERIC;
   if (variant == NRS_GEMM_AUTO && dtype == NRS_I64) {
     launch_simt_split(h, plan_split(m, n, k), m, k, n, (const int64_t*)A, rsa, csa, (const int64_t*)B, rsb, csb,
                       (int64_t*)C, ldc, acc, nullptr);
