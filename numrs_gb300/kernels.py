@@ -302,8 +302,8 @@ def save_npy(path: str, t: torch.Tensor) -> None:
 def _mat_strides(t: torch.Tensor):
     """(leading dim, transposed?) for the last two axes, or None if neither
     row- nor column-contiguous."""
-    r, c = t.stride()[-2:]
-    rows, cols = t.shape[-2:]
+    st, sh = t.stride(), t.shape  # (slices of a torch.Size cost half a call's time here)
+    r, c, rows, cols = st[-2], st[-1], sh[-2], sh[-1]
     if c == 1 or cols <= 1:
         return (r if rows > 1 else _bi.max(cols, 1)), False
     if r == 1 or rows <= 1:
