@@ -81,12 +81,25 @@ __device__ __forceinline__ void exp_table_init(bool used) {
     __syncthreads();
   }
 }
-// |x| >= 32 and non-finite arguments (a call, so that the common path's
-// registers and code do not carry it)
+// |x| >= 32 and NaN (a call, so that the common path's registers and code do
+// not carry it); from -708.5 down and 710 up no result is normal.
 __device__ __noinline__ double exp_far(double v) {
+  const uint32_t hi = (uint32_t)__double2hiint(v);
+  if (hi >= 0xC0862400u || (hi & 0x7FFFFFFFu) >= 0x40863000u) return exp(v);
   bool special;
   const double r = nrs_exp_fixed(v, exp_table(), special);
   return special ? exp(v) : r;
+}
+// Results that are 0 or Inf whatever the low bits: x <= -746 or x >= 710. (The
+// arguments of a Gaussian over spread-out points and of masked scores are mostly
+// such. 8192^2 of -Inf: 2347 us through exp_far, 2138 before the fixed-point
+// form.)
+__device__ __forceinline__ bool exp_flat(double v, double& r) {
+  const uint64_t u = (uint64_t)__double_as_longlong(v);
+  const bool zero = u - 0xC087500000000000ull <= 0xFFF0000000000000ull - 0xC087500000000000ull;
+  const bool inf = u - 0x4086300000000000ull <= 0x7FF0000000000000ull - 0x4086300000000000ull;
+  r = zero ? 0.0 : inf ? __longlong_as_double(0x7FF0000000000000ll) : r;
+  return zero | inf;
 }
 template <int W>
 __device__ __forceinline__ void exp_vec(double (&v)[W]) {
@@ -99,8 +112,15 @@ __device__ __forceinline__ void exp_vec(double (&v)[W]) {
     special |= (unsigned)far << e;
   }
   if (special) {
+    bool flat = false;  // (tested first: arguments between 32 and 710 do not pay for it)
+#pragma unroll
+    for (int e = 0; e < W; ++e) flat |= ((uint32_t)__double2hiint(v[e]) & 0x7FFFFFFFu) >= 0x40863000u;
+    if (flat) {
+#pragma unroll
+      for (int e = 0; e < W; ++e) special &= ~((unsigned)exp_flat(v[e], r[e]) << e);
+    }
 #pragma unroll 1
-    for (int e = 0; e < W; ++e) {
+    for (int e = 0; special >> e; ++e) {
       if (!((special >> e) & 1)) continue;
       double x = v[0];
 #pragma unroll
