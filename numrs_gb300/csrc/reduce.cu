@@ -1181,9 +1181,24 @@ RingDims ring_dims(const KeptDims& k) {
 // 591, 1000 x 20001 columns 111 / 121, 1000 x 50001 columns 158 / 234); along
 // contiguous lanes also for many lanes once they are long (a thread's own row
 // takes a sector per few elements: 100001 x 301 f32 60 / 43, x 101 22 / 24).
+// From 56000 of them on a full GPU of threads streams the rows as fast: f64
+// folds stay there (300001 x 401 sums 254 / 288, argmax 257 / 367, 60001 x 301
+// 54 / 57 and 68 / 76, 50001 x 301 53 / 48 and 67 / 60; variances
+// 1005 / 946, the ring squares in its movers), other 8-byte elements and f32
+// variances below about 288 elements (i64 100001 x 257 52 / 55, x 301 68 / 64).
+// f32 variances of columns just below 20000: 257 x 19999 21 / 24, 601 36 / 38,
+// 3001 408 / 181. OP: NRS_ARGMAX for both arg scans.
+template <typename T, int OP>
 bool ring_pays(int64_t alen, int64_t astride, int64_t n_out) {
-  if (n_out < 20000) return alen >= (astride == 1 ? 64 : 256);
-  return astride == 1 && alen >= 256;
+  constexpr bool var = OP == NRS_VAR || OP == NRS_STD;
+  if (n_out < 20000) {
+    if (astride == 1) return alen >= 64;
+    return alen >= (var && std::is_same<T, float>::value && n_out >= 16384 ? 1024 : 256);
+  }
+  if (astride != 1) return false;
+  if (n_out < 56000) return alen >= 256;
+  if (std::is_same<T, double>::value && !var) return false;
+  return alen >= (sizeof(T) == 8 || var ? 288 : 256);
 }
 
 template <typename T, typename Kern, typename... Args>
@@ -1216,7 +1231,7 @@ int launch_arg(nrs_handle* h, const AxisProblem& p) {
     const int st = launch_arg_tma<T, MAX>(h, p);
     if (st != NRS_ERR_UNSUPPORTED) return st;
   }
-  if (ring_pays(p.alen, p.astride, p.n_out)) return launch_arg_ring<T, MAX>(h, p);
+  if (ring_pays<T, NRS_ARGMAX>(p.alen, p.astride, p.n_out)) return launch_arg_ring<T, MAX>(h, p);
   int64_t blocks = (p.n_out + 255) / 256;
   int grid = (int)(blocks < (int64_t)h->num_sms * 16 ? blocks : (int64_t)h->num_sms * 16);
   if (grid < 1) grid = 1;
@@ -1435,7 +1450,7 @@ int dispatch_axis_t(nrs_handle* h, const AxisProblem& p) {
     int st = launch_tma<T, OP>(h, p);
     if (st != NRS_ERR_UNSUPPORTED) return st;
   }
-  if (ring_pays(p.alen, p.astride, p.n_out)) return launch_ring<T, OP>(h, p);
+  if (ring_pays<T, OP>(p.alen, p.astride, p.n_out)) return launch_ring<T, OP>(h, p);
   return launch_generic<T, OP>(h, p);
 }
 

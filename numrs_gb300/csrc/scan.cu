@@ -1232,7 +1232,9 @@ int launch_lanes(nrs_handle* h, const LaneProblem& p) {
   // per few elements when a thread owns its row: 100001 x 301 f64 329 / 172
   // us, and 1000 x 50001 columns 225 / 286).
   const bool rows = p.xastride == 1, few = p.n_lanes < 20000;
-  if (p.alen >= (rows && (few || RUNNING) ? 64 : 256) && (rows || few)) {
+  const bool many = !RUNNING && sizeof(T) == 8 && p.n_lanes >= 56000;
+  constexpr bool f64_chain = std::is_same<T, double>::value && OP != NRS_OP_MAX && OP != NRS_OP_MIN;
+  if (p.alen >= (rows && (few || RUNNING) ? 64 : many ? 288 : 256) && (rows || few) && !(many && f64_chain)) {
     RingDims g{};
     g.n = p.lanes.n;
     for (int d = 0; d < g.n; ++d) {
