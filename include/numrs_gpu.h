@@ -68,6 +68,11 @@ const char* nrs_status_string(int status);
 /* Creates a handle bound to `device`, with its own non-blocking stream. */
 int nrs_create(int device, nrs_handle** out);
 int nrs_destroy(nrs_handle* h);
+/* Gives the scratch that the handle keeps between NRS_GEMM_AUTO calls (up to
+ * 4.6 GB, whatever they took; more goes back at each synchronisation) back to
+ * the device, after the work on its stream. The next such call takes its own
+ * again. */
+int nrs_trim(nrs_handle* h);
 /* Enqueue on a caller-owned cudaStream_t; NULL means CUDA's default stream. */
 int nrs_set_stream(nrs_handle* h, void* cuda_stream);
 /* Enqueue on the handle's own non-blocking stream (the state after create). */

@@ -83,6 +83,7 @@ SIGNATURES = {
     "nrs_status_string": (C.c_char_p, [_i]),
     "nrs_create": (_i, [_i, C.POINTER(_vp)]),
     "nrs_destroy": (_i, [_vp]),
+    "nrs_trim": (_i, [_vp]),
     "nrs_set_stream": (_i, [_vp, _vp]),
     "nrs_use_own_stream": (_i, [_vp]),
     "nrs_get_stream": (_vp, [_vp]),

@@ -43,7 +43,8 @@ struct nrs_handle {
   size_t workspace_bytes = 0;
   // Stream-ordered scratch of the calls that choose the tensor cores by
   // themselves (null: they keep to the plain kernels). Up to kPoolKeep bytes
-  // stay with the pool between calls; it goes with the handle.
+  // stay with the pool between calls (nrs_trim gives them back); it goes with
+  // the handle.
   cudaMemPool_t pool = nullptr;
   // Device error word written by kernels whose waits are bounded.
   uint32_t* dev_error = nullptr;

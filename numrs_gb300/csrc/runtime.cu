@@ -158,6 +158,14 @@ extern "C" int nrs_destroy(nrs_handle* h) {
   return NRS_OK;
 }
 
+extern "C" int nrs_trim(nrs_handle* h) {
+  if (!h) return NRS_ERR_INVALID;
+  int st = nrs_cuda_check(h, cudaSetDevice(h->device), "cudaSetDevice");
+  if (st == NRS_OK) st = nrs_cuda_check(h, cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+  if (st == NRS_OK && h->pool) st = nrs_cuda_check(h, cudaMemPoolTrimTo(h->pool, 0), "cudaMemPoolTrimTo");
+  return st;
+}
+
 extern "C" int nrs_set_stream(nrs_handle* h, void* s) {
   if (!h) return NRS_ERR_INVALID;
   // NULL is CUDA's default stream (the one a framework's "current stream"

@@ -70,6 +70,13 @@ def synchronize() -> None:
     L.check(L.load().nrs_synchronize(h), h)
 
 
+def trim() -> None:
+    """Gives the scratch that large products leave with the library (up to
+    4.6 GB) back to the device."""
+    h = handle()
+    L.check(L.load().nrs_trim(h), h)
+
+
 # ---------------------------------------------------------------------------
 # Reductions
 # ---------------------------------------------------------------------------
