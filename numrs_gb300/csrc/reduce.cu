@@ -1008,10 +1008,14 @@ template <typename T>
 bool flat_is_small(int64_t n, int64_t nchunks) {
   return nchunks >= 1 && nchunks <= kSmallChunks && n * (int64_t)sizeof(T) <= 512 * 1024;
 }
-template <typename T, int OP, bool VEC>
-__global__ void __launch_bounds__(32 * kSmallChunks)
+// MOST: chunks of the launch at most. 32 warps leave a thread 64 registers, and
+// the f64 chunks are slower for it, so up to 8 chunks have a kernel of their own
+// (us per call with 64 and without that limit: product of 8192 f64 20.8 / 16.6,
+// variance of 32768 146 / 129).
+template <typename T, int OP, bool VEC, int MOST>
+__global__ void __launch_bounds__(32 * MOST)
     flat_small(const T* __restrict__ x, int64_t n, int64_t chunk, int fin_op, double ddof, void* out) {
-  __shared__ Partial<T> part[kSmallChunks];
+  __shared__ Partial<T> part[MOST];
   __shared__ T mean;
   const int w = threadIdx.x >> 5, nchunks = (int)(blockDim.x >> 5);
   const int64_t lo = w * chunk, len = (n - lo) < chunk ? (n - lo) : chunk;
@@ -1051,11 +1055,11 @@ __global__ void __launch_bounds__(32 * kSmallChunks)
 
 template <typename T, int OP>
 int launch_flat_small(nrs_handle* h, const T* x, int64_t n, int64_t chunk, int fin_op, double ddof, void* out) {
-  const int threads = 32 * (int)((n + chunk - 1) / chunk);
-  if ((reinterpret_cast<uintptr_t>(x) & 15) == 0)
-    flat_small<T, OP, true><<<1, threads, 0, h->stream>>>(x, n, chunk, fin_op, ddof, out);
-  else
-    flat_small<T, OP, false><<<1, threads, 0, h->stream>>>(x, n, chunk, fin_op, ddof, out);
+  const int chunks = (int)((n + chunk - 1) / chunk);
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  auto kern = chunks <= 8 ? (vec ? flat_small<T, OP, true, 8> : flat_small<T, OP, false, 8>)
+                          : (vec ? flat_small<T, OP, true, kSmallChunks> : flat_small<T, OP, false, kSmallChunks>);
+  kern<<<1, 32 * chunks, 0, h->stream>>>(x, n, chunk, fin_op, ddof, out);
   return nrs_after_launch(h, "flat_small");
 }
 template <typename T>
