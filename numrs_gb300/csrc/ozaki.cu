@@ -190,19 +190,6 @@ NRS_DEV bool elect_one() {
   return p != 0;
 }
 
-// 32 lanes x 16 consecutive 32-bit columns.
-NRS_DEV void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // 32 lanes x 16 columns into v[0..15] without waiting: several loads can be
 // in flight before one tcgen05.wait::ld.
 NRS_DEV void tmem_ld16_nowait(uint32_t taddr, uint32_t* v) {
@@ -317,7 +304,7 @@ struct OzParams {
   int group_m;     // tile rasterisation group height
   const int* ea;   // row exponents of A
   const int* eb;   // column exponents of B
-  __int128* acc;   // per-CTA digit slots (16-byte aligned)
+  uint8_t* acc;    // per-CTA digit slots (16-byte aligned)
   double* C;       // float when f32 (and not split)
   int64_t ldc;
   int digit_bits;  // b
@@ -932,7 +919,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const uint32_t dig_t = lane_base + 3 * BN;   // digits 0..3
     const int b = B8 ? 8 : P.digit_bits, nd = S - 1;
     const uint32_t dmask = (1u << b) - 1;
-    uint8_t* const slot = reinterpret_cast<uint8_t*>(P.acc) + (size_t)blockIdx.x * (kColPitch * BN) +
+    uint8_t* const slot = P.acc + (size_t)blockIdx.x * (kColPitch * BN) +
                           (size_t)row_in_tile * OZ_DIGIT_BYTES;
     uint32_t dreg[BN / 2];  // this thread's digit word per element (chunk i, column e: [i * 16 + e])
     // this warp's column exponents, [i * 16 + e] for chunk i, column e
@@ -1108,7 +1095,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const int b = B8 ? 8 : P.digit_bits, nd = S - 1;
     constexpr size_t kChunk = (size_t)OZ_BM * 16;        // bytes of 16 columns of a digit
     constexpr size_t kPlane = (size_t)OZ_BM * OZ_BN;      // bytes of a digit
-    uint8_t* const slot = reinterpret_cast<uint8_t*>(P.acc) + (size_t)blockIdx.x * (kPlane * 16) +
+    uint8_t* const slot = P.acc + (size_t)blockIdx.x * (kPlane * 16) +
                           (size_t)(half * (OZ_BN / 32)) * kChunk + (size_t)row_in_tile * 16;
     const uint32_t acce0 = cluster_addr(&acce[0], 0);  // rank 0's barriers
     auto release = [&](int buf) {
@@ -2097,7 +2084,7 @@ int ozaki_run(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m,
   P.slices = S;
   P.ea = w.ea;
   P.eb = w.eb;
-  P.acc = reinterpret_cast<__int128*>(w.tail);
+  P.acc = w.tail;
   P.C = C;
   P.ldc = ldc;
   P.digit_bits = b;
@@ -2160,7 +2147,7 @@ int tc_gemm(nrs_handle* h, const OzOperand& a, const OzOperand& bT, int64_t m, i
     P.count = w.words + OZ_W_COUNT;
     P.ea = w.ea;
     P.eb = w.eb;
-    P.acc = reinterpret_cast<__int128*>(w.tail);
+    P.acc = w.tail;
     P.C = pl.splits > 1 ? slab : static_cast<double*>(C);
     P.ldc = ldc;
     P.digit_bits = b;
@@ -2522,7 +2509,7 @@ struct nrs_ozaki_group {
   int *d_ea = nullptr, *d_eb = nullptr;
   unsigned long long* d_colmax = nullptr;
   uint16_t *d_sa = nullptr, *d_sb = nullptr;
-  __int128* d_acc = nullptr;
+  uint8_t* d_acc = nullptr;
 };
 
 void nrs_ozaki_group_free(nrs_ozaki_group* g) {
@@ -2681,7 +2668,7 @@ int nrs_ozaki_group_build(nrs_handle* h, int64_t count, const nrs_gemm_desc* d, 
   G->d_colmax = (unsigned long long*)take(b_cm);
   G->d_sa = (uint16_t*)take(b_sa);
   G->d_sb = (uint16_t*)take(b_sb);
-  G->d_acc = (__int128*)take(b_acc);
+  G->d_acc = take(b_acc);
   G->S = S;
   G->b = b;
   G->f32 = f32 ? 1 : 0;
