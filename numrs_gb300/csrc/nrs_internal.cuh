@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/numrs_gpu.h"
 
@@ -38,9 +39,13 @@ struct nrs_handle {
   int hw_sms = 0;    // the device's SM count
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
-  // Grow-only device workspace for kernels that need scratch memory.
+  // Grow-only device workspace for kernels that need scratch memory. A capture
+  // that used it leaves its address in a graph: growing then sets it aside
+  // until the handle goes.
   void* workspace = nullptr;
   size_t workspace_bytes = 0;
+  bool workspace_captured = false;
+  std::vector<void*> set_aside;
   // Stream-ordered scratch of the calls that choose the tensor cores by
   // themselves (null: they keep to the plain kernels). Up to kPoolKeep bytes
   // stay with the pool between calls (nrs_trim gives them back); it goes with

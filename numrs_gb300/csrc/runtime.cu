@@ -52,22 +52,33 @@ size_t nrs_dtype_size(int dtype) {
 
 void* nrs_workspace(nrs_handle* h, size_t bytes, int* status) {
   *status = NRS_OK;
-  if (bytes <= h->workspace_bytes) return h->workspace;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) cudaGetLastError();
+  if (bytes <= h->workspace_bytes) {
+    h->workspace_captured |= cap != cudaStreamCaptureStatusNone;
+    return h->workspace;
+  }
   size_t want = bytes < (1u << 20) ? (1u << 20) : bytes;
   want = (want + 255) & ~size_t(255);
-  if (h->workspace) {
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  const bool keep = h->workspace && (h->workspace_captured || capturing);
+  if (h->workspace && !keep) {
     // The old workspace may still be read by queued work on this stream.
     cudaStreamSynchronize(h->stream);
     cudaFree(h->workspace);
     h->workspace = nullptr;
     h->workspace_bytes = 0;
   }
-  if (cudaMalloc(&h->workspace, want) != cudaSuccess) {
+  void* fresh = nullptr;
+  if (cudaMalloc(&fresh, want) != cudaSuccess) {
     cudaGetLastError();
     *status = nrs_fail(h, NRS_ERR_ALLOC, "workspace cudaMalloc failed");
     return nullptr;
   }
+  if (keep) h->set_aside.push_back(h->workspace);
+  h->workspace = fresh;
   h->workspace_bytes = want;
+  h->workspace_captured = capturing;
   return h->workspace;
 }
 
@@ -124,14 +135,14 @@ extern "C" int nrs_create(int device, nrs_handle** out) {
     if (h->pool) cudaMemPoolDestroy(h->pool);
     h->pool = nullptr;
   }
+  h->hw_sms = h->num_sms;
+  h->stream = h->own_stream;
   // The workspace's smallest size from the start: a short flat reduction runs
   // without it, and a longer one that is captured next could not get it then.
   // (No room now: the first call that needs it asks again.)
   int ws = NRS_OK;
   nrs_workspace(h, 1, &ws);
   h->last_error.clear();
-  h->hw_sms = h->num_sms;
-  h->stream = h->own_stream;
   *out = h;
   return NRS_OK;
 }
@@ -149,6 +160,7 @@ extern "C" int nrs_destroy(nrs_handle* h) {
   cudaSetDevice(h->device);
   cudaStreamSynchronize(h->stream);
   if (h->workspace) cudaFree(h->workspace);
+  for (void* p : h->set_aside) cudaFree(p);
   if (h->pool) cudaMemPoolDestroy(h->pool);
   if (h->dev_error) cudaFree(h->dev_error);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -160,7 +172,10 @@ extern "C" int nrs_destroy(nrs_handle* h) {
 
 extern "C" int nrs_trim(nrs_handle* h) {
   if (!h) return NRS_ERR_INVALID;
-  int st = nrs_cuda_check(h, cudaSetDevice(h->device), "cudaSetDevice");
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  int st = nrs_cuda_check(h, cudaStreamIsCapturing(h->stream, &cap), "cudaStreamIsCapturing");
+  if (st == NRS_OK && cap != cudaStreamCaptureStatusNone) return nrs_fail(h, NRS_ERR_INVALID, "the stream is being captured");
+  if (st == NRS_OK) st = nrs_cuda_check(h, cudaSetDevice(h->device), "cudaSetDevice");
   if (st == NRS_OK) st = nrs_cuda_check(h, cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
   if (st == NRS_OK && h->pool) st = nrs_cuda_check(h, cudaMemPoolTrimTo(h->pool, 0), "cudaMemPoolTrimTo");
   return st;

@@ -67,3 +67,30 @@ def test_flat_reduction_after_a_short_one(K, call):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, K.sum(x))
+
+
+def test_a_larger_call_leaves_a_captured_workspace_alone(K, call):
+    """The graph's launches hold the workspace's address; the variances of
+    200,000 rows need a larger one (1.6 MB of means)."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(300_000, dtype=torch.float64, device="cuda", generator=g)
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    rows = torch.randn((200_000, 40), dtype=torch.float64, device="cuda", generator=g)
+    var = torch.zeros(200_000, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+
+    def total():
+        call("nrs_reduce", L.F64, L.SUM, 1, L.i64_array([300_000]), L.i64_array([1]), L.AXIS_NONE, 0, _p(x), _p(out))
+    total()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        total()
+    call("nrs_reduce", L.F64, L.VAR, 2, L.i64_array([200_000, 40]), L.i64_array([40, 1]), 1, 0, _p(rows), _p(var))
+    others = [torch.full((1 << 18,), -1, dtype=torch.int64, device="cuda") for _ in range(8)]
+    x.mul_(2.0)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, K.sum(x)) and torch.equal(var, K.var(rows, 1))
+    assert all(int(t.min()) == -1 and int(t.max()) == -1 for t in others)
