@@ -363,8 +363,11 @@ typedef enum nrs_gemm_variant {
  * K runs in up to 16 ranges; a K-long FMA chain's bound is K units. Everything
  * else and calls under stream capture run the plain kernels, and so do operands
  * that the slices cannot carry to that (Inf or NaN, sums that may overflow,
- * entries too far apart for 12 slices), after the measurement that finds them.
- * Their scratch is stream-ordered and the library's own. */
+ * entries too far apart for 12 slices; 8 for f32), after the measurement that
+ * finds them. (Units of a result that is normal; one rounding otherwise.)
+ * Their scratch is stream-ordered and the library's own (nrs_trim). A
+ * captured f64 product takes the room for the FP64 kernel's K ranges from the
+ * workspace, where a call of the same sizes outside a capture leaves it. */
 int nrs_gemm(nrs_handle* h, int dtype, int64_t m, int64_t k, int64_t n, const void* A,
              int64_t lda, const void* B, int64_t ldb, void* C, int64_t ldc, unsigned flags,
              int variant);
@@ -397,9 +400,11 @@ typedef struct nrs_ozaki_info {
   int32_t products;      /* slice-pair GEMM work units executed              */
   int32_t slice_bits;    /* bits carried by each slice after the first       */
   int32_t k_chunk;       /* K block inside which fp32 accumulation is exact  */
-  double est_rel_error;  /* slices = 0 (auto): estimated max_ij |C - AB|_ij /
-                            (|A||B|)_ij; explicit count: a-priori bound on
-                            |C - AB| / (rowmax|A| colmax|B| k)               */
+  double est_rel_error;  /* slices = 0 (auto): bound on max_ij |C - AB|_ij /
+                            (|A||B|)_ij from the measured spread (entries that
+                            do not repeat along K stay far below it); explicit
+                            count: a-priori bound on |C - AB| / (rowmax|A|
+                            colmax|B| k)                                      */
   double spread;         /* auto: max_ij R_ij measured (below); else 0       */
 } nrs_ozaki_info;
 
